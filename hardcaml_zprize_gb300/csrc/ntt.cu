@@ -2,23 +2,18 @@
 // NTT track (zprize/ntt).  The transform is the reference's (zprize/ntt/host/reference.cpp:94-139):
 // X[k] = sum_j x[j] w^(j k) with w = OMEGA[log2 n] of zprize/ntt/host/gf.h:65-99, natural order in
 // and out.  The reference evaluates 2^24 points on the FPGA with the 4-step decomposition into
-// 2^12-point transforms (zprize/ntt/docs/zprize_ntt_top.mld:6-31); this engine does the same split,
-// n = n1 n2 with n1, n2 <= 2^12:
-//   pass A: for every column j1 of the n2 x n1 row-major input, the n2-point transform over j2,
-//           times w^(j1 k2), written to Z[k2][j1];
-//   pass B: for every row k2 of Z, the n1-point transform over j1, written to X[k2 + n2 k1].
-// One kernel (k_ntt_pass8) does both passes: a block holds C <= 4 of the short transforms in
-// shared memory, runs them as radix-8 decimation-in-frequency rounds (three stages per round in
-// registers), and gathers the outputs in natural order, optionally twisted.  With C = 4 every row
-// of a column load and every output group of a store is 32 contiguous bytes, one DRAM sector.
-// HBM traffic: n x 8 B read and written per pass.  k_ntt_pass, the first form (radix-2
-// decimation-in-time stages on bit-reversed positions), stays for comparison (NTT_RADIX2=1).
-// Transforms of at most 2^12 points are one pass.  An inverse context (ntt_init_inverse) runs the
-// same kernels with the inverse roots and multiplies by 1/n: the factor sits in pass A's twist
-// table, or in the store of a transform of one pass.
-//
-// Field arithmetic: elements in [0, p).  The 128-bit product hi 2^64 + lo reduces with
-// 2^64 = 2^32 - 1 and 2^96 = -1 (mod p): hi = hh 2^32 + hl gives lo - hh + hl (2^32 - 1).
+// 2^12-point transforms (zprize/ntt/docs/zprize_ntt_top.mld:6-31); this engine splits further, into
+// passes of at most 2^8 points: one up to 2^8 points, two up to 2^12, three up to 2^24.  With
+// n = a b c (c = 1 for two passes) and the input index j = (ja, jb, jc), most significant first:
+//   pass 1: over ja for every column (jb, jc), times w_ab^(ka jb), to Z[ka][jb][jc];
+//   pass 2: over jb for every (ka, jc), times w^(jc (ka + a kb)), in place;
+//   pass 3: over jc for every (ka, kb), to X[ka + a kb + a b kc].
+// One kernel template (k_ntt_pass) does every pass: a block holds eight of the short transforms
+// (64 contiguous bytes of every row it reads or writes) and runs each as two rounds of at most 16
+// points in registers, whose roots are powers of two (goldilocks.cuh).
+// An inverse context (ntt_init_inverse) runs the same forward kernels, stores output k at place
+// (n - k) mod n and multiplies by 1/n: the factor sits in a twist table, or in the store of a
+// transform of one pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,12 +26,19 @@
 #include <vector>
 
 #include "../../include/ntt_gb300.h"
+#include "goldilocks.cuh"
 
 namespace {
 
-constexpr uint64_t GL_P = 0xffffffff00000001ull;
-constexpr uint32_t NTT_MAX_LOG_M = 12;      // longest transform of one block
-constexpr uint32_t NTT_THREADS = 1024;
+constexpr uint32_t NTT_MAX_LOG_N = 24;
+constexpr uint32_t NTT_ONE_PASS = 8;   // largest log2 of a transform of one pass
+// Two passes up to here, three above: three short ones spread over more blocks.  Measured on GB300
+// (us, two passes / three): 2^12 5.4 / 5.4, 2^13 6.8 / 5.4, 2^14 8.1 / 5.5, 2^16 10.0 / 7.0.
+constexpr uint32_t NTT_TWO_PASS = 12;
+// log2 transforms per block of a split transform.  Eight: 64 contiguous bytes of every row.
+// Measured with four / eight / sixteen (us): the passes of 2^24 points without their arithmetic
+// 160 / 127 / 125, whole 335 / 248 / 258; 2^16 points 9.6 / 7.0, 2^12 points 5.5 / 5.4.
+constexpr int NTT_LOG_COLS = 3;
 
 // 2^i-th roots of unity of the reference's table (gf.h:65-99); OMEGA[i+1]^2 = OMEGA[i]
 const uint64_t GL_OMEGA[33] = {
@@ -50,268 +52,286 @@ const uint64_t GL_OMEGA[33] = {
     0x59049500004a4485ull, 0xdfa8c93ba46d2666ull, 0x7e9bd009b86a0845ull, 0x400a7f755588e659ull,
     0x185629dcda58878cull};
 
-// ---- host-side field arithmetic (table set-up) ----
+// ---- host-side field arithmetic (set-up) ----
 uint64_t h_mul(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) % GL_P); }
-
-// ---- device field arithmetic ----
-// Carry-chain forms on 32-bit halves: every correction is driven by a carry or borrow flag, so no
-// 64-bit comparison or select chain is needed.  Inputs and outputs are canonical (below p).
-__device__ __forceinline__ uint64_t gl_pack(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
-
-// a + b: S = a + b < 2p; S >= p exactly when S + (2^32 - 1) carries out of 64 bits (counting
-// the first carry), and then S - p = (S + 2^32 - 1) mod 2^64
-__device__ __forceinline__ uint64_t gl_add(uint64_t a, uint64_t b) {
-  uint32_t s0, s1, t0, t1, c;
-  asm("{\n\t.reg .u32 c1;\n\t"
-      "add.cc.u32 %0, %5, %7;\n\t"
-      "addc.cc.u32 %1, %6, %8;\n\t"
-      "addc.u32 c1, 0, 0;\n\t"
-      "add.cc.u32 %2, %0, 0xffffffff;\n\t"
-      "addc.cc.u32 %3, %1, 0;\n\t"
-      "addc.u32 %4, c1, 0;\n\t}"
-      : "=&r"(s0), "=&r"(s1), "=&r"(t0), "=&r"(t1), "=&r"(c)
-      : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
-  return c ? gl_pack(t0, t1) : gl_pack(s0, s1);
+uint64_t h_pow(uint64_t b, uint64_t e) {
+  uint64_t r = 1;
+  for (; e; e >>= 1, b = h_mul(b, b))
+    if (e & 1) r = h_mul(r, b);
+  return r;
 }
-
-// a - b: on a borrow the wrapped difference d = a - b + 2^64 >= 2^32, and d - (2^32 - 1) is
-// a - b + p
-__device__ __forceinline__ uint64_t gl_sub(uint64_t a, uint64_t b) {
-  uint32_t d0, d1;
-  asm("{\n\t.reg .u32 bw;\n\t"
-      "sub.cc.u32 %0, %2, %4;\n\t"
-      "subc.cc.u32 %1, %3, %5;\n\t"
-      "subc.u32 bw, 0, 0;\n\t"
-      "sub.cc.u32 %0, %0, bw;\n\t"
-      "subc.u32 %1, %1, 0;\n\t}"
-      : "=&r"(d0), "=&r"(d1)
-      : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
-  return gl_pack(d0, d1);
-}
-
-// a b: the 128-bit product (r3 r2 r1 r0) from four wide multiplies whose 64-bit addends carry
-// the partial products' overflow (the carries ride in the multiplies, which run on the multiply
-// pipe, and not in add chains on the integer ALU, which bounded the passes), then
-// lo + hl (2^32 - 1) - hh with
-// lo = r1 r0, hl = r2, hh = r3 (2^64 = 2^32 - 1, 2^96 = -1 mod p): hl (2^32 - 1) is a fifth wide
-// multiply, each step is corrected by its own carry or borrow, and a last conditional
-// subtraction of p makes the value canonical.
-//   s = lo + hl (2^32 - 1) < 2^65; a carry out adds 2^32 - 1, and then s < 2^64 - 2^32;
-//   t = s - hh; a borrow subtracts 2^32 - 1 more (t + p), which stays above zero.
-__device__ __forceinline__ uint64_t gl_mul(uint64_t a, uint64_t b) {
-  const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-  const uint64_t x = (uint64_t)a0 * b0;
-  const uint64_t y = (uint64_t)a0 * b1 + (x >> 32);
-  const uint64_t z = (uint64_t)a1 * b0 + (uint32_t)y;
-  const uint64_t w = (uint64_t)a1 * b1 + (y >> 32) + (z >> 32);
-  const uint64_t u = (uint64_t)(uint32_t)w * 0xffffffffu;  // hl (2^32 - 1)
-  uint32_t t0, t1, q0, q1, c;
-  asm("{\n\t.reg .u32 m;\n\t"
-      "add.cc.u32 %0, %5, %7;\n\t"       // s = lo + u
-      "addc.cc.u32 %1, %6, %8;\n\t"
-      "addc.u32 m, 0, 0;\n\t"
-      "neg.s32 m, m;\n\t"                // 2^32 - 1 on a carry
-      "add.cc.u32 %0, %0, m;\n\t"
-      "addc.u32 %1, %1, 0;\n\t"
-      "sub.cc.u32 %0, %0, %9;\n\t"       // t = s - hh
-      "subc.cc.u32 %1, %1, 0;\n\t"
-      "subc.u32 m, 0, 0;\n\t"            // 2^32 - 1 on a borrow
-      "sub.cc.u32 %0, %0, m;\n\t"
-      "subc.u32 %1, %1, 0;\n\t"
-      "add.cc.u32 %2, %0, 0xffffffff;\n\t"  // t >= p exactly when t + 2^32 - 1 carries
-      "addc.cc.u32 %3, %1, 0;\n\t"
-      "addc.u32 %4, 0, 0;\n\t}"
-      : "=&r"(t0), "=&r"(t1), "=&r"(q0), "=&r"(q1), "=&r"(c)
-      : "r"((uint32_t)x), "r"((uint32_t)z), "r"((uint32_t)u), "r"((uint32_t)(u >> 32)),
-        "r"((uint32_t)(w >> 32)));
-  return c ? gl_pack(q0, q1) : gl_pack(t0, t1);
-}
-
-__device__ __forceinline__ uint32_t bit_reverse(uint32_t x, uint32_t bits) {
-  return bits ? __brev(x) >> (32 - bits) : 0u;
-}
+uint64_t h_inv(uint64_t a) { return h_pow(a, GL_P - 2); }  // Fermat; a != 0
+uint64_t h_mont(uint64_t a) { return (uint64_t)(((unsigned __int128)a << 64) % GL_P); }  // gl_mul's table form
 
 struct NttPass {
   const uint64_t *src;
   uint64_t *dst;
-  uint32_t log_m;  // transform length of this pass
-  uint32_t cols;   // transforms per block (1, 2 or 4)
-  uint32_t log_cols;  // log2 cols: the block's index splits are shifts and masks, not divisions
-  uint64_t in_c, in_i;    // element i of transform g: src[g in_c + i in_i]
-  uint64_t out_c, out_k;  // output k of transform g: dst[g out_c + k out_k]
-  const uint64_t *tw_m;   // w_m^j, j < m/2
-  // twist (pass A): output k of transform g times w_n^(g k mod n), from w_n^e = hi[e >> 12] lo[e & 4095]
-  const uint64_t *tw_lo, *tw_hi;
-  uint64_t n_mask;  // n - 1 when twisting, 0 otherwise
-  uint64_t scale;   // outputs of an untwisted pass times this (0: none), the inverse's 1/n
+  // transform g = (gh, gl), gl its low log_gl bits: element i at src[gl in_c + gh in_h + i in_i],
+  // output k at dst[gl out_c + gh out_h + k out_k]
+  uint32_t log_gl, gl_mask;
+  uint32_t in_c, in_h, in_i;
+  uint32_t out_c, out_h, out_k;
+  const uint64_t *tw1;  // the round boundary's factors w_m^(k0 u), tw1[k0 U + u]
+  // twist tables (see TW_TABLE, TW_SHARED, TW_STEPS)
+  const uint64_t *tw, *tw_a;
+  uint32_t t_k, t_g, t_shift;
+  uint32_t o_mask;   // n - 1
+  uint32_t reverse;  // output places negated modulo n (last pass of an inverse)
+  uint64_t scale;    // outputs of an untwisted pass times this (0: none), the inverse's 1/n
 };
 
-__global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(NttPass ps) {
-  extern __shared__ uint64_t sm[];
-  const uint32_t m = 1u << ps.log_m, C = ps.cols, half = m >> 1;
-  uint64_t *tw = sm + (size_t)C * m;
-  const uint64_t g0 = (uint64_t)blockIdx.x * C;
-  for (uint32_t j = threadIdx.x; j < half; j += blockDim.x) tw[j] = ps.tw_m[j];
-  // load C transforms, element i to its bit-reversed slot; the unit-stride index runs fastest
-  const bool c_fast = ps.in_c == 1;
-  for (uint32_t t = threadIdx.x; t < C * m; t += blockDim.x) {
-    const uint32_t c = c_fast ? t & (C - 1) : t >> ps.log_m, i = c_fast ? t >> ps.log_cols : t & (m - 1);
-    uint64_t v = __ldcs(ps.src + (g0 + c) * ps.in_c + (uint64_t)i * ps.in_i);
-    if (v >= GL_P) v -= GL_P;  // inputs are taken modulo p
-    sm[(size_t)c * m + bit_reverse(i, ps.log_m)] = v;
-  }
-  __syncthreads();
-  for (uint32_t s = 1; s <= ps.log_m; s++) {
-    const uint32_t h = 1u << (s - 1);
-    for (uint32_t t = threadIdx.x; t < C * half; t += blockDim.x) {
-      const uint32_t c = t >> (ps.log_m - 1), r = t & (half - 1);
-      const uint32_t j = r & (h - 1), k0 = ((r >> (s - 1)) << s) + j;
-      uint64_t *a = sm + (size_t)c * m;
-      const uint64_t w = tw[j << (ps.log_m - s)];  // w_m^(j m / 2h), a primitive 2h-th root
-      const uint64_t u = a[k0], v = gl_mul(a[k0 + h], w);
-      a[k0] = gl_add(u, v);
-      a[k0 + h] = gl_sub(u, v);
-    }
-    __syncthreads();
-  }
-  // store, output groups of C consecutive transforms together
-  for (uint32_t t = threadIdx.x; t < C * m; t += blockDim.x) {
-    const uint32_t c = t & (C - 1), k = t >> ps.log_cols;
-    uint64_t v = sm[(size_t)c * m + k];
-    if (ps.n_mask) {
-      const uint64_t e = ((g0 + c) * (uint64_t)k) & ps.n_mask;
-      v = gl_mul(v, gl_mul(ps.tw_hi[e >> 12], ps.tw_lo[e & 4095]));
-    } else if (ps.scale) {
-      v = gl_mul(v, ps.scale);
-    }
-    __stcs(ps.dst + (g0 + c) * ps.out_c + (uint64_t)k * ps.out_k, v);
+// streaming accesses: a pass reads and writes every word once
+GL_FN uint64_t gl_ldcs(const uint64_t *p) {
+#ifdef __CUDA_ARCH__
+  return __ldcs(p);
+#else
+  return *p;
+#endif
+}
+GL_FN void gl_stcs(uint64_t *p, uint64_t v) {
+#ifdef __CUDA_ARCH__
+  __stcs(p, v);
+#else
+  *p = v;
+#endif
+}
+
+// two words from global to shared memory, asynchronously (both on 16-byte boundaries)
+GL_FN void gl_copy16(uint64_t *dst, const uint64_t *src) {
+#ifdef __CUDA_ARCH__
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+#else
+  dst[0] = src[0];
+  dst[1] = src[1];
+#endif
+}
+
+// ---- the pass kernel ----
+// Transforms of m = 2^(L1 + L2) points in two rounds of short transforms (one where L2 = 0):
+// element j = u + 2^L2 t,
+//   round 1, unit u:  over t -> k0, times w_m^(k0 u);
+//   round 2, unit k0: over u -> k1, output k = k0 + 2^L1 k1.
+// Inside a round every root is a power of two (goldilocks.cuh), so a value meets one general
+// product per round boundary and one per pass boundary (the twist).
+//
+// A block holds 2^LC transforms.  Round 1 reads global memory, round 2 writes it; between them
+// values sit in shared memory, point (k0, u) of transform c at k0 PITCH + u C + c, or, for ROWS
+// (transforms whose elements are contiguous: lanes run over u in round 1), k0 PITCH + c (U + 1) + u.
+// With eight transforms PITCH = 8 (mod 16), so the half warps of both rounds meet sixteen banks.
+//
+// What bounds it (ncu and timings on GB300, 2^24 points): the arithmetic and the memory passes
+// together.  Without arithmetic the three passes take 46 + 40 + 41 us (268 MB each, 87 to 100% of
+// the measured copy bandwidth); with it 75 + 83 + 65 us: about 110 instructions per point and pass,
+// of which the 32 x 32 wide multiplies hold the issue port for four cycles each.  The previous
+// kernel (radix 8 with table roots, two passes of 2^12 points, one 147 KB block per SM) took
+// 339 + 272 us: 5 general products per point and pass, and load, arithmetic and store phases that
+// nothing overlapped.  Two passes of three such rounds took 188 + 136 us for the same reason.
+template <int L1, int L2, int LC>
+struct PassShape {
+  static constexpr int LM = L1 + L2, U = 1 << L2, C = 1 << LC;
+  static constexpr int PITCH = C * (U + 1);
+  static constexpr int UNITS = C << (LM - (L1 > L2 && L2 ? L2 : L1));  // of the round with more
+  static constexpr int THREADS = UNITS < 32 ? 32 : UNITS;
+  static constexpr int TW_WORDS = (1 << LM) > C << L2 ? 1 << LM : C << L2;  // staged twist factors
+  static constexpr size_t SMEM = L2 ? (size_t)8 * ((PITCH << L1) + TW_WORDS) : 0;
+};
+
+// base[uniform + lane], the first part the same on every thread of the block (a uniform base
+// register), the second a 32-bit byte offset: no address arithmetic per access
+GL_FN const uint64_t *at_of(const uint64_t *base, uint32_t uniform, uint32_t lane) {
+  return (const uint64_t *)((const char *)(base + uniform) + (lane << 3));
+}
+
+// How a pass twists its outputs (the factor between it and the next pass).
+enum : int {
+  TW_NONE = 0,
+  TW_TABLE,   // tw[k t_k + gl t_g], read from global memory
+  TW_SHARED,  // tw[k + (gl >> t_shift) t_g], the same for the block's transforms: staged in shared memory
+  TW_STEPS,   // base (tw_a[g] tw[v t_k + gl]) times tw[(k - v) t_k + gl], the latter staged: 2^L2 a transform
+};
+
+// The block's share of the twist table, to shared memory behind the points: asynchronous copies
+// that round 1 hides.  Read from global memory in the store loop instead, the factors' latency was
+// exposed there (2^24 points: pass 1 84.6 us, pass 2 98.0 us, against 64.8 us without a twist).
+template <int L1, int L2, int LC, int TWIST>
+GL_FN void pass_stage_twist(const NttPass &ps, uint64_t *tws, uint32_t block, uint32_t tid, uint32_t threads) {
+  using S = PassShape<L1, L2, LC>;
+  const uint32_t gl = block * S::C & ps.gl_mask;
+  if (TWIST == TW_SHARED) {
+    const uint64_t *src = ps.tw + (gl >> ps.t_shift) * ps.t_g;
+    for (uint32_t i = 2 * tid; i < (1u << S::LM); i += 2 * threads) gl_copy16(tws + i, src + i);
+  } else if (TWIST == TW_STEPS) {
+    for (uint32_t i = 2 * tid; i < (1u << (L2 + LC)); i += 2 * threads)
+      gl_copy16(tws + i, ps.tw + ((i >> LC) << L1) * ps.t_k + gl + (i & (S::C - 1)));
   }
 }
 
-// ---- radix-8 decimation in frequency (the pass kernel) ----
-// Natural order in, bit-reversed order in shared memory out: stage H (half size) turns the pair
-// (k, k + H) of each block of 2H into (u + v, (u - v) w_2H^(k mod H)).  Three consecutive stages
-// only mix the 8 elements {b 2H0 + j + t h : t < 8} (h = H0 / 4), so each round of three stages
-// runs in registers: one shared-memory load and store per element per round instead of one per
-// stage, and the first round reads global memory directly (natural order: coalesced).  The last
-// step gathers X[k] = a[rev(k)].  Slots are swizzled (low four bits XOR bits 4..7 and 8..11) and
-// transforms sit 8 slots apart, which makes the rounds' and the gather's 64-bit accesses free of
-// bank conflicts for m = 4096.
-__device__ __forceinline__ uint32_t slot(uint32_t q) { return q ^ ((q >> 4) & 15u) ^ ((q >> 8) & 15u); }
-
-// LAST: the round ending at half size 1, where every unit has j = 0 and the twiddle of a pair
-// whose position within the half is 0 is 1 (7 of the 12 of a radix-8 round): no product there.
-template <int R, bool LAST>
-__device__ __forceinline__ void dif_unit(uint64_t (&x)[8], uint32_t j, uint32_t log_hmin,
-                                         uint32_t log_m, const uint64_t *tw) {
+template <int T, int LC, int TWIST>
+GL_FN void pass_store(const NttPass &ps, const uint64_t *tws, uint32_t gl, uint32_t gh, uint32_t v, uint32_t vstep,
+                      uint64_t base, const gl3 (&x)[T]) {
+  const uint32_t at = gl * ps.out_c + gh * ps.out_h + v * ps.out_k, step = vstep * ps.out_k;
 #pragma unroll
-  for (int l = 0; l < R; l++) {
-    const int d = 1 << (R - 1 - l);                    // partner distance within the unit
-    const uint32_t log_h = log_hmin + (R - 1 - l);     // this stage's half size
-#pragma unroll
-    for (int t = 0; t < (1 << R); t++) {
-      if (t & d) continue;
-      const uint64_t u = x[t], v = x[t + d];
-      x[t] = gl_add(u, v);
-      if (LAST && (t & (d - 1)) == 0) {
-        x[t + d] = gl_sub(u, v);
-      } else {
-        const uint32_t jp = j + ((uint32_t)(t & (d - 1)) << log_hmin);  // position within the half
-        const uint64_t w = tw[jp << (log_m - 1 - log_h)];              // w_2H^jp = w_m^(jp m / 2H)
-        x[t + d] = gl_mul(gl_sub(u, v), w);
-      }
-    }
-  }
-}
-
-// One round of R stages over every unit of the block's transforms; the first round reads the
-// transforms from global memory (natural order), the others from shared memory.
-template <int R, bool LAST>
-__device__ __forceinline__ void dif_round(const NttPass &ps, uint64_t *sm, uint32_t pitch,
-                                          const uint64_t *tw, uint32_t log_hmin, bool from_global) {
-  const uint32_t m = 1u << ps.log_m, C = ps.cols, units = m >> R;
-  const uint64_t g0 = (uint64_t)blockIdx.x * C;
-  const bool c_fast = from_global && ps.in_c == 1;  // consecutive lanes on consecutive transforms
-  // q0 holds no bit of t << log_hmin, so q = q0 ^ (t << log_hmin), and the swizzle is linear over
-  // XOR: slot(q) = slot(q0) ^ slot(t << log_hmin), the second term fixed for the round
-  uint32_t st[1 << R];
-#pragma unroll
-  for (int t = 0; t < (1 << R); t++) st[t] = slot((uint32_t)t << log_hmin);
-  for (uint32_t w = threadIdx.x; w < C * units; w += blockDim.x) {
-    const uint32_t c = c_fast ? w & (C - 1) : w >> (ps.log_m - R);
-    const uint32_t u = c_fast ? w >> ps.log_cols : w & (units - 1);
-    const uint32_t j = u & ((1u << log_hmin) - 1), b = u >> log_hmin;
-    const uint32_t q0 = (b << (log_hmin + R)) + j;
-    const uint32_t s0 = slot(q0);
-    uint64_t x[8];
-    uint64_t *a = sm + (size_t)c * pitch;
-#pragma unroll
-    for (int t = 0; t < (1 << R); t++) {
-      if (from_global) {
-        const uint32_t q = q0 + ((uint32_t)t << log_hmin);
-        uint64_t v = __ldcs(ps.src + (g0 + c) * ps.in_c + (uint64_t)q * ps.in_i);
-        x[t] = v >= GL_P ? v - GL_P : v;  // inputs are taken modulo p
-      } else {
-        x[t] = a[s0 ^ st[t]];
-      }
-    }
-    dif_unit<R, LAST>(x, j, log_hmin, ps.log_m, tw);
-#pragma unroll
-    for (int t = 0; t < (1 << R); t++) a[s0 ^ st[t]] = x[t];
-  }
-}
-
-__global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass8(NttPass ps) {
-  extern __shared__ uint64_t sm[];
-  const uint32_t m = 1u << ps.log_m, C = ps.cols, half = m >> 1, pitch = m + 8;
-  uint64_t *tw = sm + (size_t)C * pitch;
-  const uint64_t g0 = (uint64_t)blockIdx.x * C;
-  for (uint32_t j = threadIdx.x; j < half; j += blockDim.x) tw[j] = ps.tw_m[j];
-  __syncthreads();
-  int log_h0 = (int)ps.log_m - 1;  // half size of the next stage
-  bool first = true;
-  while (log_h0 >= 0) {
-    const int r = log_h0 + 1 >= 3 ? 3 : log_h0 + 1;
-    const uint32_t log_hmin = (uint32_t)(log_h0 - (r - 1));
-    if (log_hmin == 0) {  // the last round
-      if (r == 3) dif_round<3, true>(ps, sm, pitch, tw, 0, first);
-      else if (r == 2) dif_round<2, true>(ps, sm, pitch, tw, 0, first);
-      else dif_round<1, true>(ps, sm, pitch, tw, 0, first);
+  for (int t = 0; t < T; t++) {
+    uint64_t y = gl3_fold(x[t]);
+    if (TWIST == TW_TABLE) y = gl_mul(y, *at_of(ps.tw, t * vstep * ps.t_k, v * ps.t_k + gl * ps.t_g));
+    else if (TWIST == TW_SHARED) y = gl_mul(y, tws[v + t * vstep]);
+    else if (TWIST == TW_STEPS) y = gl_mul(y, t ? gl_mul(base, tws[(t << LC) + (gl & ((1 << LC) - 1))]) : base);
+    else if (ps.scale) y = gl_mul(y, ps.scale);
+    else y = gl_canon(y);
+    uint64_t *o;
+    if (TWIST == TW_NONE && ps.reverse) {  // the inverse transform is the forward one read backwards
+      o = ps.dst + ((0u - (at + t * step)) & ps.o_mask);
     } else {
-      if (r == 3) dif_round<3, false>(ps, sm, pitch, tw, log_hmin, first);
-      else if (r == 2) dif_round<2, false>(ps, sm, pitch, tw, log_hmin, first);
-      else dif_round<1, false>(ps, sm, pitch, tw, log_hmin, first);
+      o = const_cast<uint64_t *>(at_of(ps.dst, t * step, at));
     }
-    __syncthreads();
-    first = false;
-    log_h0 -= r;
-  }
-  if (first) {  // m = 1: no stage, the value itself
-    for (uint32_t c = threadIdx.x; c < C; c += blockDim.x) {
-      const uint64_t v = __ldcs(ps.src + (g0 + c) * ps.in_c);
-      sm[(size_t)c * pitch] = v >= GL_P ? v - GL_P : v;
-    }
-    __syncthreads();
-  }
-  // gather in natural order, output groups of C consecutive transforms together
-  for (uint32_t t = threadIdx.x; t < C * m; t += blockDim.x) {
-    const uint32_t c = t & (C - 1), k = t >> ps.log_cols;
-    uint64_t v = sm[(size_t)c * pitch + slot(bit_reverse(k, ps.log_m))];
-    if (ps.n_mask) {
-      const uint64_t e = ((g0 + c) * (uint64_t)k) & ps.n_mask;
-      v = gl_mul(v, gl_mul(ps.tw_hi[e >> 12], ps.tw_lo[e & 4095]));
-    } else if (ps.scale) {
-      v = gl_mul(v, ps.scale);
-    }
-    __stcs(ps.dst + (g0 + c) * ps.out_c + (uint64_t)k * ps.out_k, v);
+    gl_stcs(o, y);
   }
 }
 
+template <int L1, int L2, int LC, bool ROWS, int TWIST>
+GL_FN void pass_round1(const NttPass &ps, uint64_t *sm, uint32_t block, uint32_t tid, uint32_t threads) {
+  using S = PassShape<L1, L2, LC>;
+  constexpr int T = 1 << L1;
+  for (uint32_t w = tid; w < ((uint32_t)S::U << LC); w += threads) {
+    const uint32_t c = ROWS ? w >> L2 : w & (S::C - 1), u = ROWS ? w & (S::U - 1) : w >> LC;
+    const uint32_t g = block * S::C + c, gl = g & ps.gl_mask, gh = g >> ps.log_gl;
+    const uint32_t at = gl * ps.in_c + gh * ps.in_h + u * ps.in_i, step = S::U * ps.in_i;
+    gl3 x[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) x[t] = gl3_from(gl_ldcs(at_of(ps.src, t * step, at)));
+    if (L1 > 0) {
+      x[0] = gl3_biased(x[0]);
+      gl_dft<L1>(x);
+    }
+    if (L2 == 0) {
+      pass_store<T, LC, TWIST>(ps, nullptr, gl, gh, 0, 1, 0, x);
+    } else {
+      uint64_t *s = sm + (ROWS ? c * (S::U + 1) + u : w);
+#pragma unroll
+      for (int k = 0; k < T; k++) {
+        uint64_t y = gl3_fold(x[k]);
+        if (k) y = gl_mul(y, ps.tw1[k * S::U + u]);
+        s[k * S::PITCH] = y;
+      }
+    }
+  }
+}
+
+template <int L1, int L2, int LC, bool ROWS, int TWIST>
+GL_FN void pass_round2(const NttPass &ps, const uint64_t *sm, uint32_t block, uint32_t tid, uint32_t threads) {
+  using S = PassShape<L1, L2, LC>;
+  constexpr int T = 1 << L2;
+  for (uint32_t w = tid; w < (1u << (L1 + LC)); w += threads) {
+    const uint32_t c = w & (S::C - 1), k0 = w >> LC;
+    const uint32_t g = block * S::C + c, gl = g & ps.gl_mask, gh = g >> ps.log_gl;
+    const uint64_t *s = sm + k0 * S::PITCH + c * (ROWS ? S::U + 1 : 1);
+    uint64_t base = 0;
+    if (TWIST == TW_STEPS) base = gl_mul(ps.tw_a[g], ps.tw[k0 * ps.t_k + gl]);
+    gl3 x[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) x[t] = gl3_from(s[t * (ROWS ? 1 : S::C)]);
+    x[0] = gl3_biased(x[0]);
+    gl_dft<L2>(x);
+    pass_store<T, LC, TWIST>(ps, sm + (S::PITCH << L1), gl, gh, k0, 1u << L1, base, x);
+  }
+}
+
+template <int L1, int L2, int LC, bool ROWS, int TWIST>
+__global__ void __launch_bounds__(PassShape<L1, L2, LC>::THREADS, PassShape<L1, L2, LC>::THREADS == 128 ? 6 : 1)
+    k_ntt_pass(const NttPass ps) {
+  using S = PassShape<L1, L2, LC>;
+  extern __shared__ __align__(16) uint64_t sm[];
+  if constexpr (L2 > 0 && TWIST != TW_NONE)
+    pass_stage_twist<L1, L2, LC, TWIST>(ps, sm + (S::PITCH << L1), blockIdx.x, threadIdx.x, blockDim.x);
+  // launched while the kernel ahead of it in the stream drains (see enqueue_ntt): from here on that
+  // kernel's results are there, and the one behind may be set up
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  pass_round1<L1, L2, LC, ROWS, TWIST>(ps, sm, blockIdx.x, threadIdx.x, blockDim.x);
+  if constexpr (L2 > 0) {
+#ifdef __CUDA_ARCH__
+    if (TWIST != TW_NONE) asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+    __syncthreads();
+    pass_round2<L1, L2, LC, ROWS, TWIST>(ps, sm, blockIdx.x, threadIdx.x, blockDim.x);
+  }
+}
+
+// The rounds (L1, L2) of a pass of 2^log_m points.
+struct Rounds { int l1, l2; };
+constexpr Rounds kRounds[NTT_ONE_PASS + 1] = {{0, 0}, {1, 0}, {2, 0}, {3, 0}, {2, 2},
+                                              {3, 2}, {3, 3}, {4, 3}, {4, 4}};
+
+struct PassKernel {
+  void (*fn)(const NttPass);
+  uint32_t threads;
+  size_t smem;
+};
+template <int LM, int LC, bool ROWS, int TWIST>
+PassKernel pass_kernel() {
+  using S = PassShape<kRounds[LM].l1, kRounds[LM].l2, LC>;
+  return {k_ntt_pass<kRounds[LM].l1, kRounds[LM].l2, LC, ROWS, TWIST>, (uint32_t)S::THREADS, S::SMEM};
+}
+// the whole transform as one block
+PassKernel whole_kernel(uint32_t log_m) {
+  switch (log_m) {
+    case 0: return pass_kernel<0, 0, true, TW_NONE>();
+    case 1: return pass_kernel<1, 0, true, TW_NONE>();
+    case 2: return pass_kernel<2, 0, true, TW_NONE>();
+    case 3: return pass_kernel<3, 0, true, TW_NONE>();
+    case 4: return pass_kernel<4, 0, true, TW_NONE>();
+    case 5: return pass_kernel<5, 0, true, TW_NONE>();
+    case 6: return pass_kernel<6, 0, true, TW_NONE>();
+    case 7: return pass_kernel<7, 0, true, TW_NONE>();
+    default: return pass_kernel<8, 0, true, TW_NONE>();
+  }
+}
+// a pass of a split transform (2^4 to 2^8 points, at least 2^4 transforms)
+template <bool ROWS, int TWIST>
+PassKernel split_kernel(uint32_t log_m) {
+  if constexpr (TWIST == TW_TABLE) {  // the first of two passes: 2^5 or 2^6 points
+    return log_m == 5 ? pass_kernel<5, NTT_LOG_COLS, ROWS, TWIST>() : pass_kernel<6, NTT_LOG_COLS, ROWS, TWIST>();
+  } else {
+    switch (log_m) {
+      case 4: return pass_kernel<4, NTT_LOG_COLS, ROWS, TWIST>();
+      case 5: return pass_kernel<5, NTT_LOG_COLS, ROWS, TWIST>();
+      case 6: return pass_kernel<6, NTT_LOG_COLS, ROWS, TWIST>();
+      case 7: return pass_kernel<7, NTT_LOG_COLS, ROWS, TWIST>();
+      default: return pass_kernel<8, NTT_LOG_COLS, ROWS, TWIST>();
+    }
+  }
+}
+
+// Table set-up: out[i] = s w^(k j) for i = (k, j), j its low log_j bits, from s and the squares
+// w^(2^b) in gl_mul's table form; the entries get that form too.
+struct TableSpec {
+  uint64_t *out;
+  uint64_t n, s;
+  uint32_t log_j;
+  uint64_t sq[NTT_MAX_LOG_N];
+};
+__global__ void __launch_bounds__(256) k_ntt_table(const TableSpec ts) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ts.n) return;
+  const uint32_t j = (uint32_t)i & ((1u << ts.log_j) - 1);
+  const uint32_t e = j * (uint32_t)(i >> ts.log_j);
+  uint64_t r = ts.s;
+#pragma unroll
+  for (int b = 0; b < (int)NTT_MAX_LOG_N; b++)
+    if ((e >> b) & 1u) r = gl_mul(r, ts.sq[b]);
+  ts.out[i] = r;
+}
+
+constexpr uint64_t kMontSq = 0xfffffffe00000001ull;  // 2^128 modulo p
 // self-test hook: element-wise a op b (0 add, 1 sub, 2 mul)
 __global__ void k_gl_test(int op, const uint64_t *a, const uint64_t *b, uint64_t *out, uint64_t n) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = op == 0 ? gl_add(a[i], b[i]) : op == 1 ? gl_sub(a[i], b[i]) : gl_mul(a[i], b[i]);
+  const gl3 x = gl3_from(a[i]), y = gl3_from(b[i]);
+  out[i] = gl_canon(op == 0   ? gl3_fold(gl3_add(x, y))
+                    : op == 1 ? gl3_fold(gl3_biased(gl3_sub(x, y)))
+                              : gl_mul(gl_mul(a[i], gl_canon(b[i])), kMontSq));
 }
 
 // Linear copy of n values in 16-byte vectors; the source may be host memory that the device
@@ -343,16 +363,20 @@ int fail(int code, const char *fmt, ...) {
 
 struct NttCtx {
   int device = 0;
-  uint32_t log_n = 0, log_n1 = 0, log_n2 = 0, cols = 4;
+  uint32_t log_n = 0;
   uint64_t n = 0;
-  uint64_t *d_in = nullptr, *d_out = nullptr, *d_tmp = nullptr;
-  uint64_t *d_tw1 = nullptr, *d_tw2 = nullptr, *d_twlo = nullptr, *d_twhi = nullptr;
+  uint64_t *d_in = nullptr, *d_out = nullptr, *d_tmp = nullptr, *d_tab = nullptr;
+  // the passes in order; the first reads the input, the last writes the output, the rest d_tmp
+  struct Pass {
+    PassKernel k;
+    NttPass ps;
+    uint32_t blocks;
+  } pass[3] = {};
+  int n_pass = 0;
   // the device reads pageable host memory through the host's page tables: the input vector
   // moves by a copy kernel instead of a driver copy
   bool host_direct = false;
-  bool radix2 = false;  // the radix-2 pass kernel (comparison)
-  bool inverse = false;   // roots w^-1 and outputs times 1/n
-  uint64_t scale_single = 0;  // 1/n for an inverse of one pass (the twist carries it otherwise)
+  bool inverse = false;  // outputs in reverse order and times 1/n
   int num_sms = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t ev[5] = {};
@@ -363,7 +387,7 @@ struct NttCtx {
   cudaStream_t st_up = nullptr, st_down = nullptr;
   cudaEvent_t up_done[2] = {}, comp_done[2] = {}, down_done[2] = {};
   ~NttCtx() {
-    for (uint64_t *p : {d_in, d_out, d_tmp, d_tw1, d_tw2, d_twlo, d_twhi, d_in2, d_out2})
+    for (uint64_t *p : {d_in, d_out, d_tmp, d_tab, d_in2, d_out2})
       if (p) cudaFree(p);
     for (cudaEvent_t e : ev)
       if (e) cudaEventDestroy(e);
@@ -375,79 +399,130 @@ struct NttCtx {
   }
 };
 
-uint64_t h_pow(uint64_t b, uint64_t e) {
-  uint64_t r = 1;
-  for (; e; e >>= 1, b = h_mul(b, b))
-    if (e & 1) r = h_mul(r, b);
-  return r;
-}
-uint64_t h_inv(uint64_t a) { return h_pow(a, GL_P - 2); }  // Fermat; a != 0
-
-// the 2^k-th root the context transforms with: the reference's, or its inverse
-uint64_t ctx_root(const NttCtx *cx, uint32_t k) {
-  return cx->inverse ? h_inv(GL_OMEGA[k]) : GL_OMEGA[k];
-}
-
-// w^0 .. w^(count - 1)
-std::vector<uint64_t> powers(uint64_t w, uint64_t count) {
-  std::vector<uint64_t> v(std::max<uint64_t>(count, 1));
-  v[0] = 1;
-  for (uint64_t i = 1; i < count; i++) v[i] = h_mul(v[i - 1], w);
-  return v;
-}
-
-int upload(uint64_t **dst, const std::vector<uint64_t> &v) {
-  NCK(cudaMalloc(dst, v.size() * 8));
-  NCK(cudaMemcpy(*dst, v.data(), v.size() * 8, cudaMemcpyHostToDevice));
+// The passes of a transform of cx->n points and their tables, in one allocation.
+int plan_passes(NttCtx *cx) {
+  const uint32_t ln = cx->log_n;
+  // digits of the split, most significant first
+  uint32_t d[3] = {ln, 0, 0};
+  cx->n_pass = ln <= NTT_ONE_PASS ? 1 : ln <= NTT_TWO_PASS ? 2 : 3;
+  if (cx->n_pass == 2) {
+    d[1] = ln / 2;
+    d[0] = ln - d[1];
+  } else if (cx->n_pass == 3) {
+    d[2] = ln / 3;
+    d[1] = (ln - d[2]) / 2;
+    d[0] = ln - d[1] - d[2];
+  }
+  const uint32_t la = d[0], lb = d[1], lc = d[2];
+  const uint64_t inv_n = cx->inverse ? h_inv(cx->n % GL_P) : 1;
+  struct Table {
+    uint32_t log_k, log_j, log_root;  // 2^(log_k + log_j) entries s w^(k j), w of 2^log_root points
+    uint64_t s;
+  };
+  // round factors of each pass, then the twists
+  std::vector<Table> tabs;
+  for (int p = 0; p < cx->n_pass; p++)
+    tabs.push_back({(uint32_t)kRounds[d[p]].l1, (uint32_t)kRounds[d[p]].l2, d[p], 1});
+  if (cx->n_pass == 2) {
+    tabs.push_back({lb, la, ln, inv_n});  // w^(jb ka)
+  } else if (cx->n_pass == 3) {
+    tabs.push_back({lb, la, la + lb, 1});  // w_ab^(jb ka)
+    tabs.push_back({lb, lc, lb + lc, 1});  // w_bc^(kb jc)
+    tabs.push_back({la, lc, ln, inv_n});   // w^(ka jc)
+  }
+  std::vector<uint64_t> off;
+  uint64_t total = 0;
+  for (const Table &t : tabs) {
+    off.push_back(total);
+    total += 1ull << (t.log_k + t.log_j);
+  }
+  NCK(cudaMalloc(&cx->d_tab, total * 8));
+  for (size_t i = 0; i < tabs.size(); i++) {
+    const Table &t = tabs[i];
+    TableSpec ts{};
+    ts.out = cx->d_tab + off[i];
+    ts.n = 1ull << (t.log_k + t.log_j);
+    ts.s = h_mont(t.s);
+    ts.log_j = t.log_j;
+    uint64_t w = GL_OMEGA[t.log_root];
+    for (uint32_t b = 0; b < NTT_MAX_LOG_N; b++, w = h_mul(w, w)) ts.sq[b] = h_mont(w);
+    k_ntt_table<<<(unsigned)((ts.n + 255) / 256), 256, 0, cx->st>>>(ts);
+    NCK(cudaGetLastError());
+  }
+  const uint32_t a = 1u << la, b = 1u << lb, c = 1u << lc;
+  for (int p = 0; p < cx->n_pass; p++) {
+    NttPass &ps = cx->pass[p].ps;
+    ps.o_mask = (uint32_t)(cx->n - 1);
+    ps.log_gl = 31;
+    ps.gl_mask = 0x7fffffffu;
+    ps.tw1 = cx->d_tab + off[p];
+    const bool last = p + 1 == cx->n_pass;
+    ps.reverse = last && cx->inverse;
+    cx->pass[p].blocks = cx->n_pass == 1 ? 1 : (uint32_t)(cx->n >> (d[p] + NTT_LOG_COLS));
+    if (cx->n_pass == 1) {
+      cx->pass[p].k = whole_kernel(ln);
+      ps.in_i = ps.out_k = 1;
+      ps.scale = cx->inverse ? h_mont(inv_n) : 0;
+    } else if (p == 0) {
+      cx->pass[p].k = cx->n_pass == 2 ? split_kernel<false, TW_TABLE>(la) : split_kernel<false, TW_SHARED>(la);
+      ps.in_c = ps.out_c = 1;
+      ps.in_i = ps.out_k = b * c;
+      ps.tw = cx->d_tab + off[cx->n_pass];
+      ps.t_k = 1;
+      ps.t_g = a;
+      ps.t_shift = lc;
+    } else if (!last) {
+      cx->pass[p].k = split_kernel<false, TW_STEPS>(lb);
+      ps.log_gl = lc;
+      ps.gl_mask = c - 1;
+      ps.in_c = ps.out_c = 1;
+      ps.in_h = ps.out_h = b * c;
+      ps.in_i = ps.out_k = c;
+      ps.tw = cx->d_tab + off[4];
+      ps.tw_a = cx->d_tab + off[5];
+      ps.t_k = c;
+      ps.t_g = 1;
+    } else {
+      cx->pass[p].k = split_kernel<true, TW_NONE>(d[p]);
+      ps.log_gl = la;
+      ps.gl_mask = a - 1;
+      ps.in_c = b * c;
+      ps.in_h = c;
+      ps.in_i = 1;
+      ps.out_c = 1;
+      ps.out_h = a;
+      ps.out_k = a * b;
+      if (cx->n_pass == 2) ps.in_c = b, ps.in_h = 0, ps.out_h = 0, ps.out_k = a;
+    }
+    NCK(cudaFuncSetAttribute(cx->pass[p].k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cx->pass[p].k.smem));
+  }
+  NCK(cudaStreamSynchronize(cx->st));
   return 0;
 }
 
-size_t pass_smem(uint32_t log_m, uint32_t cols) {
-  return ((size_t)cols * ((1u << log_m) + 8) + (1u << log_m) / 2 + 1) * 8;
-}
-
-// one pass: `count` transforms of 2^log_m points, `cols` per block
-cudaError_t launch_pass(const NttCtx *cx, const uint64_t *src, uint64_t *dst, uint32_t log_m,
-                        uint64_t count, uint64_t in_c, uint64_t in_i, uint64_t out_c, uint64_t out_k,
-                        const uint64_t *tw_m, bool twist, cudaStream_t st, uint64_t scale = 0) {
-  NttPass ps;
-  ps.src = src;
-  ps.dst = dst;
-  ps.log_m = log_m;
-  ps.cols = (uint32_t)std::min<uint64_t>(cx->cols, count);  // powers of two
-  ps.log_cols = (uint32_t)__builtin_ctz(ps.cols);
-  ps.in_c = in_c;
-  ps.in_i = in_i;
-  ps.out_c = out_c;
-  ps.out_k = out_k;
-  ps.tw_m = tw_m;
-  ps.tw_lo = cx->d_twlo;
-  ps.tw_hi = cx->d_twhi;
-  ps.n_mask = twist ? cx->n - 1 : 0;
-  ps.scale = twist ? 0 : scale;
-  const uint32_t blocks = (uint32_t)(count / ps.cols);
-  const uint32_t threads = std::min<uint32_t>(NTT_THREADS, std::max<uint32_t>(32, ps.cols << (log_m - (log_m ? 1 : 0))));
-  if (cx->radix2)
-    k_ntt_pass<<<blocks, threads, pass_smem(log_m, ps.cols), st>>>(ps);
-  else
-    k_ntt_pass8<<<blocks, threads, pass_smem(log_m, ps.cols), st>>>(ps);
-  return cudaGetLastError();
-}
-
-// the transform of cx->n points from d_src to d_dst (device memory), enqueued on st
+// The transform of cx->n points from d_src to d_dst (device memory), enqueued on st.  Every pass is
+// a programmatic dependent launch: it may be set up while the kernel ahead of it in the stream
+// drains, and waits for that kernel's results itself before it reads the points
+// (griddepcontrol.wait).  Measured (us): 2^12 points 9.3 -> 5.3, 2^19 19.6 -> 12.7, 2^24 233.7 -> 226.5.
 int enqueue_ntt(NttCtx *cx, uint64_t *d_dst, const uint64_t *d_src, cudaStream_t st, bool marks) {
-  if (cx->log_n <= NTT_MAX_LOG_M) {
-    NCK(launch_pass(cx, d_src, d_dst, cx->log_n, 1, 0, 1, 0, 1, cx->d_tw1, false, st,
-                    cx->scale_single));
-    if (marks) NCK(cudaEventRecord(cx->ev[2], st));
-    return 0;
+  for (int p = 0; p < cx->n_pass; p++) {
+    NttPass ps = cx->pass[p].ps;
+    ps.src = p == 0 ? d_src : cx->d_tmp;
+    ps.dst = p + 1 == cx->n_pass ? d_dst : cx->d_tmp;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cx->pass[p].blocks);
+    cfg.blockDim = dim3(cx->pass[p].k.threads);
+    cfg.dynamicSmemBytes = cx->pass[p].k.smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    NCK(cudaLaunchKernelEx(&cfg, cx->pass[p].k.fn, (const NttPass)ps));
+    if (marks && p == 0) NCK(cudaEventRecord(cx->ev[2], st));
   }
-  const uint64_t n1 = 1ull << cx->log_n1, n2 = 1ull << cx->log_n2;
-  // pass A: n1 columns of n2 points (stride n1), twisted, to Z[k2][j1]
-  NCK(launch_pass(cx, d_src, cx->d_tmp, cx->log_n2, n1, 1, n1, 1, n1, cx->d_tw2, true, st));
-  if (marks) NCK(cudaEventRecord(cx->ev[2], st));
-  // pass B: n2 rows of n1 points, to X[k2 + n2 k1]
-  NCK(launch_pass(cx, cx->d_tmp, d_dst, cx->log_n1, n2, n1, 1, 1, n2, cx->d_tw1, false, st));
   return 0;
 }
 
@@ -470,22 +545,16 @@ namespace {
 // a context of either direction (ntt_init, ntt_init_inverse)
 void *ntt_create(uint32_t log_n, bool inverse) {
   g_err = 0;
-  if (log_n > 2 * NTT_MAX_LOG_M) {
-    fail(NTT_ERR_ARG, "ntt_init: 2^%u points is over the maximum of 2^%u", log_n, 2 * NTT_MAX_LOG_M);
+  if (log_n > NTT_MAX_LOG_N) {
+    fail(NTT_ERR_ARG, "ntt_init: 2^%u points is over the maximum of 2^%u", log_n, NTT_MAX_LOG_N);
     return nullptr;
   }
   auto *cx = new NttCtx();
   cx->inverse = inverse;
   const char *dev = getenv("MSM_DEVICE");
   cx->device = dev ? atoi(dev) : 0;
-  if (const char *c = getenv("NTT_COLS")) {  // transforms per block: 1, 2 or 4
-    const int v = atoi(c);
-    cx->cols = v >= 4 ? 4 : v >= 2 ? 2 : 1;
-  }
   cx->log_n = log_n;
   cx->n = 1ull << log_n;
-  cx->log_n2 = log_n / 2;
-  cx->log_n1 = log_n - cx->log_n2;
   int rc = 0;
   auto step = [&](cudaError_t e, const char *what) {
     if (!rc && e != cudaSuccess) rc = fail(NTT_ERR_CUDA, "ntt_init: %s: %s", what, cudaGetErrorString(e));
@@ -500,37 +569,10 @@ void *ntt_create(uint32_t log_n, bool inverse) {
   cx->host_direct = pageable && host_tables && !(hd && strcmp(hd, "0") == 0);
   step(cudaStreamCreateWithFlags(&cx->st, cudaStreamNonBlocking), "stream");
   for (auto &e : cx->ev) step(cudaEventCreate(&e), "event");
-  step(cudaFuncSetAttribute(k_ntt_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)pass_smem(NTT_MAX_LOG_M, 4)),
-       "shared memory size");
-  step(cudaFuncSetAttribute(k_ntt_pass8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)pass_smem(NTT_MAX_LOG_M, 4)),
-       "shared memory size");
-  if (const char *r2 = getenv("NTT_RADIX2")) cx->radix2 = strcmp(r2, "1") == 0;
   step(cudaMalloc(&cx->d_in, cx->n * 8), "input buffer");
   step(cudaMalloc(&cx->d_out, cx->n * 8), "output buffer");
-  if (log_n > NTT_MAX_LOG_M) step(cudaMalloc(&cx->d_tmp, cx->n * 8), "intermediate buffer");
-  if (!rc) {
-    // short-transform roots: w_m = w_n^(n/m), from the reference's table (inverted for the
-    // inverse transform)
-    const uint32_t l1 = log_n > NTT_MAX_LOG_M ? cx->log_n1 : log_n;
-    rc = upload(&cx->d_tw1, powers(ctx_root(cx, l1), (1ull << l1) / 2));
-    // the inverse's 1/n: in the twist of pass A (every entry of the high table), or in the
-    // store of a transform of one pass
-    const uint64_t inv_n = h_inv(cx->n % GL_P);
-    if (inverse && log_n <= NTT_MAX_LOG_M) cx->scale_single = inv_n;
-    if (!rc && log_n > NTT_MAX_LOG_M) {
-      rc = upload(&cx->d_tw2, powers(ctx_root(cx, cx->log_n2), (1ull << cx->log_n2) / 2));
-      const uint64_t w = ctx_root(cx, log_n);
-      if (!rc) rc = upload(&cx->d_twlo, powers(w, std::min<uint64_t>(cx->n, 4096)));
-      uint64_t w4096 = w;
-      for (int i = 0; i < 12; i++) w4096 = h_mul(w4096, w4096);
-      std::vector<uint64_t> hi = powers(w4096, std::max<uint64_t>(cx->n >> 12, 1));
-      if (inverse)
-        for (uint64_t &v : hi) v = h_mul(v, inv_n);
-      if (!rc) rc = upload(&cx->d_twhi, hi);
-    }
-  }
+  if (log_n > NTT_ONE_PASS) step(cudaMalloc(&cx->d_tmp, cx->n * 8), "intermediate buffer");
+  if (!rc) rc = plan_passes(cx);
   if (rc) {
     delete cx;
     return nullptr;
@@ -556,7 +598,7 @@ int ntt_evaluate_device(void *context, uint64_t *d_out, const uint64_t *d_in, vo
   g_err = 0;
   auto *cx = (NttCtx *)context;
   if (!cx || !d_out || !d_in) return fail(NTT_ERR_ARG, "ntt_evaluate_device: null argument");
-  if (d_out == d_in && cx->log_n <= NTT_MAX_LOG_M)
+  if (d_out == d_in && cx->log_n <= 12)
     return fail(NTT_ERR_ARG, "ntt_evaluate_device: the transform is out of place");
   NCK(cudaSetDevice(cx->device));
   return enqueue_ntt(cx, d_out, d_in, stream ? (cudaStream_t)stream : cx->st, false);
