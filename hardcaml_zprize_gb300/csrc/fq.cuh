@@ -6,8 +6,8 @@
 // below 2q without a final subtraction.  Addition/subtraction reduce by 2q.  fq_canon() brings a
 // value to [0, q) for comparisons and for the ABI.
 //
-// The multiplier is operand-scanning CIOS with 32 x 32 -> 64 wide multiplies: 12 + 11 limb
-// products per row (q's lowest limb is 1), 276 wide IMADs per product.  The algorithmic count for
+// The multiplier is operand-scanning CIOS with 32 x 32 + 64 -> 64 wide multiplies in carry chains:
+// 12 + 11 limb products per row (q's lowest limb is 1), 276 wide IMADs per product.  The algorithmic count for
 // the roofline stays 588 32-bit IMAD per product (lo and hi halves of 12 x 12 + 12 x 12).
 // The field is the one the reference computes in with GMP (host/msm_compute/include/
 // bls12_377_g1/bls12_377_g1.h:31-33, 90-219); the limb layout is new.
@@ -45,31 +45,6 @@ struct fq_t {
 };
 
 // ---- carry-chain primitives (one PTX instruction each; the carry flag lives between them) ----
-__device__ __forceinline__ uint32_t madlo_cc(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm volatile("mad.lo.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t madclo_cc(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm volatile("madc.lo.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t madhi_cc(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm volatile("mad.hi.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t madchi_cc(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm volatile("madc.hi.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t madchi(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm volatile("madc.hi.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
 __device__ __forceinline__ uint32_t add_cc(uint32_t a, uint32_t b) {
   uint32_t r;
   asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
@@ -120,66 +95,126 @@ __device__ __forceinline__ fq_t fq_one() {
 }
 
 // ---- a * b * 2^-384 mod q (CIOS; inputs and output in [0, 2q)) ----
-// Each row adds b_i * a and then m * q to the running value t, m = -t0 (q = 1 mod 2^32 and
-// -q^-1 = -1 mod 2^32, so the row factor needs no product and m * q0 + t0 = 0 with a carry of
-// (t0 != 0)).  The limb products are wide multiplies with no addend: a wide multiply whose 64-bit
-// addend is a 32-bit carry needs that carry moved into an aligned register pair with a zero high
-// half, and a carry folded in before the multiply needs an add-with-carry that the compiler puts
-// on the multiply pipe.  Instead each row sums four word vectors -- the products' low words, their
-// high words one word up, and the same two of m * q -- in four add.cc/addc.cc chains, which run on
-// the integer ALU pipe.  Per product (ncu, sm_103a): 276 wide multiplies and about 50 other
-// multiply-pipe instructions, against 276 and 336 for a 64-bit-accumulator CIOS; the two pipes
-// are then about equally busy.
-// Bound: at the start of a row t < 4q < 2^384 (so t[12] = 0) and no row sum leaves 13 words, for
-// any a < 2^383 and any b.
-__device__ __forceinline__ fq_t fq_mul(const fq_t &a, const fq_t &b) {
+// Row i adds b_i a and then m q to the running value and drops its lowest word, m = -t0 (q = 1 mod
+// 2^32 and -q^-1 = -1 mod 2^32, so the row factor needs no product and m q0 + t0 = 0 with a carry of
+// (t0 != 0)).  The running value is the sum of two word vectors on 64-bit lanes: E, words 0 to 11,
+// takes the products of the even words of a (and q), O, words 1 to 12, those of the odd ones.  All
+// lanes of a vector are one carry chain of mad.lo.cc / madc.hi.cc pairs, and ptxas makes each pair
+// one wide multiply with a 64-bit addend, carry in and carry out.  Dropping word 0 swaps the two
+// vectors' roles: O becomes the new E, the old E moves down two words and becomes the new O, and its
+// word 1 is added to the new E's word 0 on the way (that carry starts the new O's chain).
+//
+// The negation of t0 is written as ~t0 + 1: ptxas folds a plain negation into the products of m and
+// then splits each pair of that chain into a low and a high multiply (ncu opcode counts: 144 wide
+// multiplies and 132 pairs; with it written so, 276 wide multiplies, 42 + 31 carry adds, 12 LOP3,
+// 36 moves).  What bounds it is the multiply pipe: a wide multiply holds it four cycles, 1104 of
+// about 1195 cycles per warp-product.  Products/s on GB300 in a chain of products (mixed adds/s in
+// k_accumulate's loop): wide multiplies without addend and four carry chains per row, the form
+// before, 2.18e10 (3.01e9); this one with the pairs of m split 2.61e10 (3.61e9); this one 3.12e10
+// (4.25e9); 13 signed 30-bit limbs with 64-bit accumulators and no carry chains 2.46e10 (3.44e9).
+// Bound: at the start of a row t < 4q < 2^384, and no row sum leaves 13 words, for any a < 2^383
+// and any b; so O, which is at most the sum, has no carry out of its top word.
+struct fq_lanes {  // six 64-bit lanes
+  uint32_t w[FQ_LIMBS];
+};
+
+// x += sum over k of a[k] b at lane k, carry out added to top
+__device__ __forceinline__ void fq_chain(fq_lanes &x, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                         uint32_t a4, uint32_t a5, uint32_t b, uint32_t &top) {
+  asm("mad.lo.cc.u32 %0, %13, %19, %0;\n\tmadc.hi.cc.u32 %1, %13, %19, %1;\n\t"
+      "madc.lo.cc.u32 %2, %14, %19, %2;\n\tmadc.hi.cc.u32 %3, %14, %19, %3;\n\t"
+      "madc.lo.cc.u32 %4, %15, %19, %4;\n\tmadc.hi.cc.u32 %5, %15, %19, %5;\n\t"
+      "madc.lo.cc.u32 %6, %16, %19, %6;\n\tmadc.hi.cc.u32 %7, %16, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8, %17, %19, %8;\n\tmadc.hi.cc.u32 %9, %17, %19, %9;\n\t"
+      "madc.lo.cc.u32 %10, %18, %19, %10;\n\tmadc.hi.cc.u32 %11, %18, %19, %11;\n\t"
+      "addc.u32 %12, %12, 0;"
+      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
+        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11]), "+r"(top)
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b));
+}
+// the same without a carry out
+__device__ __forceinline__ void fq_chain_end(fq_lanes &x, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                             uint32_t a4, uint32_t a5, uint32_t b) {
+  asm("mad.lo.cc.u32 %0, %12, %18, %0;\n\tmadc.hi.cc.u32 %1, %12, %18, %1;\n\t"
+      "madc.lo.cc.u32 %2, %13, %18, %2;\n\tmadc.hi.cc.u32 %3, %13, %18, %3;\n\t"
+      "madc.lo.cc.u32 %4, %14, %18, %4;\n\tmadc.hi.cc.u32 %5, %14, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6, %15, %18, %6;\n\tmadc.hi.cc.u32 %7, %15, %18, %7;\n\t"
+      "madc.lo.cc.u32 %8, %16, %18, %8;\n\tmadc.hi.cc.u32 %9, %16, %18, %9;\n\t"
+      "madc.lo.cc.u32 %10, %17, %18, %10;\n\tmadc.hi.u32 %11, %17, %18, %11;"
+      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
+        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b));
+}
+// e0 += s, then lanes 0 to 4 of x and a new lane 5 (from zero) take the products, the sum's carry first
+__device__ __forceinline__ void fq_chain_shifted(fq_lanes &x, uint32_t &e0, uint32_t s, uint32_t a0, uint32_t a1,
+                                                 uint32_t a2, uint32_t a3, uint32_t a4, uint32_t a5, uint32_t b) {
+  asm("add.cc.u32 %12, %12, %20;\n\t"
+      "madc.lo.cc.u32 %0, %13, %19, %0;\n\tmadc.hi.cc.u32 %1, %13, %19, %1;\n\t"
+      "madc.lo.cc.u32 %2, %14, %19, %2;\n\tmadc.hi.cc.u32 %3, %14, %19, %3;\n\t"
+      "madc.lo.cc.u32 %4, %15, %19, %4;\n\tmadc.hi.cc.u32 %5, %15, %19, %5;\n\t"
+      "madc.lo.cc.u32 %6, %16, %19, %6;\n\tmadc.hi.cc.u32 %7, %16, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8, %17, %19, %8;\n\tmadc.hi.cc.u32 %9, %17, %19, %9;\n\t"
+      "madc.lo.cc.u32 %10, %18, %19, 0;\n\tmadc.hi.u32 %11, %18, %19, 0;"
+      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
+        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "=r"(x.w[10]), "=r"(x.w[11]), "+r"(e0)
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b), "r"(s));
+}
+// x += m (1 + sum over k >= 1 of a[k] 2^64k), word 0 becomes zero (m = -x.w[0]), carry out added to top
+__device__ __forceinline__ void fq_chain_reduce(fq_lanes &x, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t a4,
+                                                uint32_t a5, uint32_t m, uint32_t &top) {
+  asm("{\n\t.reg .u32 z;\n\tadd.cc.u32 z, %0, %18;\n\taddc.cc.u32 %1, %1, 0;\n\t"
+      "madc.lo.cc.u32 %2, %13, %18, %2;\n\tmadc.hi.cc.u32 %3, %13, %18, %3;\n\t"
+      "madc.lo.cc.u32 %4, %14, %18, %4;\n\tmadc.hi.cc.u32 %5, %14, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6, %15, %18, %6;\n\tmadc.hi.cc.u32 %7, %15, %18, %7;\n\t"
+      "madc.lo.cc.u32 %8, %16, %18, %8;\n\tmadc.hi.cc.u32 %9, %16, %18, %9;\n\t"
+      "madc.lo.cc.u32 %10, %17, %18, %10;\n\tmadc.hi.cc.u32 %11, %17, %18, %11;\n\t"
+      "addc.u32 %12, %12, 0;\n\t}"
+      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
+        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11]), "+r"(top)
+      : "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(m));
+}
+// -x, kept apart from the products that use it (see above)
+__device__ __forceinline__ uint32_t fq_row_factor(uint32_t x) {
+  uint32_t m;
+  asm("{\n\t.reg .u32 t;\n\tnot.b32 t, %1;\n\tadd.u32 %0, t, 1;\n\t}" : "=r"(m) : "r"(x));
+  return m;
+}
+
+__device__ __forceinline__ fq_t fq_mul(const fq_t &x, const fq_t &y) {
   const uint32_t q[FQ_LIMBS] = BLS_Q;
-  uint32_t t[FQ_LIMBS + 1];
+  const uint32_t *a = x.v;
+  fq_lanes E, O;
 #pragma unroll
   for (int i = 0; i < FQ_LIMBS; i++) {
-    const uint32_t bi = b.v[i];
-    uint32_t lo[FQ_LIMBS], hi[FQ_LIMBS];
-#pragma unroll
-    for (int j = 0; j < FQ_LIMBS; j++) {
-      const uint64_t p = (uint64_t)a.v[j] * bi;
-      lo[j] = (uint32_t)p;
-      hi[j] = (uint32_t)(p >> 32);
-    }
+    const uint32_t b = y.v[i];
     if (i == 0) {
 #pragma unroll
-      for (int j = 0; j < FQ_LIMBS; j++) t[j] = lo[j];
-      t[FQ_LIMBS] = 0;
+      for (int j = 0; j < FQ_LIMBS; j += 2) {
+        const uint64_t e = (uint64_t)a[j] * b, o = (uint64_t)a[j + 1] * b;
+        E.w[j] = (uint32_t)e;
+        E.w[j + 1] = (uint32_t)(e >> 32);
+        O.w[j] = (uint32_t)o;
+        O.w[j + 1] = (uint32_t)(o >> 32);
+      }
     } else {
-      t[0] = add_cc(t[0], lo[0]);
+      fq_lanes N;  // the old E, two words down
 #pragma unroll
-      for (int j = 1; j < FQ_LIMBS; j++) t[j] = addc_cc(t[j], lo[j]);
-      t[FQ_LIMBS] = addc(0u, 0u);
+      for (int k = 0; k < FQ_LIMBS - 2; k++) N.w[k] = E.w[k + 2];
+      const uint32_t s = E.w[1];
+      E = O;
+      fq_chain_shifted(N, E.w[0], s, a[1], a[3], a[5], a[7], a[9], a[11], b);
+      O = N;
+      fq_chain(E, a[0], a[2], a[4], a[6], a[8], a[10], b, O.w[11]);
     }
-    t[1] = add_cc(t[1], hi[0]);
-#pragma unroll
-    for (int j = 2; j < FQ_LIMBS; j++) t[j] = addc_cc(t[j], hi[j - 1]);
-    t[FQ_LIMBS] = addc(t[FQ_LIMBS], hi[FQ_LIMBS - 1]);
-    const uint32_t m = 0u - t[0];
-#pragma unroll
-    for (int j = 1; j < FQ_LIMBS; j++) {
-      const uint64_t p = (uint64_t)m * q[j];
-      lo[j] = (uint32_t)p;
-      hi[j] = (uint32_t)(p >> 32);
-    }
-    add_cc(t[0], m);  // t0 + m = 0 mod 2^32 with a carry of (t0 != 0)
-#pragma unroll
-    for (int j = 1; j < FQ_LIMBS; j++) t[j] = addc_cc(t[j], lo[j]);
-    t[FQ_LIMBS] = addc(t[FQ_LIMBS], 0u);
-    t[2] = add_cc(t[2], hi[1]);
-#pragma unroll
-    for (int j = 3; j < FQ_LIMBS; j++) t[j] = addc_cc(t[j], hi[j - 1]);
-    t[FQ_LIMBS] = addc(t[FQ_LIMBS], hi[FQ_LIMBS - 1]);
-#pragma unroll
-    for (int j = 0; j < FQ_LIMBS; j++) t[j] = t[j + 1];
+    const uint32_t m = fq_row_factor(E.w[0]);
+    fq_chain_end(O, q[1], q[3], q[5], q[7], q[9], q[11], m);
+    fq_chain_reduce(E, q[2], q[4], q[6], q[8], q[10], m, O.w[11]);
   }
-  fq_t r;
+  fq_t r;  // E without its zero word 0, plus O
+  r.v[0] = add_cc(O.w[0], E.w[1]);
 #pragma unroll
-  for (int j = 0; j < FQ_LIMBS; j++) r.v[j] = t[j];
+  for (int k = 1; k < FQ_LIMBS - 1; k++) r.v[k] = addc_cc(O.w[k], E.w[k + 1]);
+  r.v[FQ_LIMBS - 1] = addc(O.w[FQ_LIMBS - 1], 0u);
   return r;
 }
 
