@@ -83,6 +83,7 @@ struct PassBuffers {
   uint32_t n_classes;
   uint64_t n_bases;             // resident bases (bounds of every base index)
   uint32_t acc_blocks_per_sm;   // resident k_accumulate blocks per SM (0: 4, the whole SM)
+  uint32_t quads;               // 1: runs and split buckets summed by four lanes each
 
   const uint4 *scalars;         // 2 x uint4 per scalar
   const uint4 *host_scalars;    // or null: k_count first copies each scalar from this host buffer

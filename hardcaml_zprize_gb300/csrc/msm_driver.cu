@@ -220,6 +220,23 @@ uint32_t whole_bucket_run(double mean) {
   return s;
 }
 
+// A pass of at most this many entries sums each run with four lanes (k_accumulate_quad): it has too
+// few runs to fill the GPU with one thread each.
+constexpr uint64_t kQuadEntries = 1ull << 20;
+
+// Run length of such a pass: a run costs a quad two product latencies per entry, a split bucket a
+// merge kernel's passes over its parts, so buckets stay whole but for the upper tail: the smallest
+// power of two (at least 8) at or above 1.3 mean loads.  Measured on GB300 (ms per MSM on width-16
+// tables, runs of 8 / 16 / 32 / 64): 10000 points (mean 4.9) 0.407 / 0.416 / 0.421 / 0.422; 16384 (8)
+// 0.470 / 0.443 / 0.458 / 0.457; 25000 (12.2) 0.566 / 0.506 / 0.522 / 0.543; 50000 (24.4) 0.731 /
+// 0.704 / 0.665 / 0.681.  One thread per run at its best run length: 0.474, 0.524, 0.602, 0.738; at
+// 75000 points (1.2e6 entries) 0.838 against 0.816, at 2^17 1.113 against 1.154.
+uint32_t quad_run(double mean) {
+  uint32_t s = 8;
+  while (s < 1.3 * mean && s < 4096) s <<= 1;
+  return s;
+}
+
 // Longest run of entries one accumulate thread sums: whole buckets of `nwin_sharing` windows
 // but for the tail, and short enough that the n x nwin entries make at least ~2^17 runs: with
 // few, heavily loaded buckets (a fixed-base table of small width) whole-bucket runs would leave
@@ -232,6 +249,7 @@ uint32_t seg_len_for(uint64_t n, uint32_t nb, uint32_t nwin_sharing, uint32_t nw
   const double mean = (double)n * nwin_sharing / std::max<uint32_t>(nb, 1);
   const uint32_t s = whole_bucket_run(mean);
   const uint64_t entries = n * (uint64_t)nwin;
+  if (entries <= kQuadEntries) return quad_run(mean);
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 18) <= entries) cap <<= 1;  // entries / cap >= 2^17
   uint32_t r = std::min(s, cap);
@@ -305,6 +323,7 @@ uint32_t pass_seg_len(const std::vector<JobSpec> &specs) {
     mean = std::max(mean, load);
     entries += sp.n * entries_per_point(sp.cfg.c, sp.cfg.signed_digits);
   }
+  if (entries <= kQuadEntries) return quad_run(mean);
   const uint32_t seg = whole_bucket_run(mean);
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 19) <= entries) cap <<= 1;
@@ -564,6 +583,7 @@ PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void
   pb.n_special = cx->n_special;
   pb.n_classes = cx->n_classes;
   pb.n_bases = cx->npoints * (cx->fb_w + cx->fb2_w);
+  pb.quads = pl.max_entries <= kQuadEntries;
   pb.scalars = (const uint4 *)d_scalars;
   pb.jobs = ws.jobs.as<JobDesc>();
   pb.wins = ws.wins.as<WinDesc>();
@@ -2171,6 +2191,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.n_special = cx->n_special;
   pb.n_classes = cx->n_classes;
   pb.n_bases = cx->npoints * (cx->fb_w + cx->fb2_w);
+  pb.quads = entries <= kQuadEntries;
   pb.scalars = (const uint4 *)d_scalars;
   pb.jobs = (const JobDesc *)(s + o_jobs);
   pb.wins = (const WinDesc *)(s + o_wins);

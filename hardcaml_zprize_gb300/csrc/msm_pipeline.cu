@@ -8,7 +8,8 @@
 //                  without a stage)
 //   4. k_tasks     split every bucket into runs of <= seg_len entries (load balance under skew)
 //   5. k_accumulate persistent: each thread sums one run of bases into a partial bucket sum
-//                  (the run's first base taken as is, then a 7-product mixed add per base)
+//                  (the run's first base taken as is, then a 7-product mixed add per base);
+//                  k_accumulate_quad, k_merge_quad, k_reduce1_quad: four lanes a run, small passes
 //   6. k_merge_*   buckets split over several runs: sum of their partials (a thread, a warp or
 //                  a block per bucket, by the number of runs)
 //   7. k_reduce1   per run of buckets: running sum R and triangle sum A (pippenger.h:25-33),
@@ -914,6 +915,148 @@ static __device__ __noinline__ fq_t dq_add(fq_t p, fq_t q, uint32_t mask) {
   return pid ? q : qid ? p : r;
 }
 
+// ---------------------------------------------------------------------------------------------
+// 5-7 on quads, for passes too small to fill the GPU with one thread per run: their time is a chain
+// of product latencies (about 1 us each), so a run's additions are spread over four lanes: two
+// product latencies a mixed add instead of seven, two a general one instead of eight.
+// A quad costs eight products' work a mixed add for a thread's seven, and 48 shuffles, so passes
+// that fill the GPU keep the threads.  Measured on GB300 (one MSM, accumulate + merge, threads /
+// quads, us): 4096 points 117 / 50, 16384 192 / 112, 50000 409 / 307, 2^17 724 / 760; the rules are
+// kQuadEntries in the driver and kReduceQuadSegs below.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t dq_mask() { return 0xfu << (threadIdx.x & 28); }
+
+// This lane's operand of a mixed add of base `v` (index | sign << 31): (y-x)/2 on lane 0, d x y on 1,
+// (y+x)/2 on 2 (a negative digit swaps lanes 0 and 2); lane 3 multiplies Z by one.
+__device__ __forceinline__ fq_t dq_load_base(const uint4 *bases, uint32_t v) {
+  const int l = dq_lane();
+  if (l == 3) return fq_one();
+  const int part = l == 1 ? 2 : ((l == 2) != (v >> 31) ? 1 : 0);
+  fq_t r;
+  fq_load(r, bases + (size_t)(v & 0x7fffffffu) * 9 + part * 3);
+  return r;
+}
+
+// p + base (te_madd_staged on four lanes): A = (Y-X) b0, C = T b2, B = (Y+X) b1, D = Z, then
+// X3 = E F, T3 = E H, Y3 = G H, Z3 = F G.
+static __device__ __noinline__ fq_t dq_madd(fq_t p, fq_t b, bool neg, uint32_t mask) {
+  const int l = dq_lane();
+  const fq_t po = dq_xchg(p, 2, mask);
+  const fq_t m1 = l == 0 ? fq_sub_lazy(po, p) : l == 2 ? fq_add_lazy(p, po) : p;
+  const fq_t pr = fq_mul(m1, b);  // A, C, B, D on lanes 0..3
+  const fq_t o = dq_xchg(pr, 2, mask);
+  const fq_t lo = l < 2 ? pr : o, hi = l < 2 ? o : pr;
+  fq_t u = fq_sub_lazy(hi, lo), w = fq_add_lazy(hi, lo);  // E, H on lanes 0, 2; F, G on 1, 3
+  const bool swap = neg && (l & 1);                       // a negative digit negates C
+  const fq_t un = fq_select(swap, w, u);
+  w = fq_select(swap, u, w);
+  u = un;
+  const fq_t u1 = dq_xchg(u, 1, mask), w1 = dq_xchg(w, 1, mask);
+  return fq_mul(l == 1 ? u1 : l == 2 ? w1 : u, l == 0 ? u1 : l == 1 ? w1 : w);
+}
+
+// the point of base v itself: X = ypx - ymx (negated for a negative digit), Y = ypx + ymx, Z = 1, T = X Y
+__device__ __forceinline__ fq_t dq_from_base(const uint4 *bases, uint32_t v) {
+  const int l = dq_lane();
+  const uint4 *src = bases + (size_t)(v & 0x7fffffffu) * 9;
+  fq_t a, b;
+  fq_load(a, src);
+  fq_load(b, src + 3);
+  const fq_t x = (v >> 31) ? fq_sub(a, b) : fq_sub(b, a), y = fq_add(b, a);
+  const fq_t t = fq_mul(x, y);
+  return pick4(l, x, t, y, fq_one());
+}
+
+// One quad per run, the next base fetched while the current one is added.
+__global__ void __launch_bounds__(128, 4) k_accumulate_quad(PassBuffers pb) {
+  const uint32_t ntasks = pb.counters[CNT_TASKS];
+  if (pb.counters[CNT_ERROR]) return;
+  const uint32_t mask = dq_mask();
+  const uint32_t stride = gridDim.x * (blockDim.x / 4);
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; i < ntasks; i += stride) {
+    const uint32_t t = pb.order[i];
+    const Task tk = pb.tasks[t];
+    uint32_t v = pb.vals[tk.start];
+    if ((v & 0x7fffffffu) >= pb.n_bases) {  // cannot happen for a consistent sort; never read out of bounds
+      set_error(pb.counters, 5, v & 0x7fffffffu);
+      continue;
+    }
+    fq_t acc = dq_from_base(pb.bases, v);
+    if (tk.len > 1) {
+      v = pb.vals[tk.start + 1];
+      bool ok = (v & 0x7fffffffu) < pb.n_bases;
+      fq_t nb = ok ? dq_load_base(pb.bases, v) : fq_one();
+#pragma unroll 1
+      for (uint32_t e = 1; e < tk.len; e++) {
+        if (!ok) {
+          set_error(pb.counters, 5, v & 0x7fffffffu);
+          break;
+        }
+        const fq_t b = nb;
+        const bool neg = (v >> 31) != 0;
+        if (e + 1 < tk.len) {
+          v = pb.vals[tk.start + e + 1];
+          ok = (v & 0x7fffffffu) < pb.n_bases;
+          if (ok) nb = dq_load_base(pb.bases, v);
+        }
+        acc = dq_madd(acc, b, neg, mask);
+      }
+    }
+    dq_store(pb.partials + (size_t)t * 12, acc);
+  }
+}
+
+// k_merge_small with a quad per split bucket
+__global__ void __launch_bounds__(128) k_merge_quad(PassBuffers pb) {
+  if (pb.counters[CNT_ERROR]) return;
+  const uint32_t nheavy = pb.counters[CNT_HEAVY];
+  const uint32_t mask = dq_mask();
+  const uint32_t stride = gridDim.x * (blockDim.x / 4);
+  for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; h < nheavy; h += stride) {
+    const uint32_t b = pb.heavy[h];
+    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
+    if (nt > kMergeThreadMax) continue;
+    const uint32_t t0 = pb.taskoff[b];
+    fq_t acc = dq_load(pb.partials + (size_t)t0 * 12);
+#pragma unroll 1
+    for (uint32_t k = 1; k < nt; k++) acc = dq_add(acc, dq_load(pb.partials + (size_t)(t0 + k) * 12), mask);
+    dq_store(pb.partials + (size_t)t0 * 12, acc);
+  }
+}
+
+// k_reduce1 with a quad per run of buckets.  A + R right after the first live bucket, with an empty
+// one between, is a doubling: it is taken as one.
+__global__ void __launch_bounds__(128) k_reduce1_quad(PassBuffers pb) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  if (s >= pb.n_segs) return;
+  if (pb.counters[CNT_ERROR]) return;
+  const uint32_t mask = dq_mask();
+  const WinDesc wd = pb.wins[find_win(pb.wins, pb.n_wins, s)];
+  const uint32_t L = 1u << pb.red_len_log2;
+  const uint32_t lo = (s - wd.seg_begin) * L;
+  const uint32_t hi = min(lo + L, wd.nb);
+  fq_t R = dq_identity(), A = dq_identity();
+  bool live = false, a_is_r = false;
+#pragma unroll 1
+  for (uint32_t b = hi; b-- > lo;) {
+    const uint32_t gb = wd.bucket_begin + b;
+    const bool full = pb.count[gb] != 0;
+    if (full) {
+      const fq_t B = dq_load(pb.partials + (size_t)pb.taskoff[gb] * 12);
+      R = live ? dq_add(R, B, mask) : B;
+    }
+    if (full && !live) {
+      A = R;
+      live = a_is_r = true;
+    } else if (live) {
+      A = !full && a_is_r ? dq_dbl(R, mask) : dq_add(A, R, mask);
+      a_is_r = false;
+    }
+  }
+  dq_store(pb.seg_out + (size_t)s * 24, R);
+  dq_store(pb.seg_out + (size_t)s * 24 + 12, A);
+}
+
 constexpr int kRedThreads = 256;
 constexpr uint32_t kRedQuads = kRedThreads / 4;
 constexpr uint32_t kAllLanes = 0xffffffffu;
@@ -1251,6 +1394,13 @@ size_t msm_scan_tmp_words(uint32_t n_buckets) {
   return 2ull * ((n_buckets + kScanBlock - 1) / kScanBlock) + 2;
 }
 
+// Level-1 reductions of at most this many runs take a quad each (k_reduce1_quad): one thread each
+// would leave the GPU idle behind a chain of 8 products per addition.  Measured on GB300, 8192 runs
+// of 4 buckets (tables of width 16): 61 us with a thread per run, 31 to 37 us with a quad; 32768
+// runs (2^20 points) keep the threads, whose work is then bound by product throughput (0.35 ms for
+// 2^19 buckets, of 0.27 at the product rate).
+constexpr uint32_t kReduceQuadSegs = 16384;
+
 cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st, cudaEvent_t *ev,
                             const cudaEvent_t *chunk_ready, int nchunks, uint32_t *n_kernels) {
   cudaError_t e;
@@ -1315,10 +1465,17 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
     launched++;
   }
   mark(4);
-  k_accumulate<<<num_sms * (pb.acc_blocks_per_sm ? pb.acc_blocks_per_sm : 4), 128, 0, st>>>(pb);
+  const uint32_t acc_blocks = num_sms * (pb.acc_blocks_per_sm ? pb.acc_blocks_per_sm : 4);
+  if (pb.quads)
+    k_accumulate_quad<<<acc_blocks, 128, 0, st>>>(pb);
+  else
+    k_accumulate<<<acc_blocks, 128, 0, st>>>(pb);
   launched++;
   mark(5);
-  k_merge_small<<<num_sms * 4, 128, 0, st>>>(pb);
+  if (pb.quads)
+    k_merge_quad<<<num_sms * 4, 128, 0, st>>>(pb);
+  else
+    k_merge_small<<<num_sms * 4, 128, 0, st>>>(pb);
   launched++;
   k_merge<<<num_sms, 256, 0, st>>>(pb);
   launched++;
@@ -1326,7 +1483,10 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   launched++;
   mark(6);
   if (pb.n_segs > 0) {
-    k_reduce1<<<(pb.n_segs + 127) / 128, 128, 0, st>>>(pb);
+    if (pb.n_segs <= kReduceQuadSegs)
+      k_reduce1_quad<<<(pb.n_segs + 31) / 32, 128, 0, st>>>(pb);
+    else
+      k_reduce1<<<(pb.n_segs + 127) / 128, 128, 0, st>>>(pb);
     launched++;
   }
   mark(7);

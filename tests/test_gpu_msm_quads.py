@@ -1,0 +1,53 @@
+"""MSMs whose runs, split buckets and level-1 reduction are summed by four lanes each, and their
+neighbours on the other side of each rule, against the CPU oracle, byte for byte: the smallest sizes,
+both sides of the entry limit (2^20 entries at 17 per point on width-16 tables), both sides of the
+limit on level-1 runs (tables of width 18 and 19), mostly empty buckets, and the mix with repeated
+scalars, whose heavy buckets are split and merged."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(engine, ocpu, n, kind, seed):
+    pts = engine.generate_bases(seed, n)
+    sc = engine.generate_scalars(seed + 1, n, kind=kind, msm_index=3)
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        out = engine.multi_scalar_mult(ctx, pts, sc)
+    finally:
+        ctx.close()
+    assert np.array_equal(out[0], ocpu.msm(pts, sc))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 257, 5000, 61680, 61681])
+def test_entry_limit(engine, ocpu, n, kind):
+    run(engine, ocpu, n, kind, 40 + n % 97)
+
+
+@pytest.mark.parametrize("bits", [15, 18, 19])
+@pytest.mark.parametrize("n", [9, 3000])
+def test_level_one_limit(engine, ocpu, monkeypatch, n, bits):
+    monkeypatch.setenv("MSM_FIXED_BASE", str(bits))
+    run(engine, ocpu, n, 1, 7 * bits + n)
+
+
+@pytest.mark.parametrize("bits", [6, 13])
+def test_windowed(engine, ocpu, bits):
+    n = 4099
+    pts = engine.generate_bases(91, n)
+    sc = engine.generate_scalars(92, n, kind=1, msm_index=1)
+    sc[5] = 0
+    sc[7] = np.uint64(2**64 - 1)  # at or above r: 253 bits are used
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        out = ctx.mult(sc, window_bits=bits, fixed_base=2)
+    finally:
+        ctx.close()
+    ref = engine.multi_scalar_mult_init(pts)
+    try:
+        want = engine.multi_scalar_mult(ref, pts, sc)
+    finally:
+        ref.close()
+    assert np.array_equal(out, want)
