@@ -25,11 +25,24 @@
 #include "engine.h"
 #include "curve.cuh"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanBlock = kScanThreads * kScanItems;
+
+// Start of every kernel of a pass.  They are programmatic dependent launches: a kernel may be set up
+// while the one ahead of it in the stream drains, and waits here for that one's completion (and so
+// for all before it).  pdl_begin also lets the next kernel be set up from here on; k_accumulate
+// calls pdl_wait alone: its blocks hold the SMs for the whole kernel, and blocks waiting beside them
+// would take the space that a server leaves for its other passes.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  asm volatile("griddepcontrol.launch_dependents;");
+}
 
 __device__ __forceinline__ void set_error(uint32_t *counters, uint32_t code, uint32_t info) {
   if (atomicCAS(&counters[CNT_ERROR], 0u, code) == 0u) counters[CNT_ERROR_INFO] = info;
@@ -98,6 +111,15 @@ __device__ __forceinline__ uint32_t bucket_key(const JobDesc &jd, uint32_t w, ui
 // window, nb_top and the excess (at most nb_top: the cap is at least half of 2^c_top).
 __device__ __forceinline__ uint32_t top_excess(const JobDesc &jd, uint32_t w, uint32_t mag) {
   return (w + 1 == jd.nwin && mag > jd.nb_top) ? mag - jd.nb_top : 0u;
+}
+
+// the counts, counters and run-length histogram of a pass to zero
+__global__ void __launch_bounds__(256) k_clear(PassBuffers pb) {
+  pdl_begin();
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+  for (uint32_t i = i0; i < pb.n_buckets; i += n) pb.count[i] = 0;
+  for (uint32_t i = i0; i <= pb.seg_len; i += n) pb.len_hist[i] = 0;
+  if (i0 < CNT_WORDS) pb.counters[i0] = 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -182,6 +204,7 @@ __device__ __forceinline__ void stage_digits(const PassBuffers &pb, const JobDes
 // stage, grouped by key range.
 __global__ void __launch_bounds__(MSM_POINTS_PER_CHUNK) k_count(PassBuffers pb, uint64_t g_begin,
                                                                 uint64_t g_end) {
+  pdl_begin();
   __shared__ uint32_t sh_cur[MSM_MAX_BINS];
   const uint32_t tid = threadIdx.x;
   const bool staged = pb.stage != nullptr;
@@ -276,6 +299,7 @@ __device__ __forceinline__ uint32_t ntask_of(uint32_t cnt, uint32_t seg_len) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(PassBuffers pb) {
+  pdl_begin();
   const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
   uint2 v = make_uint2(0, 0);
 #pragma unroll
@@ -295,6 +319,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(PassBuffers pb) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(PassBuffers pb, uint32_t nblk) {
+  pdl_begin();
   // one block: exclusive scan of the per-block totals, in chunks of kScanThreads
   __shared__ uint2 carry_sh;
   if (threadIdx.x == 0) carry_sh = make_uint2(0, 0);
@@ -323,6 +348,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(PassBuffers pb, ui
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
+  pdl_begin();
   const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
   uint32_t c[kScanItems];
   uint2 v = make_uint2(0, 0);
@@ -355,6 +381,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
 //    recomputes the digits and keeps only the entries in its range.
 // ---------------------------------------------------------------------------------------------
 __global__ void k_scatter(PassBuffers pb, uint32_t key_lo, uint32_t key_hi) {
+  pdl_begin();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= pb.n_points) return;
   if (pb.counters[CNT_ERROR]) return;
@@ -438,6 +465,7 @@ __global__ void k_scatter(PassBuffers pb, uint32_t key_lo, uint32_t key_hi) {
 // each to the position its bucket's slot cursor returns.  The range's slice of the sorted array
 // stays in L2 while the launch runs.
 __global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t bin) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint64_t chunk = blockIdx.x;
   const uint32_t *bo = pb.blk_off + chunk * (pb.n_bins + 1);
@@ -485,6 +513,7 @@ __global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t
 //    finishes a longer bucket; long runs also start first, which evens out the tail.
 // ---------------------------------------------------------------------------------------------
 __global__ void k_len_hist(PassBuffers pb) {
+  pdl_begin();
   extern __shared__ uint32_t h[];
   for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x) h[i] = 0;
   __syncthreads();
@@ -502,6 +531,7 @@ __global__ void k_len_hist(PassBuffers pb) {
 
 // cursor[len] = number of tasks longer than len (longest first); one thread, seg_len + 1 bins
 __global__ void k_len_scan(PassBuffers pb) {
+  pdl_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   uint32_t acc = 0;
   for (uint32_t l = pb.seg_len + 1; l-- > 0;) {
@@ -517,6 +547,7 @@ __global__ void k_len_scan(PassBuffers pb) {
 // bin's slots with one global atomic, so the few hot bin cursors (lengths cluster around the mean
 // bucket load) see one atomic per block and bin.
 __global__ void __launch_bounds__(256) k_tasks(PassBuffers pb) {
+  pdl_begin();
   extern __shared__ uint32_t sh_bins[];  // [seg_len + 1] counts, then [seg_len + 1] slot bases
   uint32_t *bin_cnt = sh_bins, *bin_base = sh_bins + pb.seg_len + 1;
   for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x) bin_cnt[i] = 0;
@@ -623,6 +654,7 @@ __device__ __forceinline__ xyzt_t te_from_staged(const uint4 *sh, bool neg) {
 }
 
 __global__ void __launch_bounds__(128, 4) k_accumulate(PassBuffers pb) {
+  pdl_wait();
   __shared__ uint4 sh[9 * 128];
   const int lane = threadIdx.x & 31;
   const uint32_t ntasks = pb.counters[CNT_TASKS];
@@ -688,6 +720,7 @@ __device__ __forceinline__ xyzt_t warp_sum_xyzt(xyzt_t acc) {
 constexpr uint32_t kMergeThreadMax = 16;
 
 __global__ void __launch_bounds__(128) k_merge_small(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t nheavy = pb.counters[CNT_HEAVY];
   for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < nheavy; h += gridDim.x * blockDim.x) {
@@ -711,6 +744,7 @@ __global__ void __launch_bounds__(128) k_merge_small(PassBuffers pb) {
 constexpr uint32_t kMergeWarpMax = 64;
 
 __global__ void __launch_bounds__(256) k_merge(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const int lane = threadIdx.x & 31;
   const uint32_t nheavy = pb.counters[CNT_HEAVY];
@@ -762,6 +796,7 @@ __device__ __forceinline__ uint32_t find_win_grp(const WinDesc *wins, uint32_t n
 }
 
 __global__ void __launch_bounds__(128) k_reduce1(PassBuffers pb) {
+  pdl_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= pb.n_segs) return;
   if (pb.counters[CNT_ERROR]) return;
@@ -969,6 +1004,7 @@ __device__ __forceinline__ fq_t dq_from_base(const uint4 *bases, uint32_t v) {
 
 // One quad per run, the next base fetched while the current one is added.
 __global__ void __launch_bounds__(128, 4) k_accumulate_quad(PassBuffers pb) {
+  pdl_begin();
   const uint32_t ntasks = pb.counters[CNT_TASKS];
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t mask = dq_mask();
@@ -1008,6 +1044,7 @@ __global__ void __launch_bounds__(128, 4) k_accumulate_quad(PassBuffers pb) {
 
 // k_merge_small with a quad per split bucket
 __global__ void __launch_bounds__(128) k_merge_quad(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t nheavy = pb.counters[CNT_HEAVY];
   const uint32_t mask = dq_mask();
@@ -1027,6 +1064,7 @@ __global__ void __launch_bounds__(128) k_merge_quad(PassBuffers pb) {
 // k_reduce1 with a quad per run of buckets.  A + R right after the first live bucket, with an empty
 // one between, is a doubling: it is taken as one.
 __global__ void __launch_bounds__(128) k_reduce1_quad(PassBuffers pb) {
+  pdl_begin();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (s >= pb.n_segs) return;
   if (pb.counters[CNT_ERROR]) return;
@@ -1170,6 +1208,7 @@ __device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log
 
 template <int NT>
 __global__ void __launch_bounds__(NT) k_reduce2(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t g = blockIdx.x;
   if (g >= pb.n_grps) return;
@@ -1195,6 +1234,7 @@ __global__ void __launch_bounds__(NT) k_reduce2(PassBuffers pb) {
 constexpr uint32_t kRed3SmallMax = 16;
 
 __global__ void __launch_bounds__(128) k_reduce3_small(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;  // one window per quad
   if (gw >= pb.n_wins) return;
@@ -1228,6 +1268,7 @@ __global__ void __launch_bounds__(128) k_reduce3_small(PassBuffers pb) {
 
 template <int NT>
 __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t gw = blockIdx.x;
   if (gw >= pb.n_wins) return;
@@ -1243,6 +1284,7 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
 // Buckets split into more than kMergeWarpMax runs: a block of 64 quads per bucket, each quad
 // summing a strided share of the partials, then a tree over the quads in shared memory.
 __global__ void __launch_bounds__(kRedThreads) k_merge_big(PassBuffers pb) {
+  pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   __shared__ uint4 sh[kRedQuads * 12];
   const uint32_t q = threadIdx.x >> 2;
@@ -1285,6 +1327,7 @@ __device__ __forceinline__ void load_class_point(wpt_t &p, const uint4 *cp) {
 }
 
 __global__ void __launch_bounds__(128) k_final(PassBuffers pb) {
+  pdl_begin();
   const uint32_t j = blockIdx.x;
   if (j >= pb.n_jobs) return;
   const JobDesc jd = pb.jobs[j];
@@ -1408,9 +1451,24 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   auto mark = [&](int k) {
     if (ev) cudaEventRecord(ev[k], st);
   };
-  if ((e = cudaMemsetAsync(pb.count, 0, (size_t)pb.n_buckets * 4, st))) return e;
-  if ((e = cudaMemsetAsync(pb.counters, 0, CNT_WORDS * 4, st))) return e;
-  if ((e = cudaMemsetAsync(pb.len_hist, 0, (size_t)(pb.seg_len + 1) * 4, st))) return e;
+  // one launch: kernel k on `grid` blocks, dependent on the one before it (see pdl_wait)
+  cudaError_t bad = cudaSuccess;
+  auto run = [&](auto k, uint32_t grid, uint32_t block, size_t smem, auto... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t r = cudaLaunchKernelEx(&cfg, k, args...);
+    if (r != cudaSuccess && bad == cudaSuccess) bad = r;
+    launched++;
+  };
+  run(k_clear, std::min<uint32_t>(num_sms * 8, pb.n_buckets / 1024 + 1), 256, 0, pb);
   mark(0);
   const uint32_t pts_blocks = (uint32_t)((pb.n_points + 255) / 256);
   if (pb.n_points > 0) {
@@ -1420,74 +1478,55 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
       for (int c = 0; c < nchunks; c++) {
         const uint64_t g0 = (uint64_t)c * per, g1 = g0 + per < pb.n_points ? g0 + per : pb.n_points;
         if ((e = cudaStreamWaitEvent(st, chunk_ready[c], 0))) return e;
-        if (g1 > g0) {
-          k_count<<<(uint32_t)((g1 - g0 + 255) / 256), 256, 0, st>>>(pb, g0, g1);
-          launched++;
-        }
+        if (g1 > g0) run(k_count, (uint32_t)((g1 - g0 + 255) / 256), 256, 0, pb, g0, g1);
       }
     } else {
-      k_count<<<pts_blocks, 256, 0, st>>>(pb, 0, pb.n_points);
-      launched++;
+      run(k_count, pts_blocks, 256, 0, pb, 0, pb.n_points);
     }
   }
   mark(1);
   const uint32_t nblk = (pb.n_buckets + kScanBlock - 1) / kScanBlock;
   if (nblk > 0) {
-    k_scan_reduce<<<nblk, kScanThreads, 0, st>>>(pb);
-    launched++;
-    k_scan_blocks<<<1, kScanThreads, 0, st>>>(pb, nblk);
-    launched++;
-    k_scan_apply<<<nblk, kScanThreads, 0, st>>>(pb);
-    launched++;
+    run(k_scan_reduce, nblk, kScanThreads, 0, pb);
+    run(k_scan_blocks, 1, kScanThreads, 0, pb, nblk);
+    run(k_scan_apply, nblk, kScanThreads, 0, pb);
   }
   mark(2);
   if (pb.n_points > 0 && pb.stage) {
-    for (uint32_t r = 0; r < pb.n_bins; r++) {
-      k_scatter_staged<<<pts_blocks, 256, 0, st>>>(pb, r);
-      launched++;
-    }
+    for (uint32_t r = 0; r < pb.n_bins; r++) run(k_scatter_staged, pts_blocks, 256, 0, pb, r);
   } else if (pb.n_points > 0) {
     const uint32_t passes = msm_scatter_passes(pb.max_entries);
     for (uint32_t p = 0; p < passes; p++) {
       const uint32_t lo = (uint32_t)((uint64_t)pb.n_buckets * p / passes);
       const uint32_t hi = (uint32_t)((uint64_t)pb.n_buckets * (p + 1) / passes);
-      k_scatter<<<pts_blocks, 256, 0, st>>>(pb, lo, hi);
-      launched++;
+      run(k_scatter, pts_blocks, 256, 0, pb, lo, hi);
     }
   }
   mark(3);
   if (pb.n_buckets > 0) {
-    k_len_hist<<<num_sms * 4, 256, (pb.seg_len + 1) * 4, st>>>(pb);
-    launched++;
-    k_len_scan<<<1, 32, 0, st>>>(pb);
-    launched++;
-    k_tasks<<<(pb.n_buckets + 255) / 256, 256, 2 * (pb.seg_len + 1) * 4, st>>>(pb);
-    launched++;
+    run(k_len_hist, num_sms * 4, 256, (pb.seg_len + 1) * 4, pb);
+    run(k_len_scan, 1, 32, 0, pb);
+    run(k_tasks, (pb.n_buckets + 255) / 256, 256, 2 * (pb.seg_len + 1) * 4, pb);
   }
   mark(4);
   const uint32_t acc_blocks = num_sms * (pb.acc_blocks_per_sm ? pb.acc_blocks_per_sm : 4);
   if (pb.quads)
-    k_accumulate_quad<<<acc_blocks, 128, 0, st>>>(pb);
+    run(k_accumulate_quad, acc_blocks, 128, 0, pb);
   else
-    k_accumulate<<<acc_blocks, 128, 0, st>>>(pb);
-  launched++;
+    run(k_accumulate, acc_blocks, 128, 0, pb);
   mark(5);
   if (pb.quads)
-    k_merge_quad<<<num_sms * 4, 128, 0, st>>>(pb);
+    run(k_merge_quad, num_sms * 4, 128, 0, pb);
   else
-    k_merge_small<<<num_sms * 4, 128, 0, st>>>(pb);
-  launched++;
-  k_merge<<<num_sms, 256, 0, st>>>(pb);
-  launched++;
-  k_merge_big<<<num_sms * 3, kRedThreads, 0, st>>>(pb);
-  launched++;
+    run(k_merge_small, num_sms * 4, 128, 0, pb);
+  run(k_merge, num_sms, 256, 0, pb);
+  run(k_merge_big, num_sms * 3, kRedThreads, 0, pb);
   mark(6);
   if (pb.n_segs > 0) {
     if (pb.n_segs <= kReduceQuadSegs)
-      k_reduce1_quad<<<(pb.n_segs + 31) / 32, 128, 0, st>>>(pb);
+      run(k_reduce1_quad, (pb.n_segs + 31) / 32, 128, 0, pb);
     else
-      k_reduce1<<<(pb.n_segs + 127) / 128, 128, 0, st>>>(pb);
-    launched++;
+      run(k_reduce1, (pb.n_segs + 127) / 128, 128, 0, pb);
   }
   mark(7);
   // Level 2 in blocks of 256 threads; level 3 (one block per window) in blocks of 128 while
@@ -1496,25 +1535,21 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   // against 0.107 / 0.123 / 0.154 / 0.206; level 2, groups of 512 runs at 2^20 / 2^24,
   // 0.188 / 0.268 against 0.214 / 0.348 (each quad then sums twice as many runs in sequence).
   if (pb.n_grps > 0) {
-    k_reduce2<256><<<pb.n_grps, 256, 0, st>>>(pb);
-    launched++;
+    run(k_reduce2<256>, pb.n_grps, 256, 0, pb);
   }
   mark(8);
   if (pb.n_wins > 0) {
-    k_reduce3_small<<<(pb.n_wins + 31) / 32, 128, 0, st>>>(pb);
-    launched++;
+    run(k_reduce3_small, (pb.n_wins + 31) / 32, 128, 0, pb);
     if (pb.n_wins <= (uint32_t)num_sms)
-      k_reduce3<128><<<pb.n_wins, 128, 0, st>>>(pb);
+      run(k_reduce3<128>, pb.n_wins, 128, 0, pb);
     else
-      k_reduce3<256><<<pb.n_wins, 256, 0, st>>>(pb);
-    launched++;
+      run(k_reduce3<256>, pb.n_wins, 256, 0, pb);
   }
   mark(9);
   if (pb.n_jobs > 0) {
-    k_final<<<pb.n_jobs, 128, 0, st>>>(pb);
-    launched++;
+    run(k_final, pb.n_jobs, 128, 0, pb);
   }
   mark(10);
   if (n_kernels) *n_kernels = launched;
-  return cudaGetLastError();
+  return bad != cudaSuccess ? bad : cudaGetLastError();
 }
