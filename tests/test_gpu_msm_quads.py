@@ -51,3 +51,25 @@ def test_windowed(engine, ocpu, bits):
     finally:
         ref.close()
     assert np.array_equal(out, want)
+
+
+@pytest.mark.parametrize("tables", ["0", "11", "16", "17"])
+@pytest.mark.parametrize("n", [1, 300, 20011, 65536])
+def test_noalloc_layouts(engine, ocpu, monkeypatch, n, tables):
+    """msm_mult_noalloc on tables of at most 16 bits and on windows where the context has none."""
+    import torch
+
+    monkeypatch.setenv("MSM_FIXED_BASE", tables)
+    pts = engine.generate_bases(71, n + 3)
+    sc = engine.generate_scalars(72, n, kind=1, msm_index=2)
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        d_sc = torch.from_numpy(sc.view(np.uint8).reshape(-1)).cuda()
+        d_out = torch.zeros(144, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(2):
+            ctx.mult_noalloc(n, 3, d_sc.data_ptr(), d_out.data_ptr())
+        torch.cuda.synchronize()
+    finally:
+        ctx.close()
+    assert np.array_equal(d_out.cpu().numpy(), ocpu.msm(pts[3:], sc))
