@@ -436,7 +436,7 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl) {
   // and the cursors 3.45 with ranges of 2^19 keys; 2^26 points (8.1e8) 16.5 against 14.0
   pl.ranks = pl.max_entries < (1ull << 27);
   pl.bin_shift =
-      msm_bin_shift(pl.n_buckets, pl.max_entries, sr ? (uint32_t)atoi(sr) : 0u, !pl.ranks);
+      msm_bin_shift(pl.n_buckets, pl.max_entries, sr ? (uint32_t)atoi(sr) : 0u, !pl.ranks, specs.size() > 1);
   pl.n_bins = pl.n_buckets ? ((pl.n_buckets - 1) >> pl.bin_shift) + 1 : 0;
   if (pl.n_bins > MSM_MAX_BINS) return fail(ERR_STATE, "too many key ranges: %u", pl.n_bins);
   snprintf(tmp, sizeof(tmp), "|r%u", pl.bin_shift);

@@ -1408,18 +1408,27 @@ uint32_t msm_scatter_passes(uint64_t max_entries) {
 }
 
 // Key ranges of the staged sort, as a shift of the bucket key (ranges of 2^shift keys, at most
-// MSM_MAX_BINS of them): one per ~150 MB of sorted array, and, for a scatter with slot cursors,
-// no more than 2^19 keys per range while that keeps MSM_MAX_BINS ranges or fewer.  The keys a
-// scatter launch touches bound its slot-cursor footprint: measured on GB300 at 2^24 points (4.9 M buckets), ranges of 2^20 keys
-// (5 launches) took 3.86 ms, 2^19 (10) 2.42 ms and 2^18 (19) 2.49 ms; 2^26 points use 2^18.
+// MSM_MAX_BINS of them).
+//   * Ranks (`cursors` false), one MSM: one range per ~16 MB of sorted array, at most ten.  Measured
+//     on GB300 (scatter, us, 1 / 4 / 8 / 16 ranges): 2^20 points (13.6e6 entries) 146 / 125 / 135 / 162,
+//     2^21 without tables (31e6) 520 / 311 / 288 / 298, 3e6 (39e6) 490 / 383 / 350 / 353.
+//   * Several MSMs (`many`): one range.  Each MSM's points and buckets are contiguous, so the blocks in
+//     flight stay within one or two MSMs' slices by themselves (the uneven mix of 64, 1.1e8 entries,
+//     1 / 2 / 4 / 8 / 16 ranges: 2.06 / 2.13 / 2.23 / 2.54 / 3.01 ms).
+//   * Slot cursors, one MSM: one per ~150 MB, and no more than 2^19 keys per range while that keeps MSM_MAX_BINS
+//     ranges or fewer.  The keys a scatter launch touches bound its slot-cursor footprint: 2^24 points
+//     (4.9 M buckets), ranges of 2^20 keys (5 launches) took 3.86 ms, 2^19 (10) 2.42 ms and 2^18 (19)
+//     2.49 ms; 2^26 points use 2^18.
 // `ranges` > 0 asks for that many ranges instead (rounded to a shift).
-uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool cursors) {
-  const uint64_t per = 150ull << 20;
-  const uint64_t want = ranges ? ranges : (max_entries * 4 + per / 2) / per;
+uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool cursors, bool many) {
+  const uint64_t per = cursors ? 150ull << 20 : 16ull << 20;
+  uint64_t want = ranges ? ranges : (max_entries * 4 + per / 2) / per;
+  if (!ranges && many) want = 1;
+  else if (!ranges && !cursors) want = std::min<uint64_t>(want, 10);
   const uint32_t target = (uint32_t)(want < 1 ? 1 : want > MSM_MAX_BINS ? MSM_MAX_BINS : want);
   uint32_t shift = 0;
   while (shift < 31 && (((uint64_t)n_buckets + (1ull << shift) - 1) >> shift) > target) shift++;
-  if (!ranges && cursors)
+  if (!ranges && cursors && !many)
     while (shift > 19 &&
            (((uint64_t)n_buckets + (1ull << (shift - 1)) - 1) >> (shift - 1)) <= MSM_MAX_BINS)
       shift--;
