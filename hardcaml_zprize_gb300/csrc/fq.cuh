@@ -18,9 +18,10 @@
 
 #define FQ_LIMBS 12
 
-// q and 2q, little-endian 32-bit limbs
+// q, 2q and 4q, little-endian 32-bit limbs
 #define BLS_Q {0x00000001u, 0x8508c000u, 0x30000000u, 0x170b5d44u, 0xba094800u, 0x1ef3622fu, 0x00f5138fu, 0x1a22d9f3u, 0x6ca1493bu, 0xc63b05c0u, 0x17c510eau, 0x01ae3a46u}
 #define BLS_Q2 {0x00000002u, 0x0a118000u, 0x60000001u, 0x2e16ba88u, 0x74129000u, 0x3de6c45fu, 0x01ea271eu, 0x3445b3e6u, 0xd9429276u, 0x8c760b80u, 0x2f8a21d5u, 0x035c748cu}
+#define BLS_Q4 {0x00000004u, 0x14230000u, 0xc0000002u, 0x5c2d7510u, 0xe8252000u, 0x7bcd88beu, 0x03d44e3cu, 0x688b67ccu, 0xb28524ecu, 0x18ec1701u, 0x5f1443abu, 0x06b8e918u}
 // -q^-1 mod 2^32 (q = 1 mod 2^46)
 #define BLS_QINV 0xffffffffu
 // Montgomery-form constants (value * 2^384 mod q)

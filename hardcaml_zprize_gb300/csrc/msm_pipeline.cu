@@ -868,21 +868,61 @@ __device__ __forceinline__ fq_t pick4(int l, const fq_t &a, const fq_t &b, const
   return fq_select(l == 0, a, fq_select(l == 1, b, fq_select(l == 2, c, d)));
 }
 
+// Sums that only feed products stay unreduced: a product of values below 8q is below
+// q + 64 q (q / 2^384) < 1.5 q, so nothing between two products needs a reduction (chains of 25 to
+// 37 dependent instructions each in a lone warp's latency).
+
+// base + term (neg 0), base - term + 2q (neg ~0), or base alone (en 0); term below 2q
+__device__ __forceinline__ fq_t fq_addsub(const fq_t &base, const fq_t &term, uint32_t en, uint32_t neg) {
+  const uint32_t q2[FQ_LIMBS] = BLS_Q2;
+  fq_t r;
+  add_cc(neg, neg);  // a carry in when negating
+#pragma unroll
+  for (int j = 0; j < FQ_LIMBS; j++) r.v[j] = addc_cc(base.v[j], (term.v[j] ^ neg) & en);
+  r.v[0] = add_cc(r.v[0], q2[0] & neg);
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS - 1; j++) r.v[j] = addc_cc(r.v[j], q2[j] & neg);
+  r.v[FQ_LIMBS - 1] = addc(r.v[FQ_LIMBS - 1], q2[FQ_LIMBS - 1] & neg);
+  return r;
+}
+// a - b + 4q, b below 4q
+__device__ __forceinline__ fq_t fq_sub_lazy4(const fq_t &a, const fq_t &b) {
+  const uint32_t q4[FQ_LIMBS] = BLS_Q4;
+  fq_t r;
+  r.v[0] = add_cc(a.v[0], q4[0]);
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = addc_cc(a.v[j], q4[j]);
+  r.v[0] = sub_cc(r.v[0], b.v[0]);
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS - 1; j++) r.v[j] = subc_cc(r.v[j], b.v[j]);
+  r.v[FQ_LIMBS - 1] = subc(r.v[FQ_LIMBS - 1], b.v[FQ_LIMBS - 1]);
+  return r;
+}
+// a 2^s, s = 0 or 1
+__device__ __forceinline__ fq_t fq_shl_lazy(const fq_t &a, uint32_t s) {
+  fq_t r;
+  r.v[0] = a.v[0] << s;
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = __funnelshift_l(a.v[j - 1], a.v[j], s);
+  return r;
+}
+
 // dbl-2008-hwcd, a = -1: A = X^2, B = Y^2, C = 2 Z^2, S = (X + Y)^2, E = S - A - B, G = B - A,
-// F = G - C, H = -A - B; X3 = E F, Y3 = G H, T3 = E H, Z3 = F G
+// F = G - C, H = -A - B; X3 = E F, Y3 = G H, T3 = E H, Z3 = F G.  (F and H change sign together
+// here, F' = A + C - B and H' = A + B, which changes the signs of all four coordinates.)
+// Every square is below 1.5q, so E < 5.5q, G < 3.5q, F' < 8q, H' < 3q.
 static __device__ __noinline__ fq_t dq_dbl(fq_t p, uint32_t mask) {
   const int l = dq_lane();
   const fq_t o1 = dq_xchg(p, 1, mask), o3 = dq_xchg(p, 3, mask);  // lane 1 gets X and Y
-  const fq_t sq = fq_sqr(l == 1 ? fq_add(o1, o3) : p);              // A, S, B, Z^2 on lanes 0..3
+  const fq_t sq = fq_sqr(l == 1 ? fq_add_lazy(o1, o3) : p);         // A, S, B, Z^2 on lanes 0..3
   const fq_t s1 = dq_xchg(sq, 1, mask), s2 = dq_xchg(sq, 2, mask), s3 = dq_xchg(sq, 3, mask);
   // the square of lane j sits in sq, s1, s2 or s3 as j ^ l is 0, 1, 2 or 3
   const fq_t A = pick4(l, sq, s1, s2, s3), S = pick4(l, s1, sq, s3, s2);
   const fq_t B = pick4(l, s2, s3, sq, s1), ZZ = pick4(l, s3, s2, s1, sq);
-  const fq_t C = fq_dbl(ZZ);
-  const fq_t E = fq_sub(fq_sub(S, A), B);
-  const fq_t G = fq_sub(B, A);
-  const fq_t F = fq_sub(G, C);
-  const fq_t H = fq_sub(fq_neg(A), B);
+  const fq_t H = fq_add_lazy(A, B);
+  const fq_t E = fq_sub_lazy4(S, H);
+  const fq_t G = fq_sub_lazy(B, A);
+  const fq_t F = fq_sub_lazy(fq_add_lazy(A, fq_shl_lazy(ZZ, 1)), B);
   return fq_mul(pick4(l, E, E, G, F), pick4(l, F, H, H, G));
 }
 
@@ -924,23 +964,13 @@ __device__ __forceinline__ bool dq_is_identity_bits(const fq_t &p, uint32_t mask
 // p + q by the dedicated formula (curve.cuh te_add_fast): two product latencies instead of three.
 //   lane 0: A = (Y1 - X1)(Y2 + X2), lane 2: B = (Y1 + X1)(Y2 - X2), lane 1: C = 2 Z1 T2,
 //   lane 3: D = 2 T1 Z2; then X3 = E F (lane 0), T3 = E H (1), Y3 = G H (2), Z3 = F G (3).
-// Where it gives Z3 = 0 the quad takes the unified formula; an operand that is the identity as
-// dq_identity() writes it (padding, empty runs) returns the other one unchanged.  Every lane of
-// `mask` calls this, and the branch to the unified formula is uniform over `mask`.
-static __device__ __noinline__ fq_t dq_add(fq_t p, fq_t q, uint32_t mask) {
-  const int l = dq_lane();
+// Where it gives Z3 = 0 the quad takes the unified formula, or, for an operand that is the identity as
+// dq_identity() writes it (padding, empty runs), the other one unchanged.  (Identity plus a point with
+// X Y != 0 is right as it comes.)  Z3 = 0 modulo q leaves 0 or q, whose lowest words are 0 and 1, so one
+// word tells whether to look closer.  Every lane of `mask` calls this, and the branches are uniform
+// over `mask`.
+static __device__ __noinline__ fq_t dq_add_rare(fq_t p, fq_t q, fq_t r, uint32_t mask) {
   const bool pid = dq_is_identity_bits(p, mask), qid = dq_is_identity_bits(q, mask);
-  const fq_t po = dq_xchg(p, 2, mask), qo = dq_xchg(q, 2, mask);  // X <-> Y on 0, 2; T <-> Z on 1, 3
-  const fq_t m1 = l == 0 ? fq_sub_lazy(po, p) : l == 2 ? fq_add_lazy(p, po) : po;
-  const fq_t m2 = l == 0 ? fq_add_lazy(qo, q) : l == 2 ? fq_sub_lazy(q, qo) : q;
-  fq_t pr = fq_mul(m1, m2);  // A, C' = Z1 T2, B, D' = T1 Z2 on lanes 0..3
-  if (l & 1) pr = fq_dbl(pr);
-  // pairs {0, 2}: F = B - A, G = B + A; pairs {1, 3}: H = D - C, E = D + C
-  const fq_t o = dq_xchg(pr, 2, mask);
-  const fq_t lo = l < 2 ? pr : o, hi = l < 2 ? o : pr;
-  const fq_t u = fq_sub_lazy(hi, lo), w = fq_add_lazy(hi, lo);
-  const fq_t u1 = dq_xchg(u, 1, mask), w1 = dq_xchg(w, 1, mask);
-  fq_t r = fq_mul(pick4(l, w1, w, w, u1), pick4(l, u, u, u1, w1));
   const int zero = fq_is_zero(r);
   const bool need = __shfl_sync(mask, zero, 3, 4) != 0 && !pid && !qid;  // Z3 = 0 on lane 3
   if (__any_sync(mask, need)) {
@@ -948,6 +978,23 @@ static __device__ __noinline__ fq_t dq_add(fq_t p, fq_t q, uint32_t mask) {
     if (need) r = ru;
   }
   return pid ? q : qid ? p : r;
+}
+
+static __device__ __noinline__ fq_t dq_add(fq_t p, fq_t q, uint32_t mask) {
+  const int l = dq_lane();
+  const uint32_t even = (l & 1) ? 0u : ~0u, neg0 = l == 0 ? ~0u : 0u, neg2 = l == 2 ? ~0u : 0u;
+  const fq_t po = dq_xchg(p, 2, mask), qo = dq_xchg(q, 2, mask);  // X <-> Y on 0, 2; T <-> Z on 1, 3
+  // lane 0: Y1 - X1 and Y2 + X2, lane 2: X1 + Y1 and Y2 - X2, lanes 1, 3: the other's Z1 or T1 and T2 or Z2
+  const fq_t m1 = fq_addsub(po, p, even, neg0), m2 = fq_addsub(q, qo, even, neg2);
+  const fq_t pr = fq_shl_lazy(fq_mul(m1, m2), l & 1);  // A, C, B, D on lanes 0..3, below 3q
+  // pairs {0, 2}: F = B - A, G = B + A; pairs {1, 3}: H = D - C, E = D + C
+  const fq_t o = dq_xchg(pr, 2, mask);
+  const fq_t u = fq_sub_lazy4(l < 2 ? o : pr, l < 2 ? pr : o), w = fq_add_lazy(o, pr);  // below 7q, 6q
+  // lane 0 lacks E, lane 2 lacks H, lane 3 lacks F and G
+  const fq_t r1 = dq_xchg(l == 1 ? w : u, 1, mask), r2 = dq_xchg(w, 1, mask);
+  const fq_t r = fq_mul(l == 0 || l == 3 ? r1 : w, l < 2 ? u : l == 2 ? r1 : r2);
+  if (__any_sync(mask, l == 3 && r.v[0] <= 1u)) return dq_add_rare(p, q, r, mask);
+  return r;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -976,18 +1023,18 @@ __device__ __forceinline__ fq_t dq_load_base(const uint4 *bases, uint32_t v) {
 // X3 = E F, T3 = E H, Y3 = G H, Z3 = F G.
 static __device__ __noinline__ fq_t dq_madd(fq_t p, fq_t b, bool neg, uint32_t mask) {
   const int l = dq_lane();
+  const uint32_t even = (l & 1) ? 0u : ~0u;
   const fq_t po = dq_xchg(p, 2, mask);
-  const fq_t m1 = l == 0 ? fq_sub_lazy(po, p) : l == 2 ? fq_add_lazy(p, po) : p;
-  const fq_t pr = fq_mul(m1, b);  // A, C, B, D on lanes 0..3
+  const fq_t m1 = fq_addsub((l & 1) ? p : po, p, even, l == 0 ? ~0u : 0u);
+  const fq_t pr = fq_mul(m1, b);  // A, C, B, D on lanes 0..3, below 1.5q
   const fq_t o = dq_xchg(pr, 2, mask);
-  const fq_t lo = l < 2 ? pr : o, hi = l < 2 ? o : pr;
-  fq_t u = fq_sub_lazy(hi, lo), w = fq_add_lazy(hi, lo);  // E, H on lanes 0, 2; F, G on 1, 3
-  const bool swap = neg && (l & 1);                       // a negative digit negates C
-  const fq_t un = fq_select(swap, w, u);
-  w = fq_select(swap, u, w);
-  u = un;
-  const fq_t u1 = dq_xchg(u, 1, mask), w1 = dq_xchg(w, 1, mask);
-  return fq_mul(l == 1 ? u1 : l == 2 ? w1 : u, l == 0 ? u1 : l == 1 ? w1 : w);
+  const fq_t d = fq_sub_lazy(l < 2 ? o : pr, l < 2 ? pr : o), a = fq_add_lazy(o, pr);
+  // E, H on lanes 0, 2; F, G on 1, 3, where a negative digit negates C
+  const bool swap = neg && (l & 1);
+  const fq_t u = swap ? a : d, w = swap ? d : a;
+  // lane 0 lacks F, lane 2 lacks G, lane 1 lacks E and H
+  const fq_t r1 = dq_xchg(l == 3 ? w : u, 1, mask), r2 = dq_xchg(w, 1, mask);
+  return fq_mul(l == 1 ? r1 : l == 2 ? w : u, l == 1 ? r2 : l == 3 ? w : r1);
 }
 
 // the point of base v itself: X = ypx - ymx (negated for a negative digit), Y = ypx + ymx, Z = 1, T = X Y
@@ -1109,11 +1156,14 @@ constexpr uint32_t kAllLanes = 0xffffffffu;
 // tree level the 3 x stride additions are spread over the quads, so the three trees take
 // log2(NT / 4) + 1 rounds of dependent additions instead of 3 log2(NT / 4).  Only warps holding an
 // active quad add (whole warps, so their shuffles stay converged).  The sums are valid in quad 0.
+// The last warp, which most rounds leave idle, doubles its D once in every such round, up to `dbl`
+// times in all (the rest after the rounds, while warp 0 goes on).
 template <int NT>
-__device__ __forceinline__ void block_sum3(fq_t (&X)[3], uint4 *sh) {
+__device__ __forceinline__ void block_sum3(fq_t (&X)[3], uint4 *sh, fq_t &D, uint32_t dbl) {
   constexpr uint32_t Q = NT / 4;
   const uint32_t q = threadIdx.x >> 2;
   const uint32_t warp_q0 = (threadIdx.x >> 5) * 8;  // first quad of this warp
+  const bool last_warp = warp_q0 + 8 == Q;
   for (int k = 0; k < 3; k++) dq_store(sh + (k * Q + q) * 12, X[k]);
   __syncthreads();
 #pragma unroll 1
@@ -1128,12 +1178,19 @@ __device__ __forceinline__ void block_sum3(fq_t (&X)[3], uint4 *sh) {
         a = dq_load(sh + slot * 12);
         o = dq_load(sh + (slot + stride) * 12);
       }
-      if (u0 + warp_q0 < 3 * stride) a = dq_add(a, o, kAllLanes);
+      if (u0 + warp_q0 < 3 * stride) {
+        a = dq_add(a, o, kAllLanes);
+      } else if (last_warp && dbl) {
+        D = dq_dbl(D, kAllLanes);
+        dbl--;
+      }
       __syncthreads();
       if (act) dq_store(sh + slot * 12, a);
       __syncthreads();
     }
   }
+  if (last_warp)
+    for (; dbl; dbl--) D = dq_dbl(D, kAllLanes);
   for (int k = 0; k < 3; k++) X[k] = dq_load(sh + k * Q * 12);
 }
 
@@ -1156,14 +1213,15 @@ __device__ __forceinline__ fq_t block_suffix_scan(fq_t X, uint4 *sh) {
   return X;
 }
 
-// Combine `cnt` runs (R, A) of 2^lin_log2 buckets each into one run (result in quad 0).
+// Combine `cnt` runs (R, A) of 2^lin_log2 buckets each into one run (A in quad 0, and R doubled
+// r_dbl times in the first quad of the last warp).
 // Quad u takes runs [u per, u per + per) (per a power of two) and forms SA = sum A_i,
 // RR = sum R_i and T = sum (i - u per) R_i.  Then
 //   A = sum_u SA_u + 2^lin_log2 (sum_u T_u + per sum_u u RR_u),  R = sum_u RR_u,
 // where sum_u u RR_u = sum_{u >= 1} (suffix sum of RR at u): one block scan and three block
 // sums (run together), and only quad 0 doubles.
 template <int NT>
-__device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log2, bool want_r,
+__device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log2, uint32_t r_dbl,
                               uint4 *sh, fq_t &A_out, fq_t &R_out) {
   constexpr uint32_t Q = NT / 4;
   const uint32_t q = threadIdx.x >> 2;
@@ -1192,9 +1250,10 @@ __device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log
     SA = dq_add(SA, A, kAllLanes);
   }
   const fq_t suf = block_suffix_scan<NT>(RR, sh);
-  if (want_r && q == 0) R_out = suf;  // suffix at 0 is the total
+  R_out = dq_load(sh);  // suffix at 0: the total
+  __syncthreads();
   fq_t S[3] = {q ? suf : dq_identity(), T, SA};
-  block_sum3<NT>(S, sh);
+  block_sum3<NT>(S, sh, R_out, r_dbl);
   if (q == 0) {  // lanes 0..3 of warp 0
     fq_t X = S[0];
 #pragma unroll 1
@@ -1218,17 +1277,17 @@ __global__ void __launch_bounds__(NT) k_reduce2(PassBuffers pb) {
   const uint32_t first = (g - wd.grp_begin) * G;
   const uint32_t cnt = min(G, wd.nseg - first);
   fq_t A, R;
-  block_combine<NT>(pb.seg_out + (size_t)(wd.seg_begin + first) * 24, cnt, pb.red_len_log2, true,
-                    sh, A, R);
-  if (threadIdx.x < 4) {  // quad 0: one coordinate per lane
-    dq_store(pb.grp_out + (size_t)g * 24, R);
-    dq_store(pb.grp_out + (size_t)g * 24 + 12, A);
-  }
+  // level 3 weighs the group's R by the buckets of a group, a power of two: the doublings are done
+  // here, beside the sums, instead of one after another at the end of level 3
+  block_combine<NT>(pb.seg_out + (size_t)(wd.seg_begin + first) * 24, cnt, pb.red_len_log2,
+                    pb.red_len_log2 + pb.grp_len_log2, sh, A, R);
+  if (threadIdx.x < 4) dq_store(pb.grp_out + (size_t)g * 24 + 12, A);  // one coordinate per lane
+  if (threadIdx.x >= NT - 32 && threadIdx.x < NT - 28) dq_store(pb.grp_out + (size_t)g * 24, R);
 }
 
 // Windows of at most kRed3SmallMax groups (windowed MSMs: 2^(c-1) buckets make a few groups)
 // are combined by one quad each, in order:
-//   A = sum_i A_i + 2^lin sum_i i R_i,  sum_i i R_i = sum_{i >= 1} (suffix sum of R at i),
+//   A = sum_i A_i + sum_i i R_i (R_i weighed by level 2),  sum_i i R_i = sum_{i >= 1} (suffix sum of R at i),
 // so hundreds of windows run side by side instead of one block each.  The quads of a warp work
 // on different windows, so each shuffles under its own 4-lane mask.
 constexpr uint32_t kRed3SmallMax = 16;
@@ -1242,7 +1301,6 @@ __global__ void __launch_bounds__(128) k_reduce3_small(PassBuffers pb) {
   const uint32_t n = wd.ngrp;
   if (n == 0 || n > kRed3SmallMax) return;
   const uint32_t mask = 0xfu << (threadIdx.x & 28);
-  const uint32_t lin = pb.red_len_log2 + pb.grp_len_log2;
   const uint4 *items = pb.grp_out + (size_t)wd.grp_begin * 24;
   fq_t RR = dq_load(items + (size_t)(n - 1) * 24);
   fq_t SA = dq_load(items + (size_t)(n - 1) * 24 + 12);
@@ -1257,13 +1315,7 @@ __global__ void __launch_bounds__(128) k_reduce3_small(PassBuffers pb) {
       T = dq_add(T, RR, mask);
     }
   }
-  fq_t out = SA;
-  if (n >= 2) {
-#pragma unroll 1
-    for (uint32_t k = 0; k < lin; k++) T = dq_dbl(T, mask);
-    out = dq_add(T, SA, mask);
-  }
-  dq_store(pb.win_sum + (size_t)gw * 12, out);
+  dq_store(pb.win_sum + (size_t)gw * 12, n >= 2 ? dq_add(T, SA, mask) : SA);
 }
 
 template <int NT>
@@ -1276,8 +1328,7 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
   const WinDesc wd = pb.wins[gw];
   if (wd.ngrp <= kRed3SmallMax) return;  // k_reduce3_small's
   fq_t A, R;
-  block_combine<NT>(pb.grp_out + (size_t)wd.grp_begin * 24, wd.ngrp,
-                    pb.red_len_log2 + pb.grp_len_log2, false, sh, A, R);
+  block_combine<NT>(pb.grp_out + (size_t)wd.grp_begin * 24, wd.ngrp, 0, 0, sh, A, R);
   if (threadIdx.x < 4) dq_store(pb.win_sum + (size_t)gw * 12, A);
 }
 
