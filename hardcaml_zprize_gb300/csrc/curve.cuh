@@ -230,8 +230,7 @@ static __device__ __noinline__ wpt_t w_add(const wpt_t &p, const wpt_t &q) {  //
 // inversion: u = (Z+Y)/(Z-Y), v = ts*u*Z/X, x_w = u/c_B + c_A/(3 c_B), y_w = v/c_B.
 // The identity maps to infinity; the order-two point (0, -1) maps to its Weierstrass image
 // (c_A/(3 c_B), 0) (the reference sends both x = 0 points to infinity, :393-396).
-template <bool QUAD>
-__device__ __forceinline__ wpt_t te_to_weierstrass_t(const xyzt_t &p, uint32_t mask) {
+static __device__ __noinline__ wpt_t te_to_weierstrass(const xyzt_t &p) {
   const uint32_t ts[FQ_LIMBS] = BLS_TWISTED_SCALE;
   const uint32_t icb[FQ_LIMBS] = BLS_INV_CB;
   const uint32_t ca3[FQ_LIMBS] = BLS_CA_OVER_3CB;
@@ -245,8 +244,7 @@ __device__ __forceinline__ wpt_t te_to_weierstrass_t(const xyzt_t &p, uint32_t m
   }
   const fq_t zpy = fq_add(p.z, p.y);
   const fq_t zmy = fq_sub(p.z, p.y);
-  const fq_t den = fq_mul_ool(zmy, p.x);
-  const fq_t inv = QUAD ? fq_inv_quad(den, mask) : fq_inv_vartime(den);
+  const fq_t inv = fq_inv_vartime(fq_mul_ool(zmy, p.x));
   const fq_t u = fq_mul_ool(fq_mul_ool(zpy, p.x), inv);
   const fq_t v = fq_mul_ool(fq_mul_ool(fq_mul_ool(zpy, p.z), inv), fq_from(ts));
   r.x = fq_add(fq_mul_ool(u, fq_from(icb)), fq_from(ca3));
@@ -255,13 +253,38 @@ __device__ __forceinline__ wpt_t te_to_weierstrass_t(const xyzt_t &p, uint32_t m
   return r;
 }
 
-static __device__ __noinline__ wpt_t te_to_weierstrass(const xyzt_t &p) {
-  return te_to_weierstrass_t<false>(p, 0u);
-}
-// The same map run by the four lanes of a quad that all hold p (`mask` covers them): the
-// inversion is shared between the lanes (fq_inv_quad); every lane returns the result.
-static __device__ __noinline__ wpt_t te_to_weierstrass_quad(const xyzt_t &p, uint32_t mask) {
-  return te_to_weierstrass_t<true>(p, mask);
+// The same map run by a whole warp whose lanes all hold X, Y, Z; lane 0 gets the result.  Lane 0 forms
+// the denominator (Z - Y) X, lanes 1 and 2 the numerators (Z + Y) X and (Z + Y) Z times their constants
+// and R^3 (so that one product with the integer inverse ends in Montgomery form): three product
+// latencies around the warp's inversion instead of eleven.
+static __device__ __noinline__ wpt_t te_to_weierstrass_warp(const fq_t &X, const fq_t &Y, const fq_t &Z) {
+  constexpr uint32_t full = 0xffffffffu;
+  const uint32_t k1[FQ_LIMBS] = BLS_INV_CB_R3X, k2[FQ_LIMBS] = BLS_TS_INV_CB_R3X;
+  const uint32_t ca3[FQ_LIMBS] = BLS_CA_OVER_3CB;
+  const int lane = threadIdx.x & 31;
+  wpt_t r;
+  if (fq_is_zero(X)) {  // the same on every lane
+    if (fq_eq(Y, Z)) return w_infinity();
+    r.x = fq_from(ca3);
+    r.y = fq_zero();
+    r.z = fq_one();
+    return r;
+  }
+  const fq_t zpy = fq_add_lazy(Z, Y), zmy = fq_sub_lazy(Z, Y);
+  fq_t n = fq_mul_nv(lane == 0 ? zmy : zpy, lane < 2 ? X : Z);
+  fq_t den;
+#pragma unroll
+  for (int k = 0; k < FQ_LIMBS; k++) den.v[k] = __shfl_sync(full, n.v[k], 0);
+  n = fq_mul_nv(n, fq_select(lane == 1, fq_from(k1), fq_from(k2)));
+  n = fq_mul_nv(fq_inv_warp(den), n);
+#pragma unroll
+  for (int k = 0; k < FQ_LIMBS; k++) {
+    r.x.v[k] = __shfl_sync(full, n.v[k], 1);
+    r.y.v[k] = __shfl_sync(full, n.v[k], 2);
+  }
+  r.x = fq_add(r.x, fq_from(ca3));
+  r.z = fq_one();
+  return r;
 }
 
 // Jacobian -> affine with z in {0, 1}, all coordinates canonical in [0, q)

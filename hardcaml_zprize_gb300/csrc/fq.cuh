@@ -36,6 +36,9 @@
 // 1/c_B and c_A/(3 c_B) of the Montgomery -> Weierstrass map (bls12_377_g1.h:366-374)
 #define BLS_INV_CB {0x776b1e1du, 0x455ce02fu, 0x63e0aa56u, 0x4b123b66u, 0x73fa6bf3u, 0x4d75723eu, 0x885e1101u, 0x468df1d4u, 0x638ee120u, 0x039e6c63u, 0x67cb3b82u, 0x005cdbd9u}
 #define BLS_CA_OVER_3CB {0x00000099u, 0x823ac000u, 0xb000004fu, 0xc5cabdc0u, 0x2f8c080du, 0x7f75ae86u, 0x9278b089u, 0x9ed4423bu, 0xec64c452u, 0x79467000u, 0x34c71c50u, 0x0120d3e4u}
+// (1/c_B) R^3 and ts (1/c_B) R^3, factors of numerators that meet a plain inverse (te_to_weierstrass_warp)
+#define BLS_INV_CB_R3X {0xa53f9bdfu, 0xe50fb361u, 0x8a41d16bu, 0x7c0b9d21u, 0xf62d549bu, 0x87b97febu, 0xa7d11b60u, 0x8ddcefe4u, 0x334f01a9u, 0xe403bc7au, 0x816dd8dbu, 0x002693d5u}
+#define BLS_TS_INV_CB_R3X {0x8249903fu, 0x89d5d01eu, 0xd7a74139u, 0x80a3ad71u, 0xa655ae9fu, 0xd0ecc29bu, 0xb333f4c5u, 0x45a17a34u, 0x4d6653fbu, 0x556d2dacu, 0x17c7aa65u, 0x000e207au}
 // R^3 mod q: turns a plain inverse of a Montgomery-form value into the Montgomery-form inverse
 #define BLS_R3 {0x8815de20u, 0x581f532fu, 0xbe329585u, 0xe50f4148u, 0x0449f513u, 0x2be8b118u, 0xc804a20eu, 0x6a2a9516u, 0x13590cb9u, 0x3f725407u, 0xc0e7dda5u, 0x01065ab4u}
 // q - 2, the Fermat inversion exponent
@@ -364,64 +367,75 @@ static __device__ __noinline__ fq_t fq_inv_vartime(const fq_t &a) {
   return fq_mul(inv, fq_from(r3));
 }
 
-// The same inverse computed by the four lanes of a quad together (all four hold `a`; `mask`
-// covers them).  Every batch's four combinations (f, g, d, e) run one per lane through one code
-// path and are exchanged by shuffles, so a batch costs one combination instead of four on one
-// thread.  All four lanes return the inverse.
-static __device__ __noinline__ fq_t fq_inv_quad(const fq_t &a, uint32_t mask) {
-  const int l = (int)(threadIdx.x & 3);
+// The integer inverse of a (not times a power of R; a != 0 modulo q) by the 32 lanes of a warp
+// together, which all hold a: a value below 2^383 congruent to it, on every lane.
+// Lane l < 13 holds digit l (30 bits, signed) of f and g, lane 16 + l of d and e.  Applying a batch's
+// matrix is then two multiply-adds per row and lane: dividing by 2^30 moves each product's low part
+// one lane down and keeps its high part, and one more carry between neighbours brings the digits back
+// below 2^29 + 3; no carry runs through the digits.  d and e first take the multiple m q, |m| <= 2^29,
+// that makes them divisible (q = 1 mod 2^30), so a batch adds at most q/2 to their magnitude.  At most
+// 37 batches (1090 divsteps) are needed for 377 bits, about 27 on average; 32 q keeps d positive.
+// k_final of a 2^12-point MSM, with the map's products shared between lanes: 57 -> 27 us against a
+// quad that applied the matrices limb by limb.
+static __device__ __noinline__ fq_t fq_inv_warp(const fq_t &a) {
+  constexpr uint32_t full = 0xffffffffu;
+  const int32_t q30[13] = {1, 337838080, 8, 47665420, 155713559, 227065576, 288944623, -159596483, 154868259, 385987205, 246178736, 293990724, 110138};
+  const int32_t off30[13] = {32, 73400320, 266, 451551616, 687866593, 823647492, 656293350, 261621672, 660816987, 540430500, 361526795, 817768583, 3524424};  // 32 q
+  const int lane = threadIdx.x & 31, l = lane & 15;
+  const bool upper = lane >= 16;
   const fq_t c = fq_canon(a);
-  const uint32_t q12[FQ_LIMBS] = BLS_Q;
-  uint32_t f[DS_LIMBS], g[DS_LIMBS], d[DS_LIMBS], e[DS_LIMBS], q[DS_LIMBS];
-  uint32_t nz = 0;
+  int32_t qd = 0, od = 0, gd = 0;
 #pragma unroll
-  for (int i = 0; i < FQ_LIMBS; i++) {
-    f[i] = q[i] = q12[i];
-    g[i] = c.v[i];
-    d[i] = e[i] = 0;
-    nz |= c.v[i];
+  for (int i = 0; i < 13; i++) {
+    const int w = 30 * i / 32, s = 30 * i % 32;
+    const uint32_t hi = w + 1 < FQ_LIMBS ? c.v[w + 1] : 0u;
+    if (l == i) {
+      qd = q30[i];
+      od = off30[i];
+      gd = (int32_t)(__funnelshift_r(c.v[w], hi, s) & 0x3fffffffu);
+    }
   }
-  f[12] = g[12] = d[12] = e[12] = q[12] = 0;
-  e[0] = 1;
-  if (!nz) return fq_zero();
+  int32_t x = upper ? 0 : qd, y = upper ? (l == 0 ? 1 : 0) : gd;
   int delta = 1;
 #pragma unroll 1
-  for (int batch = 0; batch < 64; batch++) {
+  for (int batch = 0; batch < 48; batch++) {
     int32_t u, v, qq, r;
-    delta = ds_batch30(delta, f[0], g[0], u, v, qq, r);
-    // lane 0: f' = (u f + v g) / 2^30, lane 1: g' = (qq f + r g) / 2^30, lanes 2, 3: d', e' mod q
-    uint32_t x[DS_LIMBS], y[DS_LIMBS], res[DS_LIMBS];
-#pragma unroll
-    for (int i = 0; i < DS_LIMBS; i++) {
-      x[i] = l < 2 ? f[i] : d[i];
-      y[i] = l < 2 ? g[i] : e[i];
-    }
-    ds_combine_any(res, (l & 1) ? qq : u, x, (l & 1) ? r : v, y, q, l >= 2);
-    uint32_t gz = 0;
-#pragma unroll
-    for (int i = 0; i < DS_LIMBS; i++) {
-      f[i] = __shfl_sync(mask, res[i], 0, 4);
-      g[i] = __shfl_sync(mask, res[i], 1, 4);
-      d[i] = __shfl_sync(mask, res[i], 2, 4);
-      e[i] = __shfl_sync(mask, res[i], 3, 4);
-      gz |= g[i];
-    }
-    if (gz == 0) break;  // the same on all four lanes
+    delta = ds_batch30(delta, (uint32_t)__shfl_sync(full, x, 0), (uint32_t)__shfl_sync(full, y, 0), u, v, qq, r);
+    int64_t t1 = (int64_t)u * x + (int64_t)v * y, t2 = (int64_t)qq * x + (int64_t)r * y;
+    // m = -(t mod 2^30), centred; zero for f and g, whose division is exact
+    const int32_t m1 = -((int32_t)(__shfl_sync(full, (uint32_t)t1, 0, 16) << 2) >> 2);
+    const int32_t m2 = -((int32_t)(__shfl_sync(full, (uint32_t)t2, 0, 16) << 2) >> 2);
+    t1 += (int64_t)m1 * qd;
+    t2 += (int64_t)m2 * qd;
+    const int32_t lo1 = (int32_t)((uint32_t)t1 << 2) >> 2, lo2 = (int32_t)((uint32_t)t2 << 2) >> 2;
+    const int32_t n1 = __shfl_down_sync(full, lo1, 1, 16) + (int32_t)((t1 + (1 << 29)) >> 30);
+    const int32_t n2 = __shfl_down_sync(full, lo2, 1, 16) + (int32_t)((t2 + (1 << 29)) >> 30);
+    const int32_t c1 = l < 12 ? (n1 + (1 << 29)) >> 30 : 0, c2 = l < 12 ? (n2 + (1 << 29)) >> 30 : 0;
+    const int32_t p1 = __shfl_up_sync(full, c1, 1, 16), p2 = __shfl_up_sync(full, c2, 1, 16);
+    x = n1 - (c1 << 30) + (l ? p1 : 0);
+    y = n2 - (c2 << 30) + (l ? p2 : 0);
+    if (!__any_sync(full, !upper && y != 0)) break;
   }
-  if (ds_is_neg(f)) {  // f = -1: the inverse is q - d
-    int64_t acc = 0;
+  // f = +-1: the inverse is +-d; digits of +-d + 32 q, then 32-bit words
+  const bool neg = __shfl_sync(full, x, 0) < 0;
+  const int32_t z = (neg ? -x : x) + od;
+  uint32_t d[13];
+  int32_t carry = 0;
 #pragma unroll
-    for (int i = 0; i < DS_LIMBS; i++) {
-      acc += (int64_t)q[i] - (int64_t)d[i];
-      d[i] = (uint32_t)acc;
-      acc >>= 32;
-    }
+  for (int i = 0; i < 13; i++) {
+    const int32_t t = __shfl_sync(full, z, 16 + i) + carry;
+    d[i] = (uint32_t)t & 0x3fffffffu;
+    carry = t >> 30;
   }
-  fq_t inv;
+  fq_t res;
 #pragma unroll
-  for (int i = 0; i < FQ_LIMBS; i++) inv.v[i] = d[i];
-  const uint32_t r3[FQ_LIMBS] = BLS_R3;
-  return fq_mul(inv, fq_from(r3));
+  for (int i = 0; i < FQ_LIMBS; i++) {  // word i: bits 32 i .. 32 i + 31
+    const int k = 32 * i / 30, s = 32 * i % 30;
+    uint32_t w = (d[k] >> s) | (d[k + 1] << (30 - s));
+    if (s > 28 && k + 2 < 13) w |= d[k + 2] << (60 - s);
+    res.v[i] = w;
+  }
+  return res;
 }
 
 // ---- 16-byte vector loads/stores of field elements ----

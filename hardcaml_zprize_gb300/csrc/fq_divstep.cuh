@@ -15,6 +15,8 @@
 // serial shift/subtract rounds of a binary extended Euclid.
 //
 // Plain integer code (host and device): signed values are 13 limbs of 32 bits, two's complement.
+// The pipeline's one inversion per MSM runs the same batches on a warp, a digit of 30 bits per lane
+// (fq_inv_warp).
 #pragma once
 #include <stdint.h>
 
@@ -34,54 +36,44 @@ FQ_HD int ds_ctz32(uint32_t x) {
 #endif
 }
 
-// 30 divsteps on the low words of f and g; returns delta and the transition matrix
-// [u v; q r] with 2^30 (f', g') = (u f + v g, q f + r g).
+// 30 divsteps on the low words of f and g (their low 30 bits); returns delta and the transition
+// matrix [u v; q r] with 2^30 (f', g') = (u f + v g, q f + r g).
+// Zeros of g are stripped together, and with delta <= 0 the next min(1 - delta, left) steps keep f, so
+// the multiple of f that clears up to six low bits of g is added at once (f (f^2 - 2) = -1/f mod 64 for
+// odd f): about 9 rounds a batch instead of 15 with one odd step each.
 FQ_HD int ds_batch30(int delta, uint32_t f, uint32_t g, int32_t &u, int32_t &v, int32_t &q,
                      int32_t &r) {
-  int32_t uu = 1, vv = 0, qq = 0, rr = 1;
+  uint32_t uu = 1, vv = 0, qq = 0, rr = 1;  // two's complement
   int left = 30;
-  while (left > 0) {
-    if (g == 0) {  // the rest of the batch is halvings
-      uu = (int32_t)((uint32_t)uu << left);
-      vv = (int32_t)((uint32_t)vv << left);
-      delta += left;
-      break;
-    }
-    int z = ds_ctz32(g);
-    if (z > left) z = left;
-    if (z) {  // a run of even g: halve z times at once
-      g >>= z;
-      uu = (int32_t)((uint32_t)uu << z);
-      vv = (int32_t)((uint32_t)vv << z);
-      delta += z;
-      left -= z;
-      if (left == 0) break;
-    }
-    // g is odd
-    if (delta > 0) {
-      delta = 1 - delta;
-      const uint32_t nf = g;
-      g = (g - f) >> 1;
+  for (;;) {
+    const int z = ds_ctz32(g | (1u << left));  // halvings
+    g >>= z;
+    uu <<= z;
+    vv <<= z;
+    delta += z;
+    left -= z;
+    if (left == 0) break;
+    if (delta > 0) {  // g is odd: (f, g) <- (g, -f), and the steps below add f back
+      delta = -delta;
+      const uint32_t nf = g, nu = qq, nv = rr;
+      g = 0u - f;
       f = nf;
-      const int32_t nu = 2 * qq, nv = 2 * rr;
-      qq -= uu;
-      rr -= vv;
+      qq = 0u - uu;
+      rr = 0u - vv;
       uu = nu;
       vv = nv;
-    } else {
-      delta = 1 + delta;
-      g = (g + f) >> 1;
-      qq += uu;
-      rr += vv;
-      uu *= 2;
-      vv *= 2;
     }
-    left--;
+    int k = left < 1 - delta ? left : 1 - delta;
+    if (k > 6) k = 6;
+    const uint32_t w = f * (f * f - 2) * g & ((1u << k) - 1);
+    g += f * w;
+    qq += uu * w;
+    rr += vv * w;
   }
-  u = uu;
-  v = vv;
-  q = qq;
-  r = rr;
+  u = (int32_t)uu;
+  v = (int32_t)vv;
+  q = (int32_t)qq;
+  r = (int32_t)rr;
   return delta;
 }
 
@@ -151,9 +143,9 @@ FQ_HD void ds_combine_mod(uint32_t (&out)[DS_LIMBS], int32_t a, const uint32_t (
   if (ds_geq(out, q)) ds_add_q(out, q, -1);
 }
 
-// One code path for all four combinations of a batch, so that four lanes of a warp can each take
-// one without diverging: out = (a x + b y) / 2^30, and modulo q when `mod` (x, y in [0, q), result
-// in [0, q)); without `mod`, x and y are signed and the division is exact.
+// One code path for all four combinations of a batch (the host check runs them lane after lane):
+// out = (a x + b y) / 2^30, and modulo q when `mod` (x, y in [0, q), result in [0, q)); without `mod`,
+// x and y are signed and the division is exact.
 FQ_HD void ds_combine_any(uint32_t (&out)[DS_LIMBS], int32_t a, const uint32_t (&x)[DS_LIMBS], int32_t b,
                           const uint32_t (&y)[DS_LIMBS], const uint32_t (&q)[DS_LIMBS], bool mod) {
   uint32_t w[DS_LIMBS + 1];

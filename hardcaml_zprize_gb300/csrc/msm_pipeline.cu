@@ -1394,7 +1394,7 @@ __global__ void __launch_bounds__(128) k_final(PassBuffers pb) {
     atomicAdd(&cls_sum[pb.special_cls[s] & 7], w0.x & 3u);
   }
   __syncthreads();
-  if (threadIdx.x >= 4) return;  // lanes 0..3 of warp 0 run the combine together
+  if (threadIdx.x >= 32) return;  // warp 0 goes on: lanes 0..3 run the combine, all lanes the map
   uint64_t *out = pb.results + (size_t)jd.result_slot * 18;
   if (pb.counters[CNT_ERROR]) {
     if (threadIdx.x == 0)
@@ -1403,7 +1403,7 @@ __global__ void __launch_bounds__(128) k_final(PassBuffers pb) {
   }
   // Horner over the windows: acc = 2^c * acc + WS_w (pippenger.h:36-45 doubles per offset)
   fq_t dacc = dq_identity();
-  if (jd.n > 0 && jd.nred > 0) {
+  if (threadIdx.x < 4 && jd.n > 0 && jd.nred > 0) {
     dacc = dq_load(pb.win_sum + (size_t)(jd.win_begin + jd.nred - 1) * 12);
 #pragma unroll 1
     for (int w = (int)jd.nred - 2; w >= 0; w--) {
@@ -1412,18 +1412,15 @@ __global__ void __launch_bounds__(128) k_final(PassBuffers pb) {
       dacc = dq_add(dacc, dq_load(pb.win_sum + (size_t)(jd.win_begin + w) * 12), 0xfu);
     }
   }
-  // gather the point on lane 0 (lane 1 holds T, lane 2 Y, lane 3 Z)
-  xyzt_t acc;
-  // every lane of the quad takes the whole point (lane 0 holds X, 1 T, 2 Y, 3 Z), and the four
-  // share the inversion of the map to Weierstrass
+  __syncwarp();
+  fq_t X, Y, Z;  // lane 0 holds X, 2 Y, 3 Z
 #pragma unroll
   for (int k = 0; k < FQ_LIMBS; k++) {
-    acc.x.v[k] = __shfl_sync(0xfu, dacc.v[k], 0, 4);
-    acc.t.v[k] = __shfl_sync(0xfu, dacc.v[k], 1, 4);
-    acc.y.v[k] = __shfl_sync(0xfu, dacc.v[k], 2, 4);
-    acc.z.v[k] = __shfl_sync(0xfu, dacc.v[k], 3, 4);
+    X.v[k] = __shfl_sync(kAllLanes, dacc.v[k], 0);
+    Y.v[k] = __shfl_sync(kAllLanes, dacc.v[k], 2);
+    Z.v[k] = __shfl_sync(kAllLanes, dacc.v[k], 3);
   }
-  wpt_t res = te_to_weierstrass_quad(acc, 0xfu);  // z is 1, or 0 for infinity
+  wpt_t res = te_to_weierstrass_warp(X, Y, Z);  // z is 1, or 0 for infinity
   if (threadIdx.x != 0) return;
   bool added = false;
   for (uint32_t c = 0; c < pb.n_classes && c < 8; c++) {
