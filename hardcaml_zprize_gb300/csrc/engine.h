@@ -125,7 +125,7 @@ struct PassBuffers {
   uint4 *partials;              // [max_tasks] x 12 uint4
   uint32_t *heavy;              // [n_buckets]
   uint32_t *order;              // [max_tasks] task ids, longest first
-  uint32_t *len_hist;           // [seg_len + 1] task-length histogram, then start cursors
+  uint32_t *len_hist;           // [seg_len + 1] task-length histogram, then as many slot cursors
   uint32_t *counters;           // [CNT_WORDS]
   uint4 *seg_out;               // [n_segs] x 2 x 12 uint4
   uint4 *grp_out;               // [n_grps] x 2 x 12 uint4

@@ -502,7 +502,7 @@ struct Workspace {
     CK(tasks.ensure((size_t)pl.max_tasks * sizeof(Task), &moved));
     CK(partials.ensure((size_t)pl.max_tasks * MSM_BUCKET_BYTES, &moved));
     CK(order.ensure((size_t)pl.max_tasks * 4, &moved));
-    CK(len_hist.ensure((size_t)(pl.seg_len + 1) * 4, &moved));
+    CK(len_hist.ensure((size_t)(pl.seg_len + 1) * 8, &moved));
     CK(counters.ensure(CNT_WORDS * 4, &moved));
     CK(seg_out.ensure((size_t)pl.n_segs * 2 * MSM_BUCKET_BYTES, &moved));
     CK(grp_out.ensure((size_t)pl.n_grps * 2 * MSM_BUCKET_BYTES, &moved));
@@ -2199,7 +2199,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   const size_t o_tasks = carve(off, (size_t)tasks * sizeof(Task));
   const size_t o_part = carve(off, (size_t)tasks * MSM_BUCKET_BYTES);
   const size_t o_order = carve(off, (size_t)tasks * 4);
-  const size_t o_lenh = carve(off, (size_t)(seg_len + 1) * 4);
+  const size_t o_lenh = carve(off, (size_t)(seg_len + 1) * 8);
   const size_t o_seg = carve(off, (size_t)nsegs * 2 * MSM_BUCKET_BYTES);
   const size_t o_grp = carve(off, (size_t)ngrps * 2 * MSM_BUCKET_BYTES);
   const size_t o_win = carve(off, (size_t)jd.nred * MSM_BUCKET_BYTES);

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) k_clear(PassBuffers pb) {
   pdl_begin();
   const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
   for (uint32_t i = i0; i < pb.n_buckets; i += n) pb.count[i] = 0;
-  for (uint32_t i = i0; i <= pb.seg_len; i += n) pb.len_hist[i] = 0;
+  for (uint32_t i = i0; i < 2 * (pb.seg_len + 1); i += n) pb.len_hist[i] = 0;
   if (i0 < CNT_WORDS) pb.counters[i0] = 0;
 }
 
@@ -298,6 +298,14 @@ __device__ __forceinline__ uint32_t ntask_of(uint32_t cnt, uint32_t seg_len) {
   return (cnt + seg_len - 1) / seg_len;
 }
 
+// the pass's entries and tasks, against the plan's room
+__device__ __forceinline__ void scan_totals(const PassBuffers &pb, uint32_t entries, uint32_t tasks) {
+  if ((uint64_t)entries > pb.max_entries) set_error(pb.counters, 1, entries);
+  if (tasks > pb.max_tasks) set_error(pb.counters, 2, tasks);
+  pb.counters[CNT_TASKS] = min(tasks, pb.max_tasks);
+  pb.counters[CNT_ENTRIES] = entries;
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(PassBuffers pb) {
   pdl_begin();
   const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
@@ -338,13 +346,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(PassBuffers pb, ui
     if (threadIdx.x == 0) carry_sh = make_uint2(cr.x + total.x, cr.y + total.y);
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    const uint2 t = carry_sh;
-    if ((uint64_t)t.x > pb.max_entries) set_error(pb.counters, 1, t.x);
-    if (t.y > pb.max_tasks) set_error(pb.counters, 2, t.y);
-    pb.counters[CNT_TASKS] = min(t.y, pb.max_tasks);
-    pb.counters[CNT_ENTRIES] = t.x;
-  }
+  if (threadIdx.x == 0) scan_totals(pb, carry_sh.x, carry_sh.y);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
@@ -372,6 +374,55 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
     ex.x += c[k];
     ex.y += ntask_of(c[k], pb.seg_len);
   }
+}
+
+// The three scan kernels and k_len_hist in one, for passes of at most kScanSmallBlocks blocks of
+// buckets: each block sums the counts before its own itself (at most 512 KB from L2).  A launch of
+// its own costs such a pass about 4 us.
+constexpr uint32_t kScanSmallBlocks = 32;
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
+  pdl_begin();
+  extern __shared__ uint32_t h[];  // [seg_len + 1]
+  for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x) h[i] = 0;
+  uint2 before = make_uint2(0, 0), total;
+  for (uint32_t i = threadIdx.x; i < blockIdx.x * kScanBlock; i += blockDim.x) {
+    const uint32_t c = pb.count[i];
+    before.x += c;
+    before.y += ntask_of(c, pb.seg_len);
+  }
+  block_excl_scan2(before, before);
+  const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  uint32_t c[kScanItems];
+  uint2 v = make_uint2(0, 0);
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    c[k] = base + k < pb.n_buckets ? pb.count[base + k] : 0u;
+    const uint32_t nt = ntask_of(c[k], pb.seg_len);
+    v.x += c[k];
+    v.y += nt;
+    if (nt) {
+      atomicAdd(&h[c[k] - (nt - 1) * pb.seg_len], 1u);
+      if (nt > 1) atomicAdd(&h[pb.seg_len], nt - 1);
+    }
+  }
+  uint2 ex = block_excl_scan2(v, total);
+  ex.x += before.x;
+  ex.y += before.y;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    if (base + k < pb.n_buckets) {
+      pb.offset[base + k] = ex.x;
+      pb.fill[base + k] = ex.x;
+      pb.taskoff[base + k] = ex.y;
+    }
+    ex.x += c[k];
+    ex.y += ntask_of(c[k], pb.seg_len);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x)
+    if (h[i]) atomicAdd(&pb.len_hist[i], h[i]);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) scan_totals(pb, before.x + total.x, before.y + total.y);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -529,28 +580,29 @@ __global__ void k_len_hist(PassBuffers pb) {
     if (h[i]) atomicAdd(&pb.len_hist[i], h[i]);
 }
 
-// cursor[len] = number of tasks longer than len (longest first); one thread, seg_len + 1 bins
-__global__ void k_len_scan(PassBuffers pb) {
-  pdl_begin();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  uint32_t acc = 0;
-  for (uint32_t l = pb.seg_len + 1; l-- > 0;) {
-    const uint32_t c = pb.len_hist[l];
-    pb.len_hist[l] = acc;
-    acc += c;
-  }
-}
-
 // One thread per bucket writes the bucket's runs and their slots in the processing order: the
 // last run takes a slot in the bin of its length, the full runs of a split bucket a block of
 // slots in the seg_len bin.  The block ranks its runs per bin in shared memory and reserves each
 // bin's slots with one global atomic, so the few hot bin cursors (lengths cluster around the mean
-// bucket load) see one atomic per block and bin.
+// bucket load) see one atomic per block and bin.  A bin starts after the runs longer than it: every
+// block sums the histogram for itself (one thread did it in a kernel of its own before).
 __global__ void __launch_bounds__(256) k_tasks(PassBuffers pb) {
   pdl_begin();
   extern __shared__ uint32_t sh_bins[];  // [seg_len + 1] counts, then [seg_len + 1] slot bases
   uint32_t *bin_cnt = sh_bins, *bin_base = sh_bins + pb.seg_len + 1;
-  for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x) bin_cnt[i] = 0;
+  {
+    const uint32_t per = pb.seg_len / blockDim.x + 1, d0 = threadIdx.x * per;  // lengths from the longest down
+    uint2 sum = make_uint2(0, 0), all;
+    for (uint32_t d = d0; d < d0 + per && d <= pb.seg_len; d++) {
+      bin_cnt[pb.seg_len - d] = 0;
+      sum.x += pb.len_hist[pb.seg_len - d];
+    }
+    uint32_t at = block_excl_scan2(sum, all).x;
+    for (uint32_t d = d0; d < d0 + per && d <= pb.seg_len; d++) {
+      bin_base[pb.seg_len - d] = at;
+      at += pb.len_hist[pb.seg_len - d];
+    }
+  }
   __syncthreads();
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   bool live = b < pb.n_buckets && !pb.counters[CNT_ERROR];
@@ -587,7 +639,7 @@ __global__ void __launch_bounds__(256) k_tasks(PassBuffers pb) {
   __syncthreads();
   for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x) {
     const uint32_t c = bin_cnt[i];
-    bin_base[i] = c ? atomicAdd(&pb.len_hist[i], c) : 0u;
+    if (c) bin_base[i] += atomicAdd(&pb.len_hist[pb.seg_len + 1 + i], c);
   }
   __syncthreads();
   if (live) {
@@ -1089,25 +1141,6 @@ __global__ void __launch_bounds__(128, 4) k_accumulate_quad(PassBuffers pb) {
   }
 }
 
-// k_merge_small with a quad per split bucket
-__global__ void __launch_bounds__(128) k_merge_quad(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  const uint32_t nheavy = pb.counters[CNT_HEAVY];
-  const uint32_t mask = dq_mask();
-  const uint32_t stride = gridDim.x * (blockDim.x / 4);
-  for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; h < nheavy; h += stride) {
-    const uint32_t b = pb.heavy[h];
-    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt > kMergeThreadMax) continue;
-    const uint32_t t0 = pb.taskoff[b];
-    fq_t acc = dq_load(pb.partials + (size_t)t0 * 12);
-#pragma unroll 1
-    for (uint32_t k = 1; k < nt; k++) acc = dq_add(acc, dq_load(pb.partials + (size_t)(t0 + k) * 12), mask);
-    dq_store(pb.partials + (size_t)t0 * 12, acc);
-  }
-}
-
 // k_reduce1 with a quad per run of buckets.  A + R right after the first live bucket, with an empty
 // one between, is a doubling: it is taken as one.
 __global__ void __launch_bounds__(128) k_reduce1_quad(PassBuffers pb) {
@@ -1334,17 +1367,14 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
 
 // Buckets split into more than kMergeWarpMax runs: a block of 64 quads per bucket, each quad
 // summing a strided share of the partials, then a tree over the quads in shared memory.
-__global__ void __launch_bounds__(kRedThreads) k_merge_big(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  __shared__ uint4 sh[kRedQuads * 12];
+__device__ __forceinline__ void merge_big(const PassBuffers &pb, uint32_t more_than, uint4 *sh) {
   const uint32_t q = threadIdx.x >> 2;
   const uint32_t warp_q0 = (threadIdx.x >> 5) * 8;  // first quad of this warp
   const uint32_t nheavy = pb.counters[CNT_HEAVY];
   for (uint32_t h = blockIdx.x; h < nheavy; h += gridDim.x) {
     const uint32_t b = pb.heavy[h];
     const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt <= kMergeWarpMax) continue;  // block-uniform
+    if (nt <= more_than) continue;  // block-uniform
     const uint32_t t0 = pb.taskoff[b];
     fq_t acc = dq_identity();
 #pragma unroll 1
@@ -1366,6 +1396,36 @@ __global__ void __launch_bounds__(kRedThreads) k_merge_big(PassBuffers pb) {
     if (threadIdx.x < 4) dq_store(pb.partials + (size_t)t0 * 12, acc);
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kRedThreads) k_merge_big(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  __shared__ uint4 sh[kRedQuads * 12];
+  merge_big(pb, kMergeWarpMax, sh);
+}
+
+// All split buckets of a small pass in one kernel: a quad per bucket of at most kMergeThreadMax runs,
+// then a block per larger one.
+__global__ void __launch_bounds__(kRedThreads) k_merge_quad(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  __shared__ uint4 sh[kRedQuads * 12];
+  const uint32_t nheavy = pb.counters[CNT_HEAVY];
+  const uint32_t mask = dq_mask();
+  const uint32_t stride = gridDim.x * (blockDim.x / 4);
+  for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; h < nheavy; h += stride) {
+    const uint32_t b = pb.heavy[h];
+    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
+    if (nt > kMergeThreadMax) continue;
+    const uint32_t t0 = pb.taskoff[b];
+    fq_t acc = dq_load(pb.partials + (size_t)t0 * 12);
+#pragma unroll 1
+    for (uint32_t k = 1; k < nt; k++) acc = dq_add(acc, dq_load(pb.partials + (size_t)(t0 + k) * 12), mask);
+    dq_store(pb.partials + (size_t)t0 * 12, acc);
+  }
+  __syncthreads();
+  merge_big(pb, kMergeThreadMax, sh);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1543,7 +1603,10 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   }
   mark(1);
   const uint32_t nblk = (pb.n_buckets + kScanBlock - 1) / kScanBlock;
-  if (nblk > 0) {
+  const bool scan_small = nblk <= kScanSmallBlocks;
+  if (nblk > 0 && scan_small) {
+    run(k_scan_small, nblk, kScanThreads, (pb.seg_len + 1) * 4, pb);
+  } else if (nblk > 0) {
     run(k_scan_reduce, nblk, kScanThreads, 0, pb);
     run(k_scan_blocks, 1, kScanThreads, 0, pb, nblk);
     run(k_scan_apply, nblk, kScanThreads, 0, pb);
@@ -1561,8 +1624,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   }
   mark(3);
   if (pb.n_buckets > 0) {
-    run(k_len_hist, num_sms * 4, 256, (pb.seg_len + 1) * 4, pb);
-    run(k_len_scan, 1, 32, 0, pb);
+    if (!scan_small) run(k_len_hist, num_sms * 4, 256, (pb.seg_len + 1) * 4, pb);
     run(k_tasks, (pb.n_buckets + 255) / 256, 256, 2 * (pb.seg_len + 1) * 4, pb);
   }
   mark(4);
@@ -1572,12 +1634,13 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   else
     run(k_accumulate, acc_blocks, 128, 0, pb);
   mark(5);
-  if (pb.quads)
-    run(k_merge_quad, num_sms * 4, 128, 0, pb);
-  else
+  if (pb.quads) {
+    run(k_merge_quad, num_sms * 2, kRedThreads, 0, pb);
+  } else {
     run(k_merge_small, num_sms * 4, 128, 0, pb);
-  run(k_merge, num_sms, 256, 0, pb);
-  run(k_merge_big, num_sms * 3, kRedThreads, 0, pb);
+    run(k_merge, num_sms, 256, 0, pb);
+    run(k_merge_big, num_sms * 3, kRedThreads, 0, pb);
+  }
   mark(6);
   if (pb.n_segs > 0) {
     if (pb.n_segs <= kReduceQuadSegs)
