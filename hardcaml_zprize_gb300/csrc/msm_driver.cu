@@ -778,20 +778,13 @@ bool host_pullable(const Ctx *cx, const void *h) {
   return cx->host_pull && h && ((uintptr_t)h & 15u) == 0;
 }
 
-// Run a list of MSMs whose scalars are in host memory (d_scalars == nullptr) or already on the
-// device.  mode 1: one pass per MSM with the next MSM's scalars copied during the current pass;
-// mode 2: all MSMs in one pass with one shared sort.
-int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
-             const std::vector<uint64_t> &offs, const biginteger256_t *h_scalars,
-             const void *d_scalars, const msm_options_t *opt) {
+// Run MSMs whose bases are known to be resident.  mode 1: one pass per MSM with the next MSM's scalars
+// copied during the current pass; mode 2: all MSMs in one pass with one shared sort.
+int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
+                const std::vector<uint64_t> &offs, const biginteger256_t *h_scalars,
+                const void *d_scalars, const msm_options_t *opt, int mode) {
   const size_t m = sizes.size();
   if (m == 0) return 0;
-  for (size_t j = 0; j < m; j++)
-    if (offs[j] > cx->npoints || sizes[j] > cx->npoints - offs[j])
-      return fail(ERR_ARG, "MSM %zu: bases [%llu, %llu) outside the %llu resident bases", j,
-                  (unsigned long long)offs[j], (unsigned long long)(offs[j] + sizes[j]),
-                  (unsigned long long)cx->npoints);
-  const int mode = (opt && opt->mode == 2) ? 2 : 1;
   const bool use_graph = !(opt && opt->use_graph == 2) && !cx->timing;
   Workspace &ws = cx->ws;
   std::vector<uint64_t> first(m + 1, 0);
@@ -892,6 +885,46 @@ int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
   }
   if (check_pass_errors(ws, cx->stream, cx->timing ? nullptr : cx->last_stats)) return g_err;
   memcpy(out, ws.res_host.p, m * MSM_PROJ_BYTES);
+  return 0;
+}
+
+// Points of one shared pass when the caller leaves the mode open.  A pass ends in serial reductions
+// and a final map (0.2 ms) and a small one leaves the GPU idle; together the MSMs share both.  Measured
+// on GB300 (host scalars, one pass per MSM / shared, ms): 4 x 4096 1.19 / 0.49, 4 x 50000 2.37 / 1.53,
+// 4 x 2^18 6.33 / 4.87, 4 x 2^20 15.75 / 14.46, 2 x 2^21 14.72 / 14.08.  Larger groups gain less and
+// their sort and partial sums take more memory (about 1.5 GB at this limit).
+constexpr uint64_t kSharePoints = 1ull << 22;
+
+// Run a list of MSMs whose scalars are in host memory (d_scalars == nullptr) or already on the
+// device, in the mode the options ask for, or else with consecutive MSMs of at most kSharePoints
+// points together in one pass.
+int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
+             const std::vector<uint64_t> &offs, const biginteger256_t *h_scalars,
+             const void *d_scalars, const msm_options_t *opt) {
+  const size_t m = sizes.size();
+  for (size_t j = 0; j < m; j++)
+    if (offs[j] > cx->npoints || sizes[j] > cx->npoints - offs[j])
+      return fail(ERR_ARG, "MSM %zu: bases [%llu, %llu) outside the %llu resident bases", j,
+                  (unsigned long long)offs[j], (unsigned long long)(offs[j] + sizes[j]),
+                  (unsigned long long)cx->npoints);
+  if (m <= 1 || (opt && opt->mode > 0))
+    return run_msms_as(cx, out, sizes, offs, h_scalars, d_scalars, opt, opt && opt->mode == 2 ? 2 : 1);
+  // the next group: MSMs that share a pass, or a run of MSMs that each need one of their own
+  uint64_t first = 0;
+  for (size_t a = 0; a < m;) {
+    uint64_t points = sizes[a];
+    size_t b = a + 1;
+    while (b < m && points + sizes[b] <= kSharePoints) points += sizes[b++];
+    const int mode = b > a + 1 ? 2 : 1;
+    if (mode == 1)
+      while (b < m && (b + 1 == m || sizes[b] + sizes[b + 1] > kSharePoints)) points += sizes[b++];
+    const std::vector<uint64_t> sz(sizes.begin() + a, sizes.begin() + b), of(offs.begin() + a, offs.begin() + b);
+    if (int rc = run_msms_as(cx, out + a, sz, of, h_scalars ? h_scalars + first : nullptr,
+                             d_scalars ? (const char *)d_scalars + first * 32 : nullptr, opt, mode))
+      return rc;
+    first += points;
+    a = b;
+  }
   return 0;
 }
 

@@ -93,7 +93,7 @@ typedef struct {
   int32_t seg_len;       /* max entries one thread accumulates before a bucket is split */
   int32_t red_len_log2;  /* log2 of buckets per level-1 reduction segment */
   int32_t use_graph;     /* 1 replay the pass from a captured CUDA graph, 2 never, 0 auto */
-  int32_t mode;          /* msm_mult: 1 one pass per MSM (default), 2 all MSMs in one pass */
+  int32_t mode;          /* 1 one pass per MSM, 2 all MSMs in one pass, 0 auto (small MSMs share passes) */
   int32_t fixed_base;    /* 1 use the context's fixed-base tables, 2 never, 0 auto (cost model) */
 } msm_options_t;
 
@@ -109,7 +109,8 @@ int msm_mult_ex(void *context, g1_projective_t *out, uint64_t batch_size,
 
 /* Many MSMs of uneven sizes in one pass with one shared sort. MSM j uses sizes[j] bases starting
  * at base_offsets[j] and the next sizes[j] scalars of the concatenated `scalars` array.
- * opt->mode == 1 runs them one pass per MSM instead (the plain form). */
+ * opt->mode == 1 runs them one pass per MSM instead (the plain form); 0 groups them into passes of
+ * a few million points. */
 int msm_mult_uneven(void *context, g1_projective_t *out, uint64_t num_msms, const uint64_t *sizes,
                     const uint64_t *base_offsets, const biginteger256_t *scalars,
                     const msm_options_t *opt);

@@ -73,3 +73,28 @@ def test_noalloc_layouts(engine, ocpu, monkeypatch, n, tables):
     finally:
         ctx.close()
     assert np.array_equal(d_out.cpu().numpy(), ocpu.msm(pts[3:], sc))
+
+
+def test_groups_of_an_open_mode(engine, ocpu):
+    """Without a mode, consecutive MSMs share passes up to 2^22 points; MSMs around that limit, empty
+    ones and small ones on either side, host and device scalars, as one pass each."""
+    import torch
+
+    nbase = (1 << 22) + 5
+    pts = engine.generate_bases(61, 1 << 12)
+    pts = np.concatenate([pts] * ((nbase >> 12) + 1))[:nbase]
+    sizes = [10, 0, 3000, 1 << 22, (1 << 22) - 3, 4, 7, nbase, 0, 1]
+    offs = [5, 9, 100, 2, 0, nbase - 4, 1, 0, nbase, 77]
+    sc = engine.generate_scalars(62, 1 << 16)
+    sc = np.concatenate([sc] * ((sum(sizes) >> 16) + 1))[:sum(sizes)]
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        want = ctx.mult_uneven(sizes, offs, sc, mode=1)
+        assert np.array_equal(ctx.mult_uneven(sizes, offs, sc), want)
+        d_sc = torch.from_numpy(np.ascontiguousarray(sc).view(np.uint8).reshape(-1)).cuda()
+        torch.cuda.synchronize()
+        assert np.array_equal(ctx.mult_device(sizes, offs, d_sc.data_ptr()), want)
+        at = sum(sizes[:2])
+        assert np.array_equal(want[2], ocpu.msm(pts[100:3100], sc[at:at + 3000]))
+    finally:
+        ctx.close()
