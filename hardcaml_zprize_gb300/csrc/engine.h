@@ -60,9 +60,9 @@ struct Task {             // a run of sorted entries that one thread accumulates
 
 enum : int {
   CNT_TASKS = 0,          // number of tasks built
-  CNT_HEAVY = 1,          // buckets split over more than one task
+  CNT_HEAVY = 1,          // buckets split over a few tasks
   CNT_TASK_CURSOR = 2,    // persistent accumulate work counter
-  CNT_HEAVY_CURSOR = 3,
+  CNT_BIG = 3,            // buckets split over many
   CNT_ERROR = 4,          // nonzero: a device-side bounds check fired (code)
   CNT_ERROR_INFO = 5,
   CNT_ENTRIES = 6,        // sorted entries of the pass (nonzero digits)
@@ -96,6 +96,7 @@ struct PassBuffers {
   uint32_t n_buckets;           // global bucket count
   uint32_t n_segs;              // level-1 reduction segments
   uint32_t seg_len;             // max entries per accumulate task
+  uint32_t seg_shift;           // its log2, or 32 where it is no power of two
   uint32_t red_len_log2;        // level-1 reduction segment length = 1 << red_len_log2
   uint32_t grp_len_log2;        // level-2 group = 1 << grp_len_log2 level-1 segments
   uint32_t n_grps;              // level-2 groups
@@ -123,7 +124,7 @@ struct PassBuffers {
   uint32_t *vals;               // [max_entries]
   Task *tasks;                  // [max_tasks]
   uint4 *partials;              // [max_tasks] x 12 uint4
-  uint32_t *heavy;              // [n_buckets]
+  uint32_t *heavy;              // [n_buckets] split buckets: of few tasks from the front, of many from the back
   uint32_t *order;              // [max_tasks] task ids, longest first
   uint32_t *len_hist;           // [seg_len + 1] task-length histogram, then as many slot cursors
   uint32_t *counters;           // [CNT_WORDS]

@@ -345,28 +345,23 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl) {
     }
     pl.red_log2 = red_log2_for(total);
   }
-  // Level-2 groups of 2^grp_log2 level-1 runs.  A pass whose reduction is one window (one MSM on
-  // fixed-base tables) takes groups of 128 to 512 runs, about 128 groups: level 3 then combines
-  // enough groups to use a block (a window of at most 16 groups is combined serially by one
-  // quad) and few enough to keep its tree shallow.  Measured on GB300 (ms per MSM, groups of
-  // 512 / 256 / 128 runs): 2^12 and 2^16 points (4096 runs) 0.973 / 0.993 / 0.850 and 1.427 /
-  // 1.448 / 1.300; 2^20 (32 K runs) 6.290 / 6.219 / 6.307; 2^24 (76 K runs) 71.58 / 71.79 / 72.10.
-  // Passes of many windows (windowed MSMs, batches) keep groups of 512: the uneven 64-MSM mix
-  // (64 windows of 2048 runs) took 34.44 ms with them and 34.99 ms with groups of 128, whose
-  // 1024 level-2 blocks run in several waves.
+  // Level-2 groups of 128 to 512 level-1 runs, at most about 128 groups while that allows: more blocks
+  // than SMs run in several waves, fewer and longer ones leave SMs idle behind longer serial sums.  A
+  // window of more than 16 groups is then combined by a block, one of fewer serially by one quad.
+  // Measured on GB300 (levels 2 + 3, us, groups of 128 / 256 / 512 runs): 2^12 points (8192 runs) 129 /
+  // 158 / -, 2^20 (32 K runs) 215 / 200 / 219; a shared pass of 4 x 50000 (16 K runs) 103 / - / 187;
+  // the uneven mix of 64 (131 K runs) keeps 512.
   {
-    uint32_t n_windows = 0;
-    uint64_t max_nb = 0;
+    uint64_t runs = 0;
     for (const JobSpec &s : specs) {
       if (s.n == 0) continue;
       uint32_t nwin, nb, nbt;
       layout(s.cfg.c, s.cfg.signed_digits, nwin, nb, nbt);
-      n_windows += s.cfg.fixed ? 1 : nwin;
-      max_nb = std::max<uint64_t>(max_nb, std::max(nb, nbt));
+      const uint64_t buckets = s.cfg.fixed ? std::max(nb, nbt) : (uint64_t)(nwin - 1) * nb + nbt;
+      runs += (buckets + (1ull << pl.red_log2) - 1) >> pl.red_log2;
     }
-    const uint64_t max_nseg = (max_nb + (1ull << pl.red_log2) - 1) >> pl.red_log2;
-    pl.grp_log2 = n_windows == 1 ? 7 : 9;
-    while (pl.grp_log2 < 9 && (max_nseg >> pl.grp_log2) > 128) pl.grp_log2++;
+    pl.grp_log2 = 7;
+    while (pl.grp_log2 < 9 && (runs >> pl.grp_log2) > 128) pl.grp_log2++;
   }
   uint64_t buckets = 0, segs = 0, wins = 0, grps = 0;
   char tmp[160];
@@ -572,6 +567,8 @@ void set_tables(const Ctx *cx, JobSpec &s) {
   s.tab_base = s.cfg.fixed == 2 ? cx->npoints * cx->fb_w : 0;
 }
 
+uint32_t seg_shift_of(uint32_t seg_len) { return seg_len & (seg_len - 1) ? 32u : (uint32_t)__builtin_ctz(seg_len); }
+
 PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void *d_scalars) {
   PassBuffers pb{};
   pb.acc_blocks_per_sm = ws.acc_blocks_per_sm;
@@ -594,6 +591,7 @@ PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void
   pb.n_segs = pl.n_segs;
   pb.n_grps = pl.n_grps;
   pb.seg_len = pl.seg_len;
+  pb.seg_shift = seg_shift_of(pl.seg_len);
   pb.red_len_log2 = pl.red_log2;
   pb.grp_len_log2 = pl.grp_log2;
   pb.max_entries = pl.max_entries;
@@ -680,7 +678,7 @@ int check_pass_errors(Workspace &ws, cudaStream_t st, uint64_t *stats_out) {
   CK(cudaStreamSynchronize(st));
   if (stats_out) {
     stats_out[0] = cnt[CNT_TASKS];
-    stats_out[1] = cnt[CNT_HEAVY];
+    stats_out[1] = cnt[CNT_HEAVY] + cnt[CNT_BIG];
     stats_out[2] = cnt[CNT_ENTRIES];
   }
   if (cnt[CNT_ERROR]) {
@@ -2259,6 +2257,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.n_segs = nsegs;
   pb.n_grps = ngrps;
   pb.seg_len = seg_len;
+  pb.seg_shift = seg_shift_of(seg_len);
   pb.red_len_log2 = red_log2;
   pb.grp_len_log2 = grp_log2;
   pb.max_entries = entries;

@@ -155,24 +155,8 @@ __device__ __forceinline__ void count_digits(const PassBuffers &pb, const JobDes
 }
 
 // Round 2 of the staged sort: one entry into the block's chunk, at the cursor of its key range.
-__device__ __forceinline__ void stage_key(const PassBuffers &pb, uint32_t key, uint32_t val,
+__device__ __forceinline__ void stage_key(const PassBuffers &pb, uint32_t key, uint32_t val, uint32_t rank,
                                           uint32_t *sh_cur, uint2 *chunk, uint32_t *ranks) {
-  uint32_t rank = 0;
-  if (ranks) {
-    // the bucket count's old value is the entry's rank in its bucket (one atomic per warp
-    // when its active lanes share the bucket)
-    const uint32_t active = __activemask();
-    const int leader = __ffs(active) - 1;
-    const int lane = threadIdx.x & 31;
-    const uint32_t k0 = __shfl_sync(active, key, leader);
-    if (__all_sync(active, key == k0)) {
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(&pb.count[key], (uint32_t)__popc(active));
-      rank = __shfl_sync(active, base, leader) + __popc(active & ((1u << lane) - 1u));
-    } else {
-      rank = atomicAdd(&pb.count[key], 1u);
-    }
-  }
   const uint32_t pos = atomicAdd(&sh_cur[key >> pb.bin_shift], 1u);
   if (pos < pb.stage_cap) {
     chunk[pos] = make_uint2(key, val);
@@ -182,21 +166,77 @@ __device__ __forceinline__ void stage_key(const PassBuffers &pb, uint32_t key, u
   }
 }
 
-// The entries of one point, in window order.
+// The entries of one point, in window order; with ranks four windows per step, so that their atomics
+// on the bucket counts are in flight together (a small pass is bound by their round trips: k_count of
+// 4096 points 16 -> 13 us; without ranks one by one, 2^24 points 1.07 -> 1.03 ms).  A bucket count's
+// old value is the entry's rank in its bucket; one atomic per warp when its active lanes share the bucket.
 __device__ __forceinline__ void stage_digits(const PassBuffers &pb, const JobDesc &jd, ScalarBits s,
                                              uint64_t bidx, uint32_t *sh_cur, uint2 *chunk,
                                              uint32_t *ranks) {
+  const int lane = threadIdx.x & 31;
   uint32_t carry = 0;
-  for (uint32_t w = 0; w < jd.nwin; w++) {
-    const int32_t d = next_digit(s, jd, w, carry);
-    if (d == 0) continue;
-    const uint32_t mag = (uint32_t)abs(d);
-    const uint32_t extra = top_excess(jd, w, mag);
-    const uint64_t tidx = jd.tab_base + (jd.fixed ? (uint64_t)w * jd.fb_stride : 0) + bidx;
-    const uint32_t val = (uint32_t)tidx | (d < 0 ? 0x80000000u : 0u);
-    stage_key(pb, bucket_key(jd, w, mag - extra), val, sh_cur, chunk, ranks);
-    if (extra) stage_key(pb, bucket_key(jd, w, extra), val, sh_cur, chunk, ranks);
+  if (!ranks) {
+    for (uint32_t w = 0; w < jd.nwin; w++) {
+      const int32_t d = next_digit(s, jd, w, carry);
+      if (d == 0) continue;
+      const uint32_t mag = (uint32_t)abs(d);
+      const uint32_t ex = top_excess(jd, w, mag);
+      const uint64_t tidx = jd.tab_base + (jd.fixed ? (uint64_t)w * jd.fb_stride : 0) + bidx;
+      const uint32_t val = (uint32_t)tidx | (d < 0 ? 0x80000000u : 0u);
+      stage_key(pb, bucket_key(jd, w, mag - ex), val, 0, sh_cur, chunk, nullptr);
+      if (ex) stage_key(pb, bucket_key(jd, w, ex), val, 0, sh_cur, chunk, nullptr);
+    }
+    return;
   }
+  uint32_t extra_key = 0, extra_val = 0;  // a split top digit's second entry (see top_excess)
+  bool extra = false;
+#pragma unroll 1
+  for (uint32_t w0 = 0; w0 < jd.nwin; w0 += 4) {
+    uint32_t key[4], val[4], rank[4], act[4];  // act: the lanes that share the atomic, or 0
+    bool ok[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t w = w0 + k;
+      ok[k] = false;
+      key[k] = val[k] = rank[k] = act[k] = 0;
+      if (w >= jd.nwin) continue;
+      const int32_t d = next_digit(s, jd, w, carry);
+      if (d == 0) continue;
+      const uint32_t mag = (uint32_t)abs(d);
+      const uint32_t ex = top_excess(jd, w, mag);
+      const uint64_t tidx = jd.tab_base + (jd.fixed ? (uint64_t)w * jd.fb_stride : 0) + bidx;
+      ok[k] = true;
+      key[k] = bucket_key(jd, w, mag - ex);
+      val[k] = (uint32_t)tidx | (d < 0 ? 0x80000000u : 0u);
+      if (ex) {
+        extra = true;
+        extra_key = bucket_key(jd, w, ex);
+        extra_val = val[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (!ok[k]) continue;
+      const uint32_t active = __activemask();
+      const int leader = __ffs(active) - 1;
+      const uint32_t k0 = __shfl_sync(active, key[k], leader);
+      if (__all_sync(active, key[k] == k0)) {
+        act[k] = active;
+        if (lane == leader) rank[k] = atomicAdd(&pb.count[key[k]], (uint32_t)__popc(active));
+      } else {
+        rank[k] = atomicAdd(&pb.count[key[k]], 1u);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (act[k])
+        rank[k] = __shfl_sync(act[k], rank[k], __ffs(act[k]) - 1) + __popc(act[k] & ((1u << lane) - 1u));
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (ok[k]) stage_key(pb, key[k], val[k], rank[k], sh_cur, chunk, ranks);
+  }
+  if (extra)
+    stage_key(pb, extra_key, extra_val, atomicAdd(&pb.count[extra_key], 1u), sh_cur, chunk, ranks);
 }
 
 // One thread per point, 256 points per block.  With host_scalars set, the kernel also uploads
@@ -294,8 +334,9 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint2 v, uint2 &total) {
   return make_uint2(base.x + inc.x - v.x, base.y + inc.y - v.y);
 }
 
-__device__ __forceinline__ uint32_t ntask_of(uint32_t cnt, uint32_t seg_len) {
-  return (cnt + seg_len - 1) / seg_len;
+__device__ __forceinline__ uint32_t ntask_of(uint32_t cnt, const PassBuffers &pb) {
+  const uint32_t c = cnt + pb.seg_len - 1;
+  return pb.seg_shift < 32 ? c >> pb.seg_shift : c / pb.seg_len;  // the automatic run lengths are powers of two
 }
 
 // the pass's entries and tasks, against the plan's room
@@ -315,7 +356,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(PassBuffers pb) {
     if (base + k < pb.n_buckets) {
       const uint32_t c = pb.count[base + k];
       v.x += c;
-      v.y += ntask_of(c, pb.seg_len);
+      v.y += ntask_of(c, pb);
     }
   }
   uint2 total;
@@ -358,7 +399,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
   for (int k = 0; k < kScanItems; k++) {
     c[k] = base + k < pb.n_buckets ? pb.count[base + k] : 0u;
     v.x += c[k];
-    v.y += ntask_of(c[k], pb.seg_len);
+    v.y += ntask_of(c[k], pb);
   }
   uint2 total;
   uint2 ex = block_excl_scan2(v, total);
@@ -372,7 +413,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
-    ex.y += ntask_of(c[k], pb.seg_len);
+    ex.y += ntask_of(c[k], pb);
   }
 }
 
@@ -389,7 +430,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
   for (uint32_t i = threadIdx.x; i < blockIdx.x * kScanBlock; i += blockDim.x) {
     const uint32_t c = pb.count[i];
     before.x += c;
-    before.y += ntask_of(c, pb.seg_len);
+    before.y += ntask_of(c, pb);
   }
   block_excl_scan2(before, before);
   const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
@@ -398,7 +439,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
     c[k] = base + k < pb.n_buckets ? pb.count[base + k] : 0u;
-    const uint32_t nt = ntask_of(c[k], pb.seg_len);
+    const uint32_t nt = ntask_of(c[k], pb);
     v.x += c[k];
     v.y += nt;
     if (nt) {
@@ -417,7 +458,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
-    ex.y += ntask_of(c[k], pb.seg_len);
+    ex.y += ntask_of(c[k], pb);
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x)
@@ -515,16 +556,16 @@ __global__ void k_scatter(PassBuffers pb, uint32_t key_lo, uint32_t key_hi) {
 // Staged sort: the entries of key range `bin`, chunk by chunk (one block per histogram block),
 // each to the position its bucket's slot cursor returns.  The range's slice of the sorted array
 // stays in L2 while the launch runs.
-__global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t bin) {
+__global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t bin, uint32_t parts) {
   pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
-  const uint64_t chunk = blockIdx.x;
+  const uint64_t chunk = blockIdx.x / parts;
   const uint32_t *bo = pb.blk_off + chunk * (pb.n_bins + 1);
   const uint32_t lo = bo[bin], hi = min(bo[bin + 1], pb.stage_cap);
   const uint2 *st = pb.stage + chunk * pb.stage_cap;
   const uint32_t *rk = pb.stage_rank ? pb.stage_rank + chunk * pb.stage_cap : nullptr;
   const int lane = threadIdx.x & 31;
-  for (uint32_t e = lo + threadIdx.x; e < hi; e += blockDim.x) {
+  for (uint32_t e = lo + (blockIdx.x % parts) * blockDim.x + threadIdx.x; e < hi; e += parts * blockDim.x) {
     const uint2 kv = st[e];
     if (kv.x >= pb.n_buckets) {  // cannot happen for a consistent stage; never write out of bounds
       set_error(pb.counters, 7, kv.x);
@@ -571,7 +612,7 @@ __global__ void k_len_hist(PassBuffers pb) {
   for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < pb.n_buckets; b += gridDim.x * blockDim.x) {
     const uint32_t cnt = pb.count[b];
     if (!cnt) continue;
-    const uint32_t nt = ntask_of(cnt, pb.seg_len);
+    const uint32_t nt = ntask_of(cnt, pb);
     atomicAdd(&h[cnt - (nt - 1) * pb.seg_len], 1u);
     if (nt > 1) atomicAdd(&h[pb.seg_len], nt - 1);
   }
@@ -579,6 +620,9 @@ __global__ void k_len_hist(PassBuffers pb) {
   for (uint32_t i = threadIdx.x; i <= pb.seg_len; i += blockDim.x)
     if (h[i]) atomicAdd(&pb.len_hist[i], h[i]);
 }
+
+// Split buckets of at most this many runs are summed by one quad each, larger ones by a block.
+constexpr uint32_t kMergeQuadMax = 16;
 
 // One thread per bucket writes the bucket's runs and their slots in the processing order: the
 // last run takes a slot in the bin of its length, the full runs of a split bucket a block of
@@ -612,7 +656,7 @@ __global__ void __launch_bounds__(256) k_tasks(PassBuffers pb) {
     live = cnt != 0;
   }
   if (live) {
-    nt = ntask_of(cnt, pb.seg_len);
+    nt = ntask_of(cnt, pb);
     t0 = pb.taskoff[b];
     if (t0 + nt > pb.max_tasks) {
       set_error(pb.counters, 4, t0 + nt);
@@ -633,7 +677,8 @@ __global__ void __launch_bounds__(256) k_tasks(PassBuffers pb) {
     r_last = atomicAdd(&bin_cnt[last], 1u);
     if (nt > 1) {
       r_full = atomicAdd(&bin_cnt[pb.seg_len], nt - 1);
-      pb.heavy[atomicAdd(&pb.counters[CNT_HEAVY], 1u)] = b;
+      if (nt <= kMergeQuadMax) pb.heavy[atomicAdd(&pb.counters[CNT_HEAVY], 1u)] = b;
+      else pb.heavy[pb.n_buckets - 1 - atomicAdd(&pb.counters[CNT_BIG], 1u)] = b;
     }
   }
   __syncthreads();
@@ -737,86 +782,6 @@ __global__ void __launch_bounds__(128, 4) k_accumulate(PassBuffers pb) {
       }
       xyzt_store(pb.partials + (size_t)t * 12, acc);
     }
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// 6. buckets spread over several tasks: one warp sums the partials
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ xyzt_t shfl_down_xyzt(const xyzt_t &p, int off) {
-  xyzt_t r;
-#pragma unroll
-  for (int k = 0; k < FQ_LIMBS; k++) {
-    r.x.v[k] = __shfl_down_sync(0xffffffffu, p.x.v[k], off);
-    r.y.v[k] = __shfl_down_sync(0xffffffffu, p.y.v[k], off);
-    r.z.v[k] = __shfl_down_sync(0xffffffffu, p.z.v[k], off);
-    r.t.v[k] = __shfl_down_sync(0xffffffffu, p.t.v[k], off);
-  }
-  return r;
-}
-
-__device__ __forceinline__ xyzt_t warp_sum_xyzt(xyzt_t acc) {
-#pragma unroll 1
-  for (int off = 16; off > 0; off >>= 1) {
-    const xyzt_t o = shfl_down_xyzt(acc, off);
-    acc = te_add_ool(acc, o);  // lanes >= 32 - off add garbage-free copies; only lane 0 is used
-  }
-  return acc;
-}
-
-// Split buckets of at most kMergeThreadMax runs (the common case: a few more entries than
-// seg_len) are summed by one thread each, larger ones by a warp (k_merge) or a block
-// (k_merge_big).  Lanes of a warp
-// execute one instruction stream, so a warp's tree over three partials costs as much as the
-// thread version summing 32 such buckets.
-constexpr uint32_t kMergeThreadMax = 16;
-
-__global__ void __launch_bounds__(128) k_merge_small(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  const uint32_t nheavy = pb.counters[CNT_HEAVY];
-  for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < nheavy; h += gridDim.x * blockDim.x) {
-    const uint32_t b = pb.heavy[h];
-    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt > kMergeThreadMax) continue;
-    const uint32_t t0 = pb.taskoff[b];
-    xyzt_t acc;
-    xyzt_load(acc, pb.partials + (size_t)t0 * 12);
-    for (uint32_t k = 1; k < nt; k++) {
-      xyzt_t p;
-      xyzt_load(p, pb.partials + (size_t)(t0 + k) * 12);
-      acc = te_add_fast_ool(acc, p);  // partials of disjoint runs: the dedicated formula
-    }
-    xyzt_store(pb.partials + (size_t)t0 * 12, acc);
-  }
-}
-
-// Buckets of more than kMergeWarpMax runs (a value repeated across many scalars) get a block of
-// 64 quads each (k_merge_big, after the quad arithmetic below).
-constexpr uint32_t kMergeWarpMax = 64;
-
-__global__ void __launch_bounds__(256) k_merge(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nheavy = pb.counters[CNT_HEAVY];
-  const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t h = warp_global; h < nheavy; h += nwarps) {
-    const uint32_t b = pb.heavy[h];
-    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt <= kMergeThreadMax || nt > kMergeWarpMax) continue;  // k_merge_small's, k_merge_big's
-    const uint32_t t0 = pb.taskoff[b];
-    xyzt_t acc = xyzt_identity();
-    for (uint32_t k = lane; k < nt; k += 32) {
-      xyzt_t p;
-      xyzt_load(p, pb.partials + (size_t)(t0 + k) * 12);
-      acc = te_add_ool(acc, p);
-    }
-    acc = warp_sum_xyzt(acc);
-    __syncwarp();
-    if (lane == 0) xyzt_store(pb.partials + (size_t)t0 * 12, acc);
-    __syncwarp();
   }
 }
 
@@ -1365,16 +1330,36 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
   if (threadIdx.x < 4) dq_store(pb.win_sum + (size_t)gw * 12, A);
 }
 
-// Buckets split into more than kMergeWarpMax runs: a block of 64 quads per bucket, each quad
-// summing a strided share of the partials, then a tree over the quads in shared memory.
-__device__ __forceinline__ void merge_big(const PassBuffers &pb, uint32_t more_than, uint4 *sh) {
+// ---------------------------------------------------------------------------------------------
+// 6. buckets spread over several tasks: a quad per bucket of at most kMergeQuadMax runs (the common
+//    case: a few more entries than seg_len), then a block of 64 quads per larger one (a value repeated
+//    across many scalars): each quad sums a strided share of the partials, a tree over the quads in
+//    shared memory the rest.  A thread, a warp or a block per bucket, in three kernels that each walked
+//    the whole list, took (us, then now) 68 / 23 at 2^20 points, 386 / 72 in a shared pass of 4 x 50000
+//    (121e3 split buckets), 364 / 103 in the uneven mix of 64.
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(kRedThreads) k_merge(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  __shared__ uint4 sh[kRedQuads * 12];
+  const uint32_t nsmall = pb.counters[CNT_HEAVY], nbig = pb.counters[CNT_BIG];
+  const uint32_t mask = dq_mask();
+  const uint32_t quads = gridDim.x * (blockDim.x / 4);
+  for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; h < nsmall; h += quads) {
+    const uint32_t b = pb.heavy[h];
+    const uint32_t nt = ntask_of(pb.count[b], pb);
+    const uint32_t t0 = pb.taskoff[b];
+    fq_t acc = dq_load(pb.partials + (size_t)t0 * 12);
+#pragma unroll 1
+    for (uint32_t k = 1; k < nt; k++) acc = dq_add(acc, dq_load(pb.partials + (size_t)(t0 + k) * 12), mask);
+    dq_store(pb.partials + (size_t)t0 * 12, acc);
+  }
+  __syncthreads();
   const uint32_t q = threadIdx.x >> 2;
   const uint32_t warp_q0 = (threadIdx.x >> 5) * 8;  // first quad of this warp
-  const uint32_t nheavy = pb.counters[CNT_HEAVY];
-  for (uint32_t h = blockIdx.x; h < nheavy; h += gridDim.x) {
-    const uint32_t b = pb.heavy[h];
-    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt <= more_than) continue;  // block-uniform
+  for (uint32_t h = blockIdx.x; h < nbig; h += gridDim.x) {
+    const uint32_t b = pb.heavy[pb.n_buckets - 1 - h];
+    const uint32_t nt = ntask_of(pb.count[b], pb);
     const uint32_t t0 = pb.taskoff[b];
     fq_t acc = dq_identity();
 #pragma unroll 1
@@ -1396,36 +1381,6 @@ __device__ __forceinline__ void merge_big(const PassBuffers &pb, uint32_t more_t
     if (threadIdx.x < 4) dq_store(pb.partials + (size_t)t0 * 12, acc);
     __syncthreads();
   }
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_merge_big(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  __shared__ uint4 sh[kRedQuads * 12];
-  merge_big(pb, kMergeWarpMax, sh);
-}
-
-// All split buckets of a small pass in one kernel: a quad per bucket of at most kMergeThreadMax runs,
-// then a block per larger one.
-__global__ void __launch_bounds__(kRedThreads) k_merge_quad(PassBuffers pb) {
-  pdl_begin();
-  if (pb.counters[CNT_ERROR]) return;
-  __shared__ uint4 sh[kRedQuads * 12];
-  const uint32_t nheavy = pb.counters[CNT_HEAVY];
-  const uint32_t mask = dq_mask();
-  const uint32_t stride = gridDim.x * (blockDim.x / 4);
-  for (uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; h < nheavy; h += stride) {
-    const uint32_t b = pb.heavy[h];
-    const uint32_t nt = ntask_of(pb.count[b], pb.seg_len);
-    if (nt > kMergeThreadMax) continue;
-    const uint32_t t0 = pb.taskoff[b];
-    fq_t acc = dq_load(pb.partials + (size_t)t0 * 12);
-#pragma unroll 1
-    for (uint32_t k = 1; k < nt; k++) acc = dq_add(acc, dq_load(pb.partials + (size_t)(t0 + k) * 12), mask);
-    dq_store(pb.partials + (size_t)t0 * 12, acc);
-  }
-  __syncthreads();
-  merge_big(pb, kMergeThreadMax, sh);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1555,11 +1510,11 @@ size_t msm_scan_tmp_words(uint32_t n_buckets) {
 }
 
 // Level-1 reductions of at most this many runs take a quad each (k_reduce1_quad): one thread each
-// would leave the GPU idle behind a chain of 8 products per addition.  Measured on GB300, 8192 runs
-// of 4 buckets (tables of width 16): 61 us with a thread per run, 31 to 37 us with a quad; 32768
-// runs (2^20 points) keep the threads, whose work is then bound by product throughput (0.35 ms for
-// 2^19 buckets, of 0.27 at the product rate).
-constexpr uint32_t kReduceQuadSegs = 16384;
+// would leave the GPU idle behind a chain of 8 products per addition.  Measured on GB300 (us, threads /
+// quads): 8192 runs of 4 buckets (tables of width 16) 61 / 33, 32768 runs of 16 (2^20 points) 346 / 332;
+// 65536 runs of 8 there 327 / 301, but with 35 more in level 2.  Larger reductions are bound by product
+// throughput in either form.
+constexpr uint32_t kReduceQuadSegs = 32768;
 
 cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st, cudaEvent_t *ev,
                             const cudaEvent_t *chunk_ready, int nchunks, uint32_t *n_kernels) {
@@ -1613,7 +1568,10 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   }
   mark(2);
   if (pb.n_points > 0 && pb.stage) {
-    for (uint32_t r = 0; r < pb.n_bins; r++) run(k_scatter_staged, pts_blocks, 256, 0, pb, r);
+    // few chunks: several blocks each (a block walks a chunk of 256 points in ~17 dependent steps; 4096
+    // points, 16 chunks: 12.8 us with a block each, 4.6 with eight)
+    const uint32_t parts = std::max(1u, std::min(8u, (uint32_t)num_sms * 16u / pts_blocks));
+    for (uint32_t r = 0; r < pb.n_bins; r++) run(k_scatter_staged, pts_blocks * parts, 256, 0, pb, r, parts);
   } else if (pb.n_points > 0) {
     const uint32_t passes = msm_scatter_passes(pb.max_entries);
     for (uint32_t p = 0; p < passes; p++) {
@@ -1634,13 +1592,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   else
     run(k_accumulate, acc_blocks, 128, 0, pb);
   mark(5);
-  if (pb.quads) {
-    run(k_merge_quad, num_sms * 2, kRedThreads, 0, pb);
-  } else {
-    run(k_merge_small, num_sms * 4, 128, 0, pb);
-    run(k_merge, num_sms, 256, 0, pb);
-    run(k_merge_big, num_sms * 3, kRedThreads, 0, pb);
-  }
+  run(k_merge, num_sms * 2, kRedThreads, 0, pb);
   mark(6);
   if (pb.n_segs > 0) {
     if (pb.n_segs <= kReduceQuadSegs)
