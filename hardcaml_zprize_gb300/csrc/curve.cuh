@@ -111,24 +111,24 @@ static __device__ __noinline__ fq_t fq_sqr_ool(const fq_t &a) { return fq_mul(a,
 // (x1 y1 - x2 y2) / (x1 y2 - y1 x2), the twisted-Edwards sum wherever F G != 0.  This formula and
 // the unified one are polynomial maps that agree on a dense set of pairs, so their 2 x 2 minors
 // vanish everywhere: wherever F G != 0 the result is the unified formula's point.  F G = 0
-// (doubling, the identity plus a point with T = 0, ...) is tested right after the first two
-// products, and the unified formula (9 products) is used then.  E and H feed products only, so
-// they stay unreduced (below 4q).
+// (doubling, the identity plus a point with T = 0, ...) shows as Z3 = 0 modulo q, that is 0 or q, whose
+// lowest words are 0 and 1: one word tells whether to look closer, and the unified formula
+// (9 products) is used then.  Everything between two products stays unreduced (below 7q).
 __device__ __forceinline__ xyzt_t te_add_fast(const xyzt_t &p, const xyzt_t &q) {
   const fq_t A = fq_mul_nv(fq_sub_lazy(p.y, p.x), fq_add_lazy(q.y, q.x));
   const fq_t B = fq_mul_nv(fq_add_lazy(p.y, p.x), fq_sub_lazy(q.y, q.x));
-  const fq_t F = fq_sub(B, A);
-  const fq_t G = fq_add(B, A);
-  if (fq_is_zero(F) || fq_is_zero(G)) return te_add_ool(p, q);
-  const fq_t C = fq_dbl(fq_mul_nv(p.z, q.t));
-  const fq_t D = fq_dbl(fq_mul_nv(p.t, q.z));
-  const fq_t E = fq_add_lazy(D, C);
-  const fq_t H = fq_sub_lazy(D, C);
+  const fq_t F = fq_sub_lazy(B, A);
+  const fq_t G = fq_add_lazy(B, A);
   xyzt_t r;
+  r.z = fq_mul_nv(F, G);
+  if (r.z.v[0] <= 1u && fq_is_zero(r.z)) return te_add_ool(p, q);
+  const fq_t C = fq_shl_lazy(fq_mul_nv(p.z, q.t), 1);
+  const fq_t D = fq_shl_lazy(fq_mul_nv(p.t, q.z), 1);
+  const fq_t E = fq_add_lazy(D, C);
+  const fq_t H = fq_sub_lazy4(D, C);
   r.x = fq_mul_nv(E, F);
   r.y = fq_mul_nv(G, H);
   r.t = fq_mul_nv(E, H);
-  r.z = fq_mul_nv(F, G);
   return r;
 }
 

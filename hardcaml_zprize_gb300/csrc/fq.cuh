@@ -263,7 +263,7 @@ __device__ __forceinline__ fq_t fq_sub(const fq_t &a, const fq_t &b) {
 }
 
 // Unreduced forms for operands that only feed products: for a, b < 2q, a + b and a - b + 2q are
-// below 4q, and a product of two values below 4q is again below 2q (16q < 2^384).
+// below 4q, and a product of two values below 8q is below q + 64 q (q / 2^384) < 1.5q.
 __device__ __forceinline__ fq_t fq_add_lazy(const fq_t &a, const fq_t &b) {
   fq_t r;
   r.v[0] = add_cc(a.v[0], b.v[0]);
@@ -283,6 +283,28 @@ __device__ __forceinline__ fq_t fq_sub_lazy(const fq_t &a, const fq_t &b) {
 #pragma unroll
   for (int j = 1; j < FQ_LIMBS - 1; j++) r.v[j] = subc_cc(d[j], b.v[j]);
   r.v[FQ_LIMBS - 1] = subc(d[FQ_LIMBS - 1], b.v[FQ_LIMBS - 1]);
+  return r;
+}
+
+// a - b + 4q, b below 4q
+__device__ __forceinline__ fq_t fq_sub_lazy4(const fq_t &a, const fq_t &b) {
+  const uint32_t q4[FQ_LIMBS] = BLS_Q4;
+  fq_t r;
+  r.v[0] = add_cc(a.v[0], q4[0]);
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = addc_cc(a.v[j], q4[j]);
+  r.v[0] = sub_cc(r.v[0], b.v[0]);
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS - 1; j++) r.v[j] = subc_cc(r.v[j], b.v[j]);
+  r.v[FQ_LIMBS - 1] = subc(r.v[FQ_LIMBS - 1], b.v[FQ_LIMBS - 1]);
+  return r;
+}
+// a 2^s, s = 0 or 1
+__device__ __forceinline__ fq_t fq_shl_lazy(const fq_t &a, uint32_t s) {
+  fq_t r;
+  r.v[0] = a.v[0] << s;
+#pragma unroll
+  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = __funnelshift_l(a.v[j - 1], a.v[j], s);
   return r;
 }
 

@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(128) k_reduce1(PassBuffers pb) {
         // with A = R (an empty bucket right after the first live one) A + R is a doubling, the
         // dedicated formula's failure; a warp holding such a lane takes the unified formula for
         // this step instead of running both
-        if (__any_sync(__activemask(), a_is_r)) A = te_add(A, R);
+        if (__any_sync(__activemask(), a_is_r)) A = te_add_ool(A, R);
         else A = te_add_fast(A, R);
         a_is_r = false;
       }
@@ -888,9 +888,8 @@ __device__ __forceinline__ fq_t pick4(int l, const fq_t &a, const fq_t &b, const
   return fq_select(l == 0, a, fq_select(l == 1, b, fq_select(l == 2, c, d)));
 }
 
-// Sums that only feed products stay unreduced: a product of values below 8q is below
-// q + 64 q (q / 2^384) < 1.5 q, so nothing between two products needs a reduction (chains of 25 to
-// 37 dependent instructions each in a lone warp's latency).
+// Sums that only feed products stay unreduced (fq_add_lazy and the like): a reduction is a chain of 25
+// to 37 dependent instructions in a lone warp's latency.
 
 // base + term (neg 0), base - term + 2q (neg ~0), or base alone (en 0); term below 2q
 __device__ __forceinline__ fq_t fq_addsub(const fq_t &base, const fq_t &term, uint32_t en, uint32_t neg) {
@@ -905,28 +904,6 @@ __device__ __forceinline__ fq_t fq_addsub(const fq_t &base, const fq_t &term, ui
   r.v[FQ_LIMBS - 1] = addc(r.v[FQ_LIMBS - 1], q2[FQ_LIMBS - 1] & neg);
   return r;
 }
-// a - b + 4q, b below 4q
-__device__ __forceinline__ fq_t fq_sub_lazy4(const fq_t &a, const fq_t &b) {
-  const uint32_t q4[FQ_LIMBS] = BLS_Q4;
-  fq_t r;
-  r.v[0] = add_cc(a.v[0], q4[0]);
-#pragma unroll
-  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = addc_cc(a.v[j], q4[j]);
-  r.v[0] = sub_cc(r.v[0], b.v[0]);
-#pragma unroll
-  for (int j = 1; j < FQ_LIMBS - 1; j++) r.v[j] = subc_cc(r.v[j], b.v[j]);
-  r.v[FQ_LIMBS - 1] = subc(r.v[FQ_LIMBS - 1], b.v[FQ_LIMBS - 1]);
-  return r;
-}
-// a 2^s, s = 0 or 1
-__device__ __forceinline__ fq_t fq_shl_lazy(const fq_t &a, uint32_t s) {
-  fq_t r;
-  r.v[0] = a.v[0] << s;
-#pragma unroll
-  for (int j = 1; j < FQ_LIMBS; j++) r.v[j] = __funnelshift_l(a.v[j - 1], a.v[j], s);
-  return r;
-}
-
 // dbl-2008-hwcd, a = -1: A = X^2, B = Y^2, C = 2 Z^2, S = (X + Y)^2, E = S - A - B, G = B - A,
 // F = G - C, H = -A - B; X3 = E F, Y3 = G H, T3 = E H, Z3 = F G.  (F and H change sign together
 // here, F' = A + C - B and H' = A + B, which changes the signs of all four coordinates.)
