@@ -857,6 +857,8 @@ __global__ void __launch_bounds__(128) k_reduce1(PassBuffers pb) {
 }
 
 // ---- 4-lane cooperative point operations on distributed points ----
+// Choices by lane go through fq_select, word by word: the conditional operator on a whole element
+// compiles to branches that the four lanes take in turn (k_reduce2 of 2^12 points 88 against 66 us).
 // The four lanes of a quad (lanes 4k..4k+3 of a warp) hold one extended point, one coordinate
 // each: lane 0 X, lane 1 T, lane 2 Y, lane 3 Z.  Each lane computes one of the four independent
 // products of a step and the lanes exchange what the next step needs, so a doubling costs two
@@ -904,22 +906,25 @@ __device__ __forceinline__ fq_t fq_addsub(const fq_t &base, const fq_t &term, ui
   r.v[FQ_LIMBS - 1] = addc(r.v[FQ_LIMBS - 1], q2[FQ_LIMBS - 1] & neg);
   return r;
 }
-// dbl-2008-hwcd, a = -1: A = X^2, B = Y^2, C = 2 Z^2, S = (X + Y)^2, E = S - A - B, G = B - A,
+// the value of lane k of the quad, on all four
+__device__ __forceinline__ fq_t dq_bcast(const fq_t &a, int k, uint32_t mask) {
+  fq_t r;
+#pragma unroll
+  for (int j = 0; j < FQ_LIMBS; j++) r.v[j] = __shfl_sync(mask, a.v[j], k, 4);
+  return r;
+}
+
+// dbl-2008-hwcd, a = -1, with 2 X Y as a product: A = X^2, B = Y^2, C = 2 Z^2, E = 2 X Y, G = B - A,
 // F = G - C, H = -A - B; X3 = E F, Y3 = G H, T3 = E H, Z3 = F G.  (F and H change sign together
 // here, F' = A + C - B and H' = A + B, which changes the signs of all four coordinates.)
-// Every square is below 1.5q, so E < 5.5q, G < 3.5q, F' < 8q, H' < 3q.
+// Products are below 1.5q, so E < 3q, G < 3.5q, F' < 6.5q, H' < 3q.
 static __device__ __noinline__ fq_t dq_dbl(fq_t p, uint32_t mask) {
   const int l = dq_lane();
   const fq_t o1 = dq_xchg(p, 1, mask), o3 = dq_xchg(p, 3, mask);  // lane 1 gets X and Y
-  const fq_t sq = fq_sqr(l == 1 ? fq_add_lazy(o1, o3) : p);         // A, S, B, Z^2 on lanes 0..3
-  const fq_t s1 = dq_xchg(sq, 1, mask), s2 = dq_xchg(sq, 2, mask), s3 = dq_xchg(sq, 3, mask);
-  // the square of lane j sits in sq, s1, s2 or s3 as j ^ l is 0, 1, 2 or 3
-  const fq_t A = pick4(l, sq, s1, s2, s3), S = pick4(l, s1, sq, s3, s2);
-  const fq_t B = pick4(l, s2, s3, sq, s1), ZZ = pick4(l, s3, s2, s1, sq);
-  const fq_t H = fq_add_lazy(A, B);
-  const fq_t E = fq_sub_lazy4(S, H);
-  const fq_t G = fq_sub_lazy(B, A);
-  const fq_t F = fq_sub_lazy(fq_add_lazy(A, fq_shl_lazy(ZZ, 1)), B);
+  const fq_t pr = fq_mul(fq_select(l == 1, o1, p), fq_select(l == 1, o3, p));        // A, X Y, B, Z^2 on lanes 0..3
+  const fq_t A = dq_bcast(pr, 0, mask), E = fq_shl_lazy(dq_bcast(pr, 1, mask), 1);
+  const fq_t B = dq_bcast(pr, 2, mask), C = fq_shl_lazy(dq_bcast(pr, 3, mask), 1);
+  const fq_t H = fq_add_lazy(A, B), G = fq_sub_lazy(B, A), F = fq_sub_lazy(fq_add_lazy(A, C), B);
   return fq_mul(pick4(l, E, E, G, F), pick4(l, F, H, H, G));
 }
 
@@ -986,10 +991,10 @@ static __device__ __noinline__ fq_t dq_add(fq_t p, fq_t q, uint32_t mask) {
   const fq_t pr = fq_shl_lazy(fq_mul(m1, m2), l & 1);  // A, C, B, D on lanes 0..3, below 3q
   // pairs {0, 2}: F = B - A, G = B + A; pairs {1, 3}: H = D - C, E = D + C
   const fq_t o = dq_xchg(pr, 2, mask);
-  const fq_t u = fq_sub_lazy4(l < 2 ? o : pr, l < 2 ? pr : o), w = fq_add_lazy(o, pr);  // below 7q, 6q
+  const fq_t u = fq_sub_lazy4(fq_select(l < 2, o, pr), fq_select(l < 2, pr, o)), w = fq_add_lazy(o, pr);  // below 7q, 6q
   // lane 0 lacks E, lane 2 lacks H, lane 3 lacks F and G
-  const fq_t r1 = dq_xchg(l == 1 ? w : u, 1, mask), r2 = dq_xchg(w, 1, mask);
-  const fq_t r = fq_mul(l == 0 || l == 3 ? r1 : w, l < 2 ? u : l == 2 ? r1 : r2);
+  const fq_t r1 = dq_xchg(fq_select(l == 1, w, u), 1, mask), r2 = dq_xchg(w, 1, mask);
+  const fq_t r = fq_mul(fq_select(l == 0 || l == 3, r1, w), fq_select(l < 2, u, fq_select(l == 2, r1, r2)));
   if (__any_sync(mask, l == 3 && r.v[0] <= 1u)) return dq_add_rare(p, q, r, mask);
   return r;
 }
@@ -1022,16 +1027,16 @@ static __device__ __noinline__ fq_t dq_madd(fq_t p, fq_t b, bool neg, uint32_t m
   const int l = dq_lane();
   const uint32_t even = (l & 1) ? 0u : ~0u;
   const fq_t po = dq_xchg(p, 2, mask);
-  const fq_t m1 = fq_addsub((l & 1) ? p : po, p, even, l == 0 ? ~0u : 0u);
+  const fq_t m1 = fq_addsub(fq_select(l & 1, p, po), p, even, l == 0 ? ~0u : 0u);
   const fq_t pr = fq_mul(m1, b);  // A, C, B, D on lanes 0..3, below 1.5q
   const fq_t o = dq_xchg(pr, 2, mask);
-  const fq_t d = fq_sub_lazy(l < 2 ? o : pr, l < 2 ? pr : o), a = fq_add_lazy(o, pr);
+  const fq_t d = fq_sub_lazy(fq_select(l < 2, o, pr), fq_select(l < 2, pr, o)), a = fq_add_lazy(o, pr);
   // E, H on lanes 0, 2; F, G on 1, 3, where a negative digit negates C
   const bool swap = neg && (l & 1);
-  const fq_t u = swap ? a : d, w = swap ? d : a;
+  const fq_t u = fq_select(swap, a, d), w = fq_select(swap, d, a);
   // lane 0 lacks F, lane 2 lacks G, lane 1 lacks E and H
-  const fq_t r1 = dq_xchg(l == 3 ? w : u, 1, mask), r2 = dq_xchg(w, 1, mask);
-  return fq_mul(l == 1 ? r1 : l == 2 ? w : u, l == 1 ? r2 : l == 3 ? w : r1);
+  const fq_t r1 = dq_xchg(fq_select(l == 3, w, u), 1, mask), r2 = dq_xchg(w, 1, mask);
+  return fq_mul(fq_select(l == 1, r1, fq_select(l == 2, w, u)), fq_select(l == 1, r2, fq_select(l == 3, w, r1)));
 }
 
 // the point of base v itself: X = ypx - ymx (negated for a negative digit), Y = ypx + ymx, Z = 1, T = X Y
