@@ -122,7 +122,7 @@ GL_FN void gl_copy16(uint64_t *dst, const uint64_t *src) {
 //
 // What bounds it (ncu and timings on GB300, 2^24 points): the arithmetic and the memory passes
 // together.  Without arithmetic the three passes take 46 + 40 + 41 us (268 MB each, 87 to 100% of
-// the measured copy bandwidth); with it 75 + 83 + 65 us: about 110 instructions per point and pass,
+// the measured copy bandwidth); with it 74 + 81 + 64 us: about 120 instructions per point and pass,
 // of which the 32 x 32 wide multiplies hold the issue port for four cycles each.  The previous
 // kernel (radix 8 with table roots, two passes of 2^12 points, one 147 KB block per SM) took
 // 339 + 272 us: 5 general products per point and pass, and load, arithmetic and store phases that
@@ -200,10 +200,8 @@ GL_FN void pass_round1(const NttPass &ps, uint64_t *sm, uint32_t block, uint32_t
     gl3 x[T];
 #pragma unroll
     for (int t = 0; t < T; t++) x[t] = gl3_from(gl_ldcs(at_of(ps.src, t * step, at)));
-    if (L1 > 0) {
-      x[0] = gl3_biased(x[0]);
-      gl_dft<L1>(x);
-    }
+    x[0] = gl3_biased(x[0]);
+    if (L1 > 0) gl_dft<L1>(x);
     if (L2 == 0) {
       pass_store<T, LC, TWIST>(ps, nullptr, gl, gh, 0, 1, 0, x);
     } else {
@@ -329,7 +327,7 @@ __global__ void k_gl_test(int op, const uint64_t *a, const uint64_t *b, uint64_t
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const gl3 x = gl3_from(a[i]), y = gl3_from(b[i]);
-  out[i] = gl_canon(op == 0   ? gl3_fold(gl3_add(x, y))
+  out[i] = gl_canon(op == 0   ? gl3_fold(gl3_biased(gl3_add(x, y)))
                     : op == 1 ? gl3_fold(gl3_biased(gl3_sub(x, y)))
                               : gl_mul(gl_mul(a[i], gl_canon(b[i])), kMontSq));
 }
