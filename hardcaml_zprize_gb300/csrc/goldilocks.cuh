@@ -133,6 +133,7 @@ GL_FN uint64_t gl3_fold(const gl3 &a) {
       "sub.cc.u32 %0, %0, %2;\n\tsubc.u32 %1, %1, 0;\n\tadd.u32 %1, %1, %2;"
       : "=&r"(r0), "=&r"(r1), "=&r"(c)
       : "r"(a.lo), "r"(a.hi), "r"(0u - (uint32_t)a.e), "r"((uint32_t)a.e - 1u));
+  (void)c;
   return gl_pack(r0, r1);
 #else
   const unsigned __int128 s =

@@ -10,7 +10,8 @@
 //   pass 3: over jc for every (ka, kb), to X[ka + a kb + a b kc].
 // One kernel template (k_ntt_pass) does every pass: a block holds eight of the short transforms
 // (64 contiguous bytes of every row it reads or writes) and runs each as two rounds of at most 16
-// points in registers, whose roots are powers of two (goldilocks.cuh).
+// points in registers, whose roots are powers of two (goldilocks.cuh).  Two passes run as one thread
+// block cluster that hands the rows over through its blocks' shared memory (k_ntt_cluster).
 // An inverse context (ntt_init_inverse) runs the same forward kernels, stores output k at place
 // (n - k) mod n and multiplies by 1/n: the factor sits in a twist table, or in the store of a
 // transform of one pass.
@@ -32,8 +33,8 @@ namespace {
 
 constexpr uint32_t NTT_MAX_LOG_N = 24;
 constexpr uint32_t NTT_ONE_PASS = 8;   // largest log2 of a transform of one pass
-// Two passes up to here, three above: three short ones spread over more blocks.  Measured on GB300
-// (us, two passes / three): 2^12 5.4 / 5.4, 2^13 6.8 / 5.4, 2^14 8.1 / 5.5, 2^16 10.0 / 7.0.
+// Two passes (one launch) up to here, three above: a cluster has at most eight blocks.  Measured on
+// GB300 (us, two passes as two launches / three launches): 2^12 5.4 / 5.4, 2^13 6.8 / 5.4, 2^16 10.0 / 7.0.
 constexpr uint32_t NTT_TWO_PASS = 12;
 // log2 transforms per block of a split transform.  Eight: 64 contiguous bytes of every row.
 // Measured with four / eight / sixteen (us): the passes of 2^24 points without their arithmetic
@@ -72,7 +73,7 @@ struct NttPass {
   uint32_t in_c, in_h, in_i;
   uint32_t out_c, out_h, out_k;
   const uint64_t *tw1;  // the round boundary's factors w_m^(k0 u), tw1[k0 U + u]
-  // twist tables (see TW_TABLE, TW_SHARED, TW_STEPS)
+  // twist tables (see TW_SHARED, TW_STEPS; k_ntt_cluster: tw the twist, tw_a the second pass's tw1)
   const uint64_t *tw, *tw_a;
   uint32_t t_k, t_g, t_shift;
   uint32_t o_mask;   // n - 1
@@ -146,7 +147,6 @@ GL_FN const uint64_t *at_of(const uint64_t *base, uint32_t uniform, uint32_t lan
 // How a pass twists its outputs (the factor between it and the next pass).
 enum : int {
   TW_NONE = 0,
-  TW_TABLE,   // tw[k t_k + gl t_g], read from global memory
   TW_SHARED,  // tw[k + (gl >> t_shift) t_g], the same for the block's transforms: staged in shared memory
   TW_STEPS,   // base (tw_a[g] tw[v t_k + gl]) times tw[(k - v) t_k + gl], the latter staged: 2^L2 a transform
 };
@@ -174,8 +174,7 @@ GL_FN void pass_store(const NttPass &ps, const uint64_t *tws, uint32_t gl, uint3
 #pragma unroll
   for (int t = 0; t < T; t++) {
     uint64_t y = gl3_fold(x[t]);
-    if (TWIST == TW_TABLE) y = gl_mul(y, *at_of(ps.tw, t * vstep * ps.t_k, v * ps.t_k + gl * ps.t_g));
-    else if (TWIST == TW_SHARED) y = gl_mul(y, tws[v + t * vstep]);
+    if (TWIST == TW_SHARED) y = gl_mul(y, tws[v + t * vstep]);
     else if (TWIST == TW_STEPS) y = gl_mul(y, t ? gl_mul(base, tws[(t << LC) + (gl & ((1 << LC) - 1))]) : base);
     else if (ps.scale) y = gl_mul(y, ps.scale);
     else y = gl_canon(y);
@@ -189,8 +188,10 @@ GL_FN void pass_store(const NttPass &ps, const uint64_t *tws, uint32_t gl, uint3
   }
 }
 
+// rows (not null): the block's transforms are in shared memory, transform c from rows[c (m + 1)]
 template <int L1, int L2, int LC, bool ROWS, int TWIST>
-GL_FN void pass_round1(const NttPass &ps, uint64_t *sm, uint32_t block, uint32_t tid, uint32_t threads) {
+GL_FN void pass_round1(const NttPass &ps, uint64_t *sm, uint32_t block, uint32_t tid, uint32_t threads,
+                       const uint64_t *rows = nullptr) {
   using S = PassShape<L1, L2, LC>;
   constexpr int T = 1 << L1;
   for (uint32_t w = tid; w < ((uint32_t)S::U << LC); w += threads) {
@@ -199,7 +200,8 @@ GL_FN void pass_round1(const NttPass &ps, uint64_t *sm, uint32_t block, uint32_t
     const uint32_t at = gl * ps.in_c + gh * ps.in_h + u * ps.in_i, step = S::U * ps.in_i;
     gl3 x[T];
 #pragma unroll
-    for (int t = 0; t < T; t++) x[t] = gl3_from(gl_ldcs(at_of(ps.src, t * step, at)));
+    for (int t = 0; t < T; t++)
+      x[t] = gl3_from(rows ? rows[c * ((1u << S::LM) + 1) + u + t * S::U] : gl_ldcs(at_of(ps.src, t * step, at)));
     x[0] = gl3_biased(x[0]);
     if (L1 > 0) gl_dft<L1>(x);
     if (L2 == 0) {
@@ -261,17 +263,93 @@ struct Rounds { int l1, l2; };
 constexpr Rounds kRounds[NTT_ONE_PASS + 1] = {{0, 0}, {1, 0}, {2, 0}, {3, 0}, {2, 2},
                                               {3, 2}, {3, 3}, {4, 3}, {4, 4}};
 
+// ---- two passes as one cluster ----
+// n = a b with a = 2^LA, b = 2^LB points: block r of a / 8 takes the columns 8 r .. 8 r + 7 through
+// pass 1 (the first b / 8 blocks do) and writes output ka of column jb, twisted, into the shared memory of
+// the block that owns row ka (ka / 8); after a cluster barrier every block takes its eight rows through
+// pass 2.  One launch and no trip through L2 between the passes: 2^12 points 3.8 us against 5.5 as two
+// dependent launches and 14.3 as one block of 1024 threads.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <int LA, int LB>
+struct ClusterShape {
+  using A = PassShape<kRounds[LA].l1, kRounds[LA].l2, 3>;
+  using B = PassShape<kRounds[LB].l1, kRounds[LB].l2, 3>;
+  static constexpr int BLOCKS = 1 << (LA - 3);
+  static constexpr int THREADS = A::THREADS > B::THREADS ? A::THREADS : B::THREADS;
+  static constexpr int MID_A = A::PITCH << kRounds[LA].l1, MID_B = B::PITCH << kRounds[LB].l1;
+  static constexpr int MID = MID_A > MID_B ? MID_A : MID_B;
+  static constexpr int PITCH = (1 << LB) + 1;
+  static constexpr size_t SMEM = 8 * (size_t)(MID + 8 * PITCH);
+};
+
+template <int LA, int LB>
+__global__ void __launch_bounds__(ClusterShape<LA, LB>::THREADS) k_ntt_cluster(const NttPass ps) {
+  using C = ClusterShape<LA, LB>;
+  constexpr Rounds ra = kRounds[LA], rb = kRounds[LB];
+  extern __shared__ __align__(16) uint64_t sm[];
+  uint64_t *rows = sm + C::MID;
+  uint32_t rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  cluster_arrive();  // answered below, before the first access to another block's memory
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const bool columns = rank < (1u << (LB - 3));
+  if (columns)
+    pass_round1<ra.l1, ra.l2, 3, false, TW_NONE>(ps, sm, rank, threadIdx.x, blockDim.x);
+  __syncthreads();
+  cluster_wait();
+  if (columns) {
+    constexpr int T = 1 << ra.l2;
+    for (uint32_t w = threadIdx.x; w < (1u << (ra.l1 + 3)); w += blockDim.x) {
+      const uint32_t c = w & 7, k0 = w >> 3, jb = rank * 8 + c;
+      uint64_t f[T];
+      gl3 x[T];
+#pragma unroll
+      for (int t = 0; t < T; t++) f[t] = ps.tw[(jb << LA) + k0 + (t << ra.l1)];
+#pragma unroll
+      for (int t = 0; t < T; t++) x[t] = gl3_from(sm[k0 * C::A::PITCH + c + t * 8]);
+      x[0] = gl3_biased(x[0]);
+      gl_dft<ra.l2>(x);
+#pragma unroll
+      for (int t = 0; t < T; t++) {
+        const uint32_t ka = k0 + (t << ra.l1);
+        const uint64_t y = gl_mul(gl3_fold(x[t]), f[t]);
+        uint32_t at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(at)
+            : "r"((uint32_t)__cvta_generic_to_shared(rows + (ka & 7) * C::PITCH + jb)), "r"(ka >> 3));
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(at), "l"(y) : "memory");
+      }
+    }
+  }
+  cluster_arrive();
+  cluster_wait();
+  NttPass pb = ps;
+  pb.tw1 = ps.tw_a;
+  pass_round1<rb.l1, rb.l2, 3, true, TW_NONE>(pb, sm, rank, threadIdx.x, blockDim.x, rows);
+  __syncthreads();
+  pass_round2<rb.l1, rb.l2, 3, true, TW_NONE>(pb, sm, rank, threadIdx.x, blockDim.x);
+}
+
 struct PassKernel {
   void (*fn)(const NttPass);
   uint32_t threads;
   size_t smem;
+  uint32_t cluster;  // blocks of a cluster (0: none)
 };
 template <int LM, int LC, bool ROWS, int TWIST>
 PassKernel pass_kernel() {
   using S = PassShape<kRounds[LM].l1, kRounds[LM].l2, LC>;
-  return {k_ntt_pass<kRounds[LM].l1, kRounds[LM].l2, LC, ROWS, TWIST>, (uint32_t)S::THREADS, S::SMEM};
+  return {k_ntt_pass<kRounds[LM].l1, kRounds[LM].l2, LC, ROWS, TWIST>, (uint32_t)S::THREADS, S::SMEM, 0};
 }
-// the whole transform as one block
+template <int LA, int LB>
+PassKernel cluster_kernel() {
+  using C = ClusterShape<LA, LB>;
+  return {k_ntt_cluster<LA, LB>, (uint32_t)C::THREADS, C::SMEM, (uint32_t)C::BLOCKS};
+}
+// the whole transform as one block, or one cluster
 PassKernel whole_kernel(uint32_t log_m) {
   switch (log_m) {
     case 0: return pass_kernel<0, 0, true, TW_NONE>();
@@ -282,22 +360,22 @@ PassKernel whole_kernel(uint32_t log_m) {
     case 5: return pass_kernel<5, 0, true, TW_NONE>();
     case 6: return pass_kernel<6, 0, true, TW_NONE>();
     case 7: return pass_kernel<7, 0, true, TW_NONE>();
-    default: return pass_kernel<8, 0, true, TW_NONE>();
+    case 8: return pass_kernel<8, 0, true, TW_NONE>();
+    case 9: return cluster_kernel<5, 4>();
+    case 10: return cluster_kernel<5, 5>();
+    case 11: return cluster_kernel<6, 5>();
+    default: return cluster_kernel<6, 6>();
   }
 }
 // a pass of a split transform (2^4 to 2^8 points, at least 2^4 transforms)
 template <bool ROWS, int TWIST>
 PassKernel split_kernel(uint32_t log_m) {
-  if constexpr (TWIST == TW_TABLE) {  // the first of two passes: 2^5 or 2^6 points
-    return log_m == 5 ? pass_kernel<5, NTT_LOG_COLS, ROWS, TWIST>() : pass_kernel<6, NTT_LOG_COLS, ROWS, TWIST>();
-  } else {
-    switch (log_m) {
-      case 4: return pass_kernel<4, NTT_LOG_COLS, ROWS, TWIST>();
-      case 5: return pass_kernel<5, NTT_LOG_COLS, ROWS, TWIST>();
-      case 6: return pass_kernel<6, NTT_LOG_COLS, ROWS, TWIST>();
-      case 7: return pass_kernel<7, NTT_LOG_COLS, ROWS, TWIST>();
-      default: return pass_kernel<8, NTT_LOG_COLS, ROWS, TWIST>();
-    }
+  switch (log_m) {
+    case 4: return pass_kernel<4, NTT_LOG_COLS, ROWS, TWIST>();
+    case 5: return pass_kernel<5, NTT_LOG_COLS, ROWS, TWIST>();
+    case 6: return pass_kernel<6, NTT_LOG_COLS, ROWS, TWIST>();
+    case 7: return pass_kernel<7, NTT_LOG_COLS, ROWS, TWIST>();
+    default: return pass_kernel<8, NTT_LOG_COLS, ROWS, TWIST>();
   }
 }
 
@@ -402,8 +480,9 @@ int plan_passes(NttCtx *cx) {
   const uint32_t ln = cx->log_n;
   // digits of the split, most significant first
   uint32_t d[3] = {ln, 0, 0};
-  cx->n_pass = ln <= NTT_ONE_PASS ? 1 : ln <= NTT_TWO_PASS ? 2 : 3;
-  if (cx->n_pass == 2) {
+  const bool fused = ln > NTT_ONE_PASS && ln <= NTT_TWO_PASS;  // two passes in one launch
+  cx->n_pass = ln <= NTT_TWO_PASS ? 1 : 3;
+  if (fused) {
     d[1] = ln / 2;
     d[0] = ln - d[1];
   } else if (cx->n_pass == 3) {
@@ -419,9 +498,9 @@ int plan_passes(NttCtx *cx) {
   };
   // round factors of each pass, then the twists
   std::vector<Table> tabs;
-  for (int p = 0; p < cx->n_pass; p++)
+  for (int p = 0; p < cx->n_pass + (fused ? 1 : 0); p++)
     tabs.push_back({(uint32_t)kRounds[d[p]].l1, (uint32_t)kRounds[d[p]].l2, d[p], 1});
-  if (cx->n_pass == 2) {
+  if (fused) {
     tabs.push_back({lb, la, ln, inv_n});  // w^(jb ka)
   } else if (cx->n_pass == 3) {
     tabs.push_back({lb, la, la + lb, 1});  // w_ab^(jb ka)
@@ -460,13 +539,20 @@ int plan_passes(NttCtx *cx) {
     if (cx->n_pass == 1) {
       cx->pass[p].k = whole_kernel(ln);
       ps.in_i = ps.out_k = 1;
-      ps.scale = cx->inverse ? h_mont(inv_n) : 0;
+      ps.scale = cx->inverse && !fused ? h_mont(inv_n) : 0;  // in the twist table of two passes
+      if (fused) {
+        cx->pass[p].blocks = cx->pass[p].k.cluster;
+        ps.in_c = ps.out_c = 1;
+        ps.in_i = b;
+        ps.out_k = a;
+        ps.tw_a = cx->d_tab + off[1];
+        ps.tw = cx->d_tab + off[2];
+      }
     } else if (p == 0) {
-      cx->pass[p].k = cx->n_pass == 2 ? split_kernel<false, TW_TABLE>(la) : split_kernel<false, TW_SHARED>(la);
+      cx->pass[p].k = split_kernel<false, TW_SHARED>(la);
       ps.in_c = ps.out_c = 1;
       ps.in_i = ps.out_k = b * c;
       ps.tw = cx->d_tab + off[cx->n_pass];
-      ps.t_k = 1;
       ps.t_g = a;
       ps.t_shift = lc;
     } else if (!last) {
@@ -490,7 +576,6 @@ int plan_passes(NttCtx *cx) {
       ps.out_c = 1;
       ps.out_h = a;
       ps.out_k = a * b;
-      if (cx->n_pass == 2) ps.in_c = b, ps.in_h = 0, ps.out_h = 0, ps.out_k = a;
     }
     NCK(cudaFuncSetAttribute(cx->pass[p].k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)cx->pass[p].k.smem));
@@ -508,16 +593,19 @@ int enqueue_ntt(NttCtx *cx, uint64_t *d_dst, const uint64_t *d_src, cudaStream_t
     NttPass ps = cx->pass[p].ps;
     ps.src = p == 0 ? d_src : cx->d_tmp;
     ps.dst = p + 1 == cx->n_pass ? d_dst : cx->d_tmp;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cx->pass[p].k.cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cx->pass[p].blocks);
     cfg.blockDim = dim3(cx->pass[p].k.threads);
     cfg.dynamicSmemBytes = cx->pass[p].k.smem;
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cx->pass[p].k.cluster ? 2 : 1;
     NCK(cudaLaunchKernelEx(&cfg, cx->pass[p].k.fn, (const NttPass)ps));
     if (marks && p == 0) NCK(cudaEventRecord(cx->ev[2], st));
   }
@@ -569,7 +657,7 @@ void *ntt_create(uint32_t log_n, bool inverse) {
   for (auto &e : cx->ev) step(cudaEventCreate(&e), "event");
   step(cudaMalloc(&cx->d_in, cx->n * 8), "input buffer");
   step(cudaMalloc(&cx->d_out, cx->n * 8), "output buffer");
-  if (log_n > NTT_ONE_PASS) step(cudaMalloc(&cx->d_tmp, cx->n * 8), "intermediate buffer");
+  if (log_n > NTT_TWO_PASS) step(cudaMalloc(&cx->d_tmp, cx->n * 8), "intermediate buffer");
   if (!rc) rc = plan_passes(cx);
   if (rc) {
     delete cx;
@@ -596,7 +684,7 @@ int ntt_evaluate_device(void *context, uint64_t *d_out, const uint64_t *d_in, vo
   g_err = 0;
   auto *cx = (NttCtx *)context;
   if (!cx || !d_out || !d_in) return fail(NTT_ERR_ARG, "ntt_evaluate_device: null argument");
-  if (d_out == d_in && cx->log_n <= 12)
+  if (d_out == d_in && cx->log_n <= NTT_TWO_PASS)
     return fail(NTT_ERR_ARG, "ntt_evaluate_device: the transform is out of place");
   NCK(cudaSetDevice(cx->device));
   return enqueue_ntt(cx, d_out, d_in, stream ? (cudaStream_t)stream : cx->st, false);
