@@ -70,7 +70,10 @@ enum : int {
 };
 
 #define MSM_POINTS_PER_CHUNK 256  // points per histogram block (one chunk of the stage)
-#define MSM_MAX_BINS 32           // key ranges of the staged sort
+#define MSM_MAX_BINS 32           // key ranges of the ranked sort
+#define MSM_MAX_PART_BINS 4096    // key ranges of the partitioned sort
+#define MSM_MAX_PART_SHIFT 14     // log2 of a key range's buckets there, at most
+#define MSM_PLACE_CHUNKS 2048     // chunks of a part of a key range, at most
 
 // Everything a pass needs on the device; sized by the host (msm_plan_pass).
 struct PassBuffers {
@@ -103,22 +106,33 @@ struct PassBuffers {
   uint64_t max_entries;         // capacity of vals
   uint32_t max_tasks;           // capacity of tasks / partials
 
-  // staged sort (or stage == null: the scatter re-reads the scalars once per key range).
+  // Ranked sort (stage set; noalloc passes have neither and re-read the scalars once per key range).
   // k_count writes the entries of its 256 points, (key, base index | sign << 31), into the
   // block's chunk of `stage`, grouped by key range (key >> bin_shift); blk_off holds each
   // chunk's n_bins + 1 range starts.  The scatter then reads one key range per launch and
-  // places each entry at offset + rank (stage_rank set) or at a slot-cursor atomic (null).
+  // places each entry at offset + rank.
   uint2 *stage;                 // [n_chunks * stage_cap]
-  uint32_t *stage_rank;         // or null: [n_chunks * stage_cap] each staged entry's rank in its
-                                // bucket, taken from the bucket count when the entry is staged
+  uint32_t *stage_rank;         // [n_chunks * stage_cap] each staged entry's rank in its bucket,
+                                // taken from the bucket count when the entry is staged
   uint32_t *blk_off;            // [n_chunks * (n_bins + 1)]
-  uint32_t stage_cap;           // entries per chunk: 256 x the pass's most entries per point
+  uint32_t stage_cap;           // entries per chunk: its points x the pass's most entries per point
   uint32_t bin_shift;           // key range of a bucket key
-  uint32_t n_bins;              // key ranges (<= MSM_MAX_BINS)
+  uint32_t n_bins;              // key ranges (<= MSM_MAX_BINS; <= MSM_MAX_PART_BINS when partitioned)
+
+  // Partitioned sort of large passes (bin_total set): chunks of chunk_points points, their entries by
+  // key range in stage_val and stage_key (the key within the range), blk_off indexed [range][chunk].
+  uint32_t *bin_total;          // or null: [n_bins] entries per key range
+  uint32_t *stage_val;          // [n_chunks * stage_cap]
+  uint16_t *stage_key;          // [n_chunks * stage_cap]
+  uint32_t *part_first;         // [place_blocks << bin_shift] bucket counts of a key range's parts
+  uint32_t chunk_points;
+  uint32_t n_chunks;
+  uint32_t place_part;          // entries from which a key range is split into parts
+  uint32_t place_blocks;        // room for all parts
 
   uint32_t *count;              // [n_buckets]
   uint32_t *offset;             // [n_buckets]
-  uint32_t *fill;               // [n_buckets] slot cursors (the scan seeds them with offset)
+  uint32_t *fill;               // or null: [n_buckets] slot cursors (the scan seeds them with offset)
   uint32_t *taskoff;            // [n_buckets]
   uint32_t *scan_tmp;           // block partials for the scans
   uint32_t *vals;               // [max_entries]
@@ -145,8 +159,9 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t str
 #define MSM_NUM_STAGES 10
 size_t msm_scan_tmp_words(uint32_t n_buckets);
 uint32_t msm_scatter_passes(uint64_t max_entries);
-uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool cursors, bool many);
-uint64_t msm_upload_chunk_points(uint64_t n_points, int nchunks);
+uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool many);
+size_t msm_partition_smem(uint32_t n_bins, uint32_t stage_cap);
+uint64_t msm_upload_chunk_points(uint64_t n_points, int nchunks, uint32_t chunk_points);
 
 // resident-base preparation
 cudaError_t msm_launch_precompute(const void *d_affine, size_t n, uint4 *d_bases, uint8_t *d_flags,

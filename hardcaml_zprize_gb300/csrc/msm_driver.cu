@@ -297,11 +297,13 @@ struct Plan {
   uint64_t n_points = 0, max_entries = 0;
   uint32_t n_buckets = 0, n_segs = 0, n_grps = 0, max_tasks = 0;
   uint32_t seg_len = 1024, red_log2 = 5, grp_log2 = 9;
-  // staged sort: histogram chunks of MSM_POINTS_PER_CHUNK points, each with room for the
-  // largest window count of the pass, and the key ranges of the scatter
+  // sort: chunks of chunk_points points, each with room for the largest window count of the pass, and
+  // the key ranges
   uint64_t n_chunks = 0;
   uint32_t stage_cap = 0, bin_shift = 0, n_bins = 0;
-  bool ranks = false;  // entries carry their rank in the bucket (no slot atomics in the scatter)
+  uint32_t chunk_points = MSM_POINTS_PER_CHUNK;
+  bool place = false;  // the partitioned sort
+  uint32_t place_blocks = 0;
   std::string key;
 };
 
@@ -330,7 +332,42 @@ uint32_t pass_seg_len(const std::vector<JobSpec> &specs) {
   return std::min(seg, cap);
 }
 
-int build_plan(const std::vector<JobSpec> &specs, Plan &pl) {
+// Entries from which a key range is split over several blocks: short parts keep the slices that are
+// being written small and even out the load, long ones share their set-up (2^24 points, count + scatter,
+// 16384 / 32768 / 65536: 2.46 / 2.62 / 2.80 ms; 2^20 points, 8192 / 16384: 0.208 / 0.190).
+constexpr uint32_t kPlacePart = 16384;
+
+// The partitioned sort is for passes of at least this many entries (MSM_SORT_PARTITION=1 / 0: always /
+// never, for tests and tuning).  Measured on GB300 (us per MSM, scalars in HBM, ranked / partitioned):
+// 66000 points (1.06e6 entries) 588 / 589, 100000 738 / 732, 140000 904 / 890, 350000 1748 / 1692,
+// 800000 3494 / 3403; without tables 80000 (1.6e6) 1243 / 1217, 350000 2390 / 2345.
+// A pass that reads its scalars from host memory while it counts hides the ranked sort's atomics behind
+// the C2C link, and k_place_count comes on top: for those the line lies higher (ms per call, ranked /
+// partitioned: 4 x 100000 1.96 / 1.99, 4 x 200000 3.44 / 3.48, 4 x 2^20 in one pass 14.22 / 14.26, one
+// MSM of 3e6 9.80 / 9.77).
+constexpr uint64_t kPartitionEntries = 1ull << 20;
+constexpr uint64_t kPartitionEntriesHost = 1ull << 25, kPartitionEntriesHostMany = 1ull << 27;
+
+bool partitioned(const Plan &pl, uint32_t max_epp, bool host_read) {
+  if (!pl.n_buckets || pl.n_buckets > (uint64_t)MSM_MAX_PART_BINS << MSM_MAX_PART_SHIFT) return false;
+  if ((pl.n_points + 2048) * max_epp >= 1ull << 32) return false;  // stage indices are 32 bits
+  if (const char *e = getenv("MSM_SORT_PARTITION")) return atoi(e) != 0;
+  return pl.max_entries >= (!host_read ? kPartitionEntries
+                            : pl.jobs.size() > 1 ? kPartitionEntriesHostMany : kPartitionEntriesHost);
+}
+
+// Points of a chunk: 2048, or 1024 in a pass of fewer than 2^21 points (at least 2^9 chunks to spread
+// over the SMs), as far as their entries fit a block's shared memory.  Measured on GB300 (count, ms,
+// 1024 / 2048): 2^24 points 1.45 / 1.09.
+uint32_t chunk_points_for(const Plan &pl, uint32_t max_epp) {
+  const uint32_t bins = ((pl.n_buckets - 1) >> pl.bin_shift) + 1;
+  uint32_t k = pl.n_points >= (1u << 21) ? 2048 : 1024;
+  while (k > 256 && msm_partition_smem(bins, k * max_epp) > (224u << 10)) k -= 256;
+  return k;
+}
+
+// `host_read`: the histogram will read the scalars from host memory
+int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = false) {
   pl = Plan();
   if (specs.empty()) return fail(ERR_ARG, "empty pass");
   pl.seg_len = specs[0].cfg.seg_len;
@@ -420,21 +457,28 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl) {
   uint32_t max_epp = 0;  // entries per point
   for (const JobDesc &d : pl.jobs)
     if (d.nwin) max_epp = std::max(max_epp, entries_per_point(d.c, d.signed_digits));
-  pl.n_chunks = (pl.n_points + MSM_POINTS_PER_CHUNK - 1) / MSM_POINTS_PER_CHUNK;
-  pl.stage_cap = MSM_POINTS_PER_CHUNK * max_epp;
-  // MSM_SORT_RANGES=<n> overrides the number of key ranges of the staged sort (tests, tuning)
+  // MSM_SORT_RANGES=<n> asks for the ranked sort with n key ranges (tests, tuning)
   const char *sr = getenv("MSM_SORT_RANGES");
-  // ranks from the histogram's atomics save the scatter's slot atomics, but the histogram's
-  // atomics then return a value.  Measured on GB300 (count + scatter): the uneven 64-MSM mix
-  // (up to 1.0e8 entries, 2^21 buckets) 2.03 ms with ranks, 2.67 ms without; 2^24 points on
-  // tables of width 23 (2.0e8 entries, 4.9M buckets) 5.65 against 4.86 with ranges of 2^20 keys,
-  // and the cursors 3.45 with ranges of 2^19 keys; 2^26 points (8.1e8) 16.5 against 14.0
-  pl.ranks = pl.max_entries < (1ull << 27);
-  pl.bin_shift =
-      msm_bin_shift(pl.n_buckets, pl.max_entries, sr ? (uint32_t)atoi(sr) : 0u, !pl.ranks, specs.size() > 1);
+  pl.bin_shift = msm_bin_shift(pl.n_buckets, pl.max_entries, sr ? (uint32_t)atoi(sr) : 0u, specs.size() > 1);
+  pl.place = !sr && partitioned(pl, max_epp, host_read);
+  if (pl.place) {
+    // ranges of 2^11 buckets, 2^12 from 2^22 buckets on.  Measured on GB300 (count + scatter, ms, 2^10 /
+    // 2^11 / 2^12 / 2^13 buckets): 2^20 points 0.215 / 0.190 / 0.208 / -, 2^21 without tables 0.406 /
+    // 0.392 / 0.419 / -, the uneven mix (4.1e6 buckets) 1.90 / 1.77 / 2.21 / 2.83, 2^24 points (4.9e6)
+    // - / 2.85 / 2.46 / 2.59: wide ranges are written over too much memory at a time, many of them
+    // leave a chunk few entries in each.
+    pl.bin_shift = pl.n_buckets > (1u << 22) ? 12 : 11;
+    while ((pl.n_buckets - 1) >> pl.bin_shift >= MSM_MAX_PART_BINS) pl.bin_shift++;
+    pl.chunk_points = chunk_points_for(pl, max_epp);
+  }
+  pl.n_chunks = (pl.n_points + pl.chunk_points - 1) / pl.chunk_points;
+  pl.stage_cap = pl.chunk_points * max_epp;
   pl.n_bins = pl.n_buckets ? ((pl.n_buckets - 1) >> pl.bin_shift) + 1 : 0;
-  if (pl.n_bins > MSM_MAX_BINS) return fail(ERR_STATE, "too many key ranges: %u", pl.n_bins);
-  snprintf(tmp, sizeof(tmp), "|r%u", pl.bin_shift);
+  if (pl.place)
+    pl.place_blocks = pl.n_bins * (uint32_t)((pl.n_chunks + MSM_PLACE_CHUNKS - 1) / MSM_PLACE_CHUNKS) +
+                      (uint32_t)(pl.max_entries / kPlacePart) + 1;
+  else if (pl.n_bins > MSM_MAX_BINS) return fail(ERR_STATE, "too many key ranges: %u", pl.n_bins);
+  snprintf(tmp, sizeof(tmp), "|r%u/%u", pl.bin_shift, pl.place ? pl.chunk_points : 0u);
   pl.key += tmp;
   pl.n_segs = (uint32_t)segs;
   pl.n_grps = (uint32_t)grps;
@@ -449,9 +493,10 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl) {
 // device bytes a pass needs besides the resident bases
 uint64_t plan_bytes(const Plan &pl, bool with_scalars) {
   uint64_t b = 0;
-  b += (uint64_t)pl.n_buckets * 4 * 5;                   // count, offset, fill, taskoff, heavy
+  b += (uint64_t)pl.n_buckets * 4 * 4;                   // count, offset, taskoff, heavy
   b += pl.max_entries * 4;                                // vals
-  b += pl.n_chunks * ((uint64_t)pl.stage_cap * (pl.ranks ? 12 : 8) + (pl.n_bins + 1) * 4);
+  b += pl.n_chunks * ((uint64_t)pl.stage_cap * (pl.place ? 6 : 12) + (pl.n_bins + 1) * 4);
+  if (pl.place) b += ((uint64_t)pl.place_blocks << (2 + pl.bin_shift)) + pl.n_bins * 4;
   b += (uint64_t)pl.max_tasks * (sizeof(Task) + 4 + MSM_BUCKET_BYTES);
   b += (uint64_t)(pl.n_segs + pl.n_grps) * 2 * MSM_BUCKET_BYTES;
   b += (uint64_t)pl.wins.size() * MSM_BUCKET_BYTES;
@@ -464,8 +509,8 @@ uint64_t plan_bytes(const Plan &pl, bool with_scalars) {
 // workspace: the buffers of one in-flight pass
 // ---------------------------------------------------------------------------------------------
 struct Workspace {
-  DevBuf count, offset, fill, taskoff, scan_tmp, vals, tasks, partials, heavy, counters, seg_out,
-      grp_out, win_sum, results, jobs, wins, order, len_hist, stage, stage_rank, blk_off;
+  DevBuf count, offset, taskoff, scan_tmp, vals, tasks, partials, heavy, counters, seg_out,
+      grp_out, win_sum, results, jobs, wins, order, len_hist, stage, stage_rank, blk_off, bin_total, part_first;
   DevBuf scalars[2];
   HostPinned res_host;
   cudaEvent_t ev[MSM_NUM_STAGES + 1] = {};
@@ -486,14 +531,15 @@ struct Workspace {
     bool moved = false;
     CK(count.ensure((size_t)pl.n_buckets * 4, &moved));
     CK(offset.ensure((size_t)pl.n_buckets * 4, &moved));
-    CK(fill.ensure((size_t)pl.n_buckets * 4, &moved));
     CK(taskoff.ensure((size_t)pl.n_buckets * 4, &moved));
     CK(heavy.ensure((size_t)pl.n_buckets * 4, &moved));
     CK(scan_tmp.ensure(msm_scan_tmp_words(pl.n_buckets) * 4, &moved));
     CK(vals.ensure((size_t)pl.max_entries * 4, &moved));
-    CK(stage.ensure((size_t)pl.n_chunks * pl.stage_cap * 8, &moved));
-    if (pl.ranks) CK(stage_rank.ensure((size_t)pl.n_chunks * pl.stage_cap * 4, &moved));
+    CK(stage.ensure((size_t)pl.n_chunks * pl.stage_cap * (pl.place ? 6 : 8), &moved));
+    if (!pl.place) CK(stage_rank.ensure((size_t)pl.n_chunks * pl.stage_cap * 4, &moved));
     CK(blk_off.ensure((size_t)pl.n_chunks * (pl.n_bins + 1) * 4, &moved));
+    if (pl.place) CK(part_first.ensure((size_t)pl.place_blocks << (2 + pl.bin_shift), &moved));
+    if (pl.place) CK(bin_total.ensure((size_t)pl.n_bins * 4, &moved));
     CK(tasks.ensure((size_t)pl.max_tasks * sizeof(Task), &moved));
     CK(partials.ensure((size_t)pl.max_tasks * MSM_BUCKET_BYTES, &moved));
     CK(order.ensure((size_t)pl.max_tasks * 4, &moved));
@@ -598,13 +644,20 @@ PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void
   pb.max_tasks = pl.max_tasks;
   pb.count = ws.count.as<uint32_t>();
   pb.offset = ws.offset.as<uint32_t>();
-  pb.fill = ws.fill.as<uint32_t>();
   pb.taskoff = ws.taskoff.as<uint32_t>();
   pb.scan_tmp = ws.scan_tmp.as<uint32_t>();
   pb.vals = ws.vals.as<uint32_t>();
-  pb.stage = pl.n_chunks ? ws.stage.as<uint2>() : nullptr;
+  pb.stage = pl.n_chunks && !pl.place ? ws.stage.as<uint2>() : nullptr;
   pb.blk_off = ws.blk_off.as<uint32_t>();
-  pb.stage_rank = pl.ranks && pb.stage ? ws.stage_rank.as<uint32_t>() : nullptr;
+  pb.stage_val = ws.stage.as<uint32_t>();
+  pb.stage_key = (uint16_t *)(pb.stage_val + pl.n_chunks * pl.stage_cap);
+  pb.part_first = ws.part_first.as<uint32_t>();
+  pb.place_part = kPlacePart;
+  pb.place_blocks = pl.place_blocks;
+  pb.bin_total = pl.place ? ws.bin_total.as<uint32_t>() : nullptr;
+  pb.chunk_points = pl.chunk_points;
+  pb.n_chunks = (uint32_t)pl.n_chunks;
+  pb.stage_rank = ws.stage_rank.as<uint32_t>();
   pb.stage_cap = pl.stage_cap;
   pb.bin_shift = pl.bin_shift;
   pb.n_bins = pl.n_bins;
@@ -803,11 +856,12 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
       for (JobSpec &sp : specs) sp.cfg.seg_len = seg;
     }
     Plan pl;
-    if (build_plan(specs, pl)) return g_err;
+    const bool pulls = !d_scalars && host_pullable(cx, h_scalars);
+    if (build_plan(specs, pl, pulls)) return g_err;
     const void *src = d_scalars, *pull = nullptr;
     if (!src) {
       CK(ws.scalars[0].ensure(first[m] * 32));
-      if (host_pullable(cx, h_scalars)) {
+      if (pulls) {
         pull = h_scalars;
       } else if (first[m]) {
         CK(cudaMemcpyAsync(ws.scalars[0].p, h_scalars, first[m] * 32, cudaMemcpyHostToDevice,
@@ -845,10 +899,11 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
     one[0] = {sizes[j], offs[j], d_scalars ? first[j] : 0, resolve_cfg(cx, sizes[j], opt)};
     set_tables(cx, one[0]);
     Plan pl;
-    if (build_plan(one, pl)) return g_err;
+    const bool pulls = !d_scalars && j == 0 && host_pullable(cx, h_scalars + first[j]);
+    if (build_plan(one, pl, pulls)) return g_err;
     const void *src = d_scalars, *pull = nullptr;
     const cudaEvent_t *chunks = nullptr;
-    if (!src && j == 0 && host_pullable(cx, h_scalars + first[j])) {
+    if (pulls) {
       // the first MSM's histogram kernel reads its scalars from host memory and leaves the
       // device copy; later MSMs' scalars are copied while the previous pass computes
       src = ws.scalars[(int)(j & 1)].p;
@@ -858,7 +913,7 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
       const int slot = (int)(j & 1);
       const int nch = Ctx::kCopyChunks;
       CK(cudaStreamWaitEvent(cx->copy_stream, cx->freed[slot], 0));
-      const uint64_t per = msm_upload_chunk_points(sizes[j], nch);
+      const uint64_t per = msm_upload_chunk_points(sizes[j], nch, pl.chunk_points);
       for (int c = 0; c < nch; c++) {
         const uint64_t a = std::min<uint64_t>((uint64_t)c * per, sizes[j]);
         const uint64_t b = std::min<uint64_t>(a + per, sizes[j]);

@@ -1,17 +1,18 @@
 // The MSM pipeline of one pass (one or many MSMs sharing one sort), all on the device:
 //
 //   1. k_count     signed c-bit digits of every scalar, histogram of (MSM, window, |digit|) keys;
-//                  stages each block's entries by key range (and uploads host scalars)
+//                  stages each block's entries by key range, with their ranks (and uploads host
+//                  scalars); k_partition, k_place_count: the same for large passes, by a partition
+//                  into key ranges and a count of each range in shared memory
 //   2. k_scan_*    exclusive scans -> bucket offsets in the sorted array and task offsets
-//   3. k_scatter_staged  counting-sort scatter of (base index | sign) into bucket order, one
-//                  launch per key range (k_scatter: the same from the scalars, for passes
-//                  without a stage)
+//   3. k_scatter_staged, k_place  (base index | sign) into bucket order (k_scatter: from the
+//                  scalars again, one launch per key range, for passes without a stage)
 //   4. k_tasks     split every bucket into runs of <= seg_len entries (load balance under skew)
 //   5. k_accumulate persistent: each thread sums one run of bases into a partial bucket sum
 //                  (the run's first base taken as is, then a 7-product mixed add per base);
-//                  k_accumulate_quad, k_merge_quad, k_reduce1_quad: four lanes a run, small passes
-//   6. k_merge_*   buckets split over several runs: sum of their partials (a thread, a warp or
-//                  a block per bucket, by the number of runs)
+//                  k_accumulate_quad, k_reduce1_quad: four lanes a run, small passes
+//   6. k_merge     buckets split over several runs: sum of their partials (a quad or a block per
+//                  bucket, by the number of runs)
 //   7. k_reduce1   per run of buckets: running sum R and triangle sum A (pippenger.h:25-33),
 //                  by the dedicated addition (8 products; the unified one where it fails)
 //   8. k_reduce2/3 combine runs into groups, groups into window sums (k_reduce3_small: one
@@ -29,6 +30,7 @@
 
 namespace {
 
+constexpr uint32_t kAllLanes = 0xffffffffu;
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanBlock = kScanThreads * kScanItems;
@@ -120,6 +122,8 @@ __global__ void __launch_bounds__(256) k_clear(PassBuffers pb) {
   for (uint32_t i = i0; i < pb.n_buckets; i += n) pb.count[i] = 0;
   for (uint32_t i = i0; i < 2 * (pb.seg_len + 1); i += n) pb.len_hist[i] = 0;
   if (i0 < CNT_WORDS) pb.counters[i0] = 0;
+  if (pb.bin_total)
+    for (uint32_t i = i0; i < pb.n_bins; i += n) pb.bin_total[i] = 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(256) k_clear(PassBuffers pb) {
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void count_key(const PassBuffers &pb, uint32_t key, uint32_t *sh_bins) {
   if (sh_bins) atomicAdd(&sh_bins[key >> pb.bin_shift], 1u);
-  if (pb.stage_rank) return;  // the bucket counts come with the ranks in stage_digits
+  if (pb.stage) return;  // the bucket counts come with the ranks in stage_digits
   // a warp whose active lanes all hit one bucket (e.g. equal scalars) adds once; otherwise
   // every lane adds on its own (distinct buckets for uniform scalars)
   const uint32_t active = __activemask();
@@ -160,34 +164,20 @@ __device__ __forceinline__ void stage_key(const PassBuffers &pb, uint32_t key, u
   const uint32_t pos = atomicAdd(&sh_cur[key >> pb.bin_shift], 1u);
   if (pos < pb.stage_cap) {
     chunk[pos] = make_uint2(key, val);
-    if (ranks) ranks[pos] = rank;
+    ranks[pos] = rank;
   } else {
     set_error(pb.counters, 6, pos);
   }
 }
 
-// The entries of one point, in window order; with ranks four windows per step, so that their atomics
-// on the bucket counts are in flight together (a small pass is bound by their round trips: k_count of
-// 4096 points 16 -> 13 us; without ranks one by one, 2^24 points 1.07 -> 1.03 ms).  A bucket count's
-// old value is the entry's rank in its bucket; one atomic per warp when its active lanes share the bucket.
+// The entries of one point, in window order, four windows per step, so that their atomics on the bucket
+// counts are in flight together (a small pass is bound by their round trips: k_count of 4096 points
+// 16 -> 13 us).  A bucket count's old value is the entry's rank in its bucket; one atomic per warp when its active lanes share the bucket.
 __device__ __forceinline__ void stage_digits(const PassBuffers &pb, const JobDesc &jd, ScalarBits s,
                                              uint64_t bidx, uint32_t *sh_cur, uint2 *chunk,
                                              uint32_t *ranks) {
   const int lane = threadIdx.x & 31;
   uint32_t carry = 0;
-  if (!ranks) {
-    for (uint32_t w = 0; w < jd.nwin; w++) {
-      const int32_t d = next_digit(s, jd, w, carry);
-      if (d == 0) continue;
-      const uint32_t mag = (uint32_t)abs(d);
-      const uint32_t ex = top_excess(jd, w, mag);
-      const uint64_t tidx = jd.tab_base + (jd.fixed ? (uint64_t)w * jd.fb_stride : 0) + bidx;
-      const uint32_t val = (uint32_t)tidx | (d < 0 ? 0x80000000u : 0u);
-      stage_key(pb, bucket_key(jd, w, mag - ex), val, 0, sh_cur, chunk, nullptr);
-      if (ex) stage_key(pb, bucket_key(jd, w, ex), val, 0, sh_cur, chunk, nullptr);
-    }
-    return;
-  }
   uint32_t extra_key = 0, extra_val = 0;  // a split top digit's second entry (see top_excess)
   bool extra = false;
 #pragma unroll 1
@@ -296,7 +286,7 @@ __global__ void __launch_bounds__(MSM_POINTS_PER_CHUNK) k_count(PassBuffers pb, 
   __syncthreads();
   if (ok)
     stage_digits(pb, jd, s, bidx, sh_cur, pb.stage + chunk * pb.stage_cap,
-                 pb.stage_rank ? pb.stage_rank + chunk * pb.stage_cap : nullptr);
+                 pb.stage_rank + chunk * pb.stage_cap);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -409,7 +399,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
   for (int k = 0; k < kScanItems; k++) {
     if (base + k < pb.n_buckets) {
       pb.offset[base + k] = ex.x;
-      pb.fill[base + k] = ex.x;  // the scatter's slot cursor starts at the bucket's offset
+      if (pb.fill) pb.fill[base + k] = ex.x;  // the scatter's slot cursor starts at the bucket's offset
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
@@ -454,7 +444,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
   for (int k = 0; k < kScanItems; k++) {
     if (base + k < pb.n_buckets) {
       pb.offset[base + k] = ex.x;
-      pb.fill[base + k] = ex.x;
+      if (pb.fill) pb.fill[base + k] = ex.x;
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
@@ -554,7 +544,7 @@ __global__ void k_scatter(PassBuffers pb, uint32_t key_lo, uint32_t key_hi) {
 }
 
 // Staged sort: the entries of key range `bin`, chunk by chunk (one block per histogram block),
-// each to the position its bucket's slot cursor returns.  The range's slice of the sorted array
+// each to its rank in its bucket.  The range's slice of the sorted array
 // stays in L2 while the launch runs.
 __global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t bin, uint32_t parts) {
   pdl_begin();
@@ -563,40 +553,357 @@ __global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t
   const uint32_t *bo = pb.blk_off + chunk * (pb.n_bins + 1);
   const uint32_t lo = bo[bin], hi = min(bo[bin + 1], pb.stage_cap);
   const uint2 *st = pb.stage + chunk * pb.stage_cap;
-  const uint32_t *rk = pb.stage_rank ? pb.stage_rank + chunk * pb.stage_cap : nullptr;
-  const int lane = threadIdx.x & 31;
+  const uint32_t *rk = pb.stage_rank + chunk * pb.stage_cap;
   for (uint32_t e = lo + (blockIdx.x % parts) * blockDim.x + threadIdx.x; e < hi; e += parts * blockDim.x) {
     const uint2 kv = st[e];
     if (kv.x >= pb.n_buckets) {  // cannot happen for a consistent stage; never write out of bounds
       set_error(pb.counters, 7, kv.x);
       continue;
     }
-    if (rk) {  // position known from the rank: no atomic
-      const uint32_t p = pb.offset[kv.x] + rk[e];
-      if (p < pb.max_entries) {
-        pb.vals[p] = kv.y;
-      } else {
-        set_error(pb.counters, 3, p);
-      }
-      continue;
+    const uint32_t p = pb.offset[kv.x] + rk[e];
+    if (p < pb.max_entries) pb.vals[p] = kv.y;
+    else set_error(pb.counters, 3, p);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// 1 and 3 of a large pass, without an atomic or a scattered access to global memory per entry (those
+// bound k_count and k_scatter_staged: two L2 round trips an entry each, 1e8 entries 3.4 ms, where the
+// bytes take 0.3).  k_partition sorts the entries of a chunk of points by key range in shared memory
+// and copies them out in that order; k_place_count and k_place give a key range's entries, a piece from
+// every chunk, to one block (or, split by chunks, to several), which counts and ranks them in its
+// shared memory.  The ranges are narrow enough that a block's slice of the sorted array stays in L2
+// until its sectors are full, and a bucket's entries come in the order of the points, roughly: an order
+// that is random over the whole set slows k_accumulate by 0.9% (3e6 points), by its reach in memory.
+// Measured on GB300 (count + scan + scatter, ms, ranked or cursor sort / this one): 1e6 points 0.290 /
+// 0.205, 2^21 without tables 0.596 / 0.415, 2^24 3.50 / 2.60, the uneven mix of 64 3.51 / 1.85, 4 x
+// 50000 (3.2e6 entries) 0.112 / 0.127.  What bounds them now, in the mix: k_partition 0.55 ms (issue
+// slots half used, the shared-memory pipe 65%), k_place_count 0.28 (issue slots), k_place 0.9 (L2:
+// 4-byte writes, a sector each).  Sorting k_place's entries in shared memory too, to write them out in
+// runs, halves the sectors and takes 1.2.
+// ---------------------------------------------------------------------------------------------
+constexpr int kPartThreads = 1024;
+
+constexpr uint32_t kPlaceChunks = MSM_PLACE_CHUNKS;
+constexpr int kPlaceThreads = 1024;
+constexpr int kPlaceUnroll = 4;
+
+// The job of point g, walking on from job j.
+__device__ __forceinline__ uint32_t next_job(const JobDesc *jobs, uint32_t n_jobs, uint32_t j, uint64_t g) {
+  while (j + 1 < n_jobs && jobs[j + 1].point_begin <= g) j++;
+  return j;
+}
+
+// f(key, value) for every entry of a point.  The widths that large passes use have every bit position
+// known at compile time (C), with signed digits; C = 0 takes any job.
+template <uint32_t C, class F>
+__device__ __forceinline__ void for_digits_c(const JobDesc &jd, ScalarBits s, uint64_t bidx, F f) {
+  uint32_t carry = 0;
+  uint32_t tidx = (uint32_t)(jd.tab_base + bidx);  // indices are below 2^31
+  const uint32_t tstep = jd.fixed ? (uint32_t)jd.fb_stride : 0u, kstep = jd.fixed ? 0u : jd.nb;
+  uint32_t k0 = jd.bucket_begin - 1u;
+  auto entry = [&](int32_t d, bool top) {
+    if (d == 0) return;
+    const uint32_t mag = (uint32_t)abs(d), ex = top && mag > jd.nb_top ? mag - jd.nb_top : 0u;
+    const uint32_t val = tidx | ((uint32_t)d & 0x80000000u);
+    f(k0 + mag - ex, val);
+    if (ex) f(k0 + ex, val);
+  };
+  if constexpr (C == 0) {
+    for (uint32_t w = 0; w < jd.nwin; w++) {
+      entry(next_digit(s, jd, w, carry), w + 1 == jd.nwin);
+      tidx += tstep;
+      k0 += kstep;
     }
-    uint32_t pos;
-    const uint32_t active = __activemask();
-    const int leader = __ffs(active) - 1;
-    const uint32_t k0 = __shfl_sync(active, kv.x, leader);
-    if (__all_sync(active, kv.x == k0)) {  // one bucket for the whole warp: one atomic
-      uint32_t bp = 0;
-      if (lane == leader) bp = atomicAdd(&pb.fill[kv.x], (uint32_t)__popc(active));
-      pos = __shfl_sync(active, bp, leader) + __popc(active & ((1u << lane) - 1u));
-    } else {
-      pos = atomicAdd(&pb.fill[kv.x], 1u);
-    }
-    if (pos < pb.max_entries) {
-      pb.vals[pos] = kv.y;
-    } else {
-      set_error(pb.counters, 3, pos);
+  } else {
+    constexpr uint32_t W = (MSM_SCALAR_BITS + C - 1) / C;
+#pragma unroll
+    for (uint32_t w = 0; w < W; w++) {
+      const uint32_t i = w * C / 32, o = w * C % 32;
+      const uint32_t v = o + C <= 32 || i == 7 ? s.w[i] >> o : __funnelshift_r(s.w[i], s.w[(i + 1) & 7], o);
+      int32_t d = (int32_t)((v & ((1u << C) - 1u)) + carry);
+      carry = w + 1 < W && d >= (int32_t)(1u << (C - 1));
+      if (carry) d -= (int32_t)(1u << C);
+      entry(d, w + 1 == W);
+      tidx += tstep;
+      k0 += kstep;
     }
   }
+}
+template <class F>
+__device__ __forceinline__ void for_digits(const JobDesc &jd, const ScalarBits &s, uint64_t bidx, F f) {
+  if (!jd.signed_digits) return for_digits_c<0>(jd, s, bidx, f);
+  switch (jd.c) {
+    case 14: return for_digits_c<14>(jd, s, bidx, f);
+    case 15: return for_digits_c<15>(jd, s, bidx, f);
+    case 16: return for_digits_c<16>(jd, s, bidx, f);
+    case 17: return for_digits_c<17>(jd, s, bidx, f);
+    case 18: return for_digits_c<18>(jd, s, bidx, f);
+    case 19: return for_digits_c<19>(jd, s, bidx, f);
+    case 20: return for_digits_c<20>(jd, s, bidx, f);
+    case 21: return for_digits_c<21>(jd, s, bidx, f);
+    case 22: return for_digits_c<22>(jd, s, bidx, f);
+    case 23: return for_digits_c<23>(jd, s, bidx, f);
+    default: return for_digits_c<0>(jd, s, bidx, f);
+  }
+}
+
+// One chunk of chunk_points points per block: its entries, grouped by key range in shared memory and
+// then copied to the chunk's part of the stage (values, and keys less the range's first one).
+// blk_off[range * n_chunks + chunk] is where a range starts there.
+__global__ void __launch_bounds__(kPartThreads) k_partition(PassBuffers pb, uint64_t g_begin, uint64_t g_end) {
+  pdl_begin();
+  extern __shared__ uint32_t sh[];
+  uint32_t *const cur = sh;                               // [n_bins] counts, then cursors
+  uint32_t *const sval = sh + pb.n_bins;                  // [stage_cap]
+  uint16_t *const skey = (uint16_t *)(sval + pb.stage_cap);  // [stage_cap]
+  const uint32_t tid = threadIdx.x, low = (1u << pb.bin_shift) - 1u;
+  for (uint32_t i = tid; i < pb.n_bins; i += kPartThreads) cur[i] = 0;
+  const uint64_t c0 = g_begin + (uint64_t)blockIdx.x * pb.chunk_points;
+  const uint64_t c1 = min(min(c0 + pb.chunk_points, g_end), pb.n_points);
+  const uint64_t chunk = c0 / pb.chunk_points;
+  const uint32_t j0 = find_job(pb.jobs, pb.n_jobs, c0);
+  __syncthreads();
+  uint32_t j = j0;
+  for (uint64_t g = c0 + tid; g < c1; g += kPartThreads) {
+    j = next_job(pb.jobs, pb.n_jobs, j, g);
+    const JobDesc jd = pb.jobs[j];
+    const uint64_t i = g - jd.point_begin;
+    const uint64_t si = 2 * (jd.scalar_off + i);
+    uint4 a, b;
+    if (pb.host_scalars) {  // fused upload, see k_count
+      a = pb.host_scalars[si];
+      b = pb.host_scalars[si + 1];
+      uint4 *dst = const_cast<uint4 *>(pb.scalars) + si;
+      dst[0] = a;
+      dst[1] = b;
+    } else {
+      a = pb.scalars[si];
+      b = pb.scalars[si + 1];
+    }
+    if (pb.flags[jd.base_off + i] != BASE_OK) continue;
+    for_digits(jd, scalar_bits(a, b), 0, [&](uint32_t key, uint32_t) { atomicAdd(&cur[key >> pb.bin_shift], 1u); });
+  }
+  __syncthreads();
+  uint2 all;
+  {
+    const uint32_t per = (pb.n_bins + kPartThreads - 1) / kPartThreads, r0 = tid * per;
+    const uint32_t r1 = min(r0 + per, pb.n_bins);
+    uint2 sum = make_uint2(0, 0);
+    for (uint32_t r = r0; r < r1; r++) sum.x += cur[r];
+    uint32_t at = block_excl_scan2(sum, all).x;
+    for (uint32_t r = r0; r < r1; r++) {
+      const uint32_t c = cur[r];
+      pb.blk_off[(uint64_t)r * pb.n_chunks + chunk] = at;
+      if (c) atomicAdd(&pb.bin_total[r], c);
+      cur[r] = at;
+      at += c;
+    }
+    if (tid == 0) pb.blk_off[(uint64_t)pb.n_bins * pb.n_chunks + chunk] = all.x;
+  }
+  __syncthreads();
+  j = j0;
+  for (uint64_t g = c0 + tid; g < c1; g += kPartThreads) {
+    j = next_job(pb.jobs, pb.n_jobs, j, g);
+    const JobDesc jd = pb.jobs[j];
+    const uint64_t i = g - jd.point_begin;
+    const uint64_t bidx = jd.base_off + i;
+    if (pb.flags[bidx] != BASE_OK) continue;
+    const ScalarBits s = load_scalar(pb.scalars + 2 * (jd.scalar_off + i));
+    for_digits(jd, s, bidx, [&](uint32_t key, uint32_t val) {
+      const uint32_t pos = atomicAdd(&cur[key >> pb.bin_shift], 1u);
+      if (pos < pb.stage_cap) {
+        sval[pos] = val;
+        skey[pos] = (uint16_t)(key & low);
+      } else {
+        set_error(pb.counters, 6, pos);
+      }
+    });
+  }
+  __syncthreads();
+  const uint64_t at = chunk * pb.stage_cap;
+  const uint32_t n = min(all.x, pb.stage_cap);
+  for (uint32_t e = tid; e < n; e += kPartThreads) pb.stage_val[at + e] = sval[e];
+  for (uint32_t e = tid; 2 * e < n; e += kPartThreads)  // the capacity is even
+    ((uint32_t *)(pb.stage_key + at))[e] = ((const uint32_t *)skey)[e];
+}
+
+// A part of a key range: its entries from a stretch of the chunks.  A range of more than place_part
+// entries (or more than kPlaceChunks chunks) has several parts, a block each, so that the buckets of a
+// narrow top window or of repeated scalars don't leave one block with most of the work.
+struct PlacePart {
+  uint32_t bin, k0, nk;  // key range, its first bucket and buckets
+  uint32_t part, parts;  // which of the range's parts
+  uint32_t nc, total;    // chunks and entries of the part
+  uint32_t *cnt, *pre, *src;
+};
+
+__device__ __forceinline__ uint32_t parts_of(const PassBuffers &pb, uint32_t total) {
+  const uint32_t a = (total + pb.place_part - 1) / pb.place_part, b = (pb.n_chunks + kPlaceChunks - 1) / kPlaceChunks;
+  return min(max(max(a, b), 1u), pb.n_chunks);
+}
+
+// the part of this block; false when the block has none
+__device__ __forceinline__ bool place_part(const PassBuffers &pb, uint32_t *sh, PlacePart &p) {
+  __shared__ uint32_t found[3];  // range, part, parts
+  const uint32_t tid = threadIdx.x;
+  uint2 all;
+  {
+    const uint32_t per = (pb.n_bins + kPlaceThreads - 1) / kPlaceThreads, r0 = min(tid * per, pb.n_bins);
+    const uint32_t r1 = min(r0 + per, pb.n_bins);
+    uint2 v = make_uint2(0, 0);
+    for (uint32_t r = r0; r < r1; r++) v.x += parts_of(pb, pb.bin_total[r]);
+    uint32_t at = block_excl_scan2(v, all).x;
+    for (uint32_t r = r0; r < r1; r++) {
+      const uint32_t n = parts_of(pb, pb.bin_total[r]);
+      if (blockIdx.x >= at && blockIdx.x < at + n) {
+        found[0] = r;
+        found[1] = blockIdx.x - at;
+        found[2] = n;
+      }
+      at += n;
+    }
+  }
+  if (blockIdx.x >= all.x) return false;
+  __syncthreads();
+  p.bin = found[0];
+  p.part = found[1];
+  p.parts = found[2];
+  p.k0 = p.bin << pb.bin_shift;
+  p.nk = min(1u << pb.bin_shift, pb.n_buckets - p.k0);
+  const uint32_t c0 = (uint32_t)((uint64_t)pb.n_chunks * found[1] / p.parts);
+  const uint32_t nc = (uint32_t)((uint64_t)pb.n_chunks * (found[1] + 1) / p.parts) - c0;
+  p.cnt = sh;
+  p.pre = sh + (1u << pb.bin_shift);
+  p.src = p.pre + kPlaceChunks + 1;
+  const uint32_t *row = pb.blk_off + (uint64_t)p.bin * pb.n_chunks + c0;
+  const uint32_t per = (nc + kPlaceThreads - 1) / kPlaceThreads, a = min(tid * per, nc), b = min(a + per, nc);
+  uint2 v = make_uint2(0, 0);
+  for (uint32_t c = a; c < b; c++) {
+    const uint32_t st = row[c], n = row[pb.n_chunks + c] - st;
+    p.src[c] = (c0 + c) * pb.stage_cap + st;  // below 2^32: the plan's limit on entries
+    p.pre[c] = n;
+    v.x += n;
+  }
+  uint32_t at = block_excl_scan2(v, all).x;
+  for (uint32_t c = a; c < b; c++) {
+    const uint32_t n = p.pre[c];
+    p.pre[c] = at;
+    p.src[c] -= at;
+    at += n;
+  }
+  if (tid == 0) p.pre[nc] = all.x;
+  p.nc = nc;
+  p.total = all.x;
+  __syncthreads();
+  return true;
+}
+
+// f(loaded entries, their number) for the part's entries, spread over the block's threads: its pieces, one per
+// chunk, are walked as one array, the warps taking stretches of it in turn, U entries a lane in flight.
+template <int U, class L, class F>
+__device__ __forceinline__ void for_part_entries(const PlacePart &p, L load, F f) {
+  constexpr uint32_t nw = kPlaceThreads / 32;
+  const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t stretch = 256;
+  uint32_t c = 0;
+  for (uint32_t b0 = wid * stretch; b0 < p.total; b0 += nw * stretch) {
+    uint32_t hi = p.nc;
+    while (hi - c > 1) {  // the last piece that starts at or before the stretch
+      const uint32_t mid = (c + hi) >> 1;
+      if (p.pre[mid] <= b0) c = mid; else hi = mid;
+    }
+    const uint32_t b1 = min(b0 + stretch, p.total);
+    uint32_t i = c, end = p.pre[c + 1], src = p.src[c], e = b0 + lane;
+    auto next = [&] {
+      while (e >= end) {
+        i++;
+        end = p.pre[i + 1];
+        src = p.src[i];
+      }
+      return src + e;
+    };
+    uint2 kv[U];
+    for (; e - lane + 32 * U <= b1;) {
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        kv[k] = load(next());
+        e += 32;
+      }
+      f(kv, U);
+    }
+    for (; e < b1; e += 32) {
+      kv[0] = load(next());
+      f(kv, 1);
+    }
+  }
+}
+
+// The bucket counts.  Parts of one range add theirs up; what a bucket held before is where the part's
+// entries start in it.
+__global__ void __launch_bounds__(kPlaceThreads, 2) k_place_count(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  extern __shared__ uint32_t sh[];
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  for (uint32_t i = tid; i < (1u << pb.bin_shift); i += kPlaceThreads) sh[i] = 0;
+  PlacePart p;
+  if (!place_part(pb, sh, p)) return;
+  for_part_entries<8>(p, [&](uint32_t at) { return make_uint2(__ldcs(pb.stage_key + at), 0); },
+                      [&](const uint2 *kv, int n) {
+                        for (int k = 0; k < n; k++) atomicAdd(&p.cnt[kv[k].x], 1u);
+                      });
+  __syncthreads();
+  uint32_t *const first = pb.part_first + ((uint64_t)blockIdx.x << pb.bin_shift);
+  for (uint32_t k = tid; k < p.nk; k += kPlaceThreads) {
+    if (p.parts == 1) {
+      pb.count[p.k0 + k] = p.cnt[k];
+    } else {
+      first[k] = p.cnt[k];
+      if (p.cnt[k]) atomicAdd(&pb.count[p.k0 + k], p.cnt[k]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kPlaceThreads, 2) k_place(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  extern __shared__ uint32_t sh[];
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  PlacePart p;
+  if (!place_part(pb, sh, p)) return;
+  const uint32_t *const first = pb.part_first + ((uint64_t)(blockIdx.x - p.part) << pb.bin_shift);
+  for (uint32_t k = tid; k < p.nk; k += kPlaceThreads) {
+    uint32_t at = pb.offset[p.k0 + k];
+#pragma unroll 4
+    for (uint32_t q = 0; q < p.part; q++) at += first[((uint64_t)q << pb.bin_shift) + k];
+    p.cnt[k] = at;
+  }
+  __syncthreads();
+  for_part_entries<kPlaceUnroll>(
+      p, [&](uint32_t at) { return make_uint2(__ldcs(pb.stage_key + at), __ldcs(pb.stage_val + at)); },
+      [&](const uint2 *kv, int m) {
+        uint32_t pos[kPlaceUnroll];
+        // one bucket for all of the warp's entries (equal scalars): one atomic
+        bool same = m == kPlaceUnroll;
+        if (same) {
+          const uint32_t k0 = __shfl_sync(kAllLanes, kv[0].x, 0);
+          for (int k = 0; k < kPlaceUnroll; k++) same = same && kv[k].x == k0;
+          same = __all_sync(kAllLanes, same);
+          if (same) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&p.cnt[k0], 32u * kPlaceUnroll);
+            at = __shfl_sync(kAllLanes, at, 0) + lane;
+            for (int k = 0; k < kPlaceUnroll; k++) pos[k] = at + 32 * k;
+          }
+        }
+        if (!same)
+          for (int k = 0; k < m; k++) pos[k] = atomicAdd(&p.cnt[kv[k].x], 1u);
+        for (int k = 0; k < m; k++) {
+          if (pos[k] < pb.max_entries) pb.vals[pos[k]] = kv[k].y;
+          else set_error(pb.counters, 3, pos[k]);
+        }
+      });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1127,7 +1434,6 @@ __global__ void __launch_bounds__(128) k_reduce1_quad(PassBuffers pb) {
 
 constexpr int kRedThreads = 256;
 constexpr uint32_t kRedQuads = kRedThreads / 4;
-constexpr uint32_t kAllLanes = 0xffffffffu;
 
 // Levels 2 and 3 are chains of dependent additions, so they run on quads: every quad of the
 // block executes every addition (a quad with nothing to add adds the identity), which keeps the
@@ -1455,40 +1761,32 @@ uint32_t msm_scatter_passes(uint64_t max_entries) {
   return (uint32_t)(p < 1 ? 1 : p > 8 ? 8 : p);
 }
 
-// Key ranges of the staged sort, as a shift of the bucket key (ranges of 2^shift keys, at most
+// Key ranges of the ranked sort, as a shift of the bucket key (ranges of 2^shift keys, at most
 // MSM_MAX_BINS of them).
-//   * Ranks (`cursors` false), one MSM: one range per ~16 MB of sorted array, at most ten.  Measured
-//     on GB300 (scatter, us, 1 / 4 / 8 / 16 ranges): 2^20 points (13.6e6 entries) 146 / 125 / 135 / 162,
-//     2^21 without tables (31e6) 520 / 311 / 288 / 298, 3e6 (39e6) 490 / 383 / 350 / 353.
+//   * One MSM: one range per ~16 MB of sorted array, at most ten.  Measured on GB300 (scatter, us,
+//     1 / 4 / 8 / 16 ranges): 2^20 points (13.6e6 entries) 146 / 125 / 135 / 162, 2^21 without tables
+//     (31e6) 520 / 311 / 288 / 298, 3e6 (39e6) 490 / 383 / 350 / 353.
 //   * Several MSMs (`many`): one range.  Each MSM's points and buckets are contiguous, so the blocks in
-//     flight stay within one or two MSMs' slices by themselves (the uneven mix of 64, 1.1e8 entries,
-//     1 / 2 / 4 / 8 / 16 ranges: 2.06 / 2.13 / 2.23 / 2.54 / 3.01 ms).
-//   * Slot cursors, one MSM: one per ~150 MB, and no more than 2^19 keys per range while that keeps MSM_MAX_BINS
-//     ranges or fewer.  The keys a scatter launch touches bound its slot-cursor footprint: 2^24 points
-//     (4.9 M buckets), ranges of 2^20 keys (5 launches) took 3.86 ms, 2^19 (10) 2.42 ms and 2^18 (19)
-//     2.49 ms; 2^26 points use 2^18.
+//     flight stay within one or two MSMs' slices by themselves.
 // `ranges` > 0 asks for that many ranges instead (rounded to a shift).
-uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool cursors, bool many) {
-  const uint64_t per = cursors ? 150ull << 20 : 16ull << 20;
+uint32_t msm_bin_shift(uint32_t n_buckets, uint64_t max_entries, uint32_t ranges, bool many) {
+  const uint64_t per = 16ull << 20;
   uint64_t want = ranges ? ranges : (max_entries * 4 + per / 2) / per;
-  if (!ranges && many) want = 1;
-  else if (!ranges && !cursors) want = std::min<uint64_t>(want, 10);
+  if (!ranges) want = many ? 1 : std::min<uint64_t>(want, 10);
   const uint32_t target = (uint32_t)(want < 1 ? 1 : want > MSM_MAX_BINS ? MSM_MAX_BINS : want);
   uint32_t shift = 0;
   while (shift < 31 && (((uint64_t)n_buckets + (1ull << shift) - 1) >> shift) > target) shift++;
-  if (!ranges && cursors && !many)
-    while (shift > 19 &&
-           (((uint64_t)n_buckets + (1ull << (shift - 1)) - 1) >> (shift - 1)) <= MSM_MAX_BINS)
-      shift--;
   return shift;
 }
 
 // Points per chunk of a chunked scalar upload: a multiple of the histogram block, so every block
 // of a chunk's histogram launch is a whole chunk of the stage.
-uint64_t msm_upload_chunk_points(uint64_t n_points, int nchunks) {
+uint64_t msm_upload_chunk_points(uint64_t n_points, int nchunks, uint32_t chunk_points) {
   const uint64_t per = (n_points + nchunks - 1) / nchunks;
-  return (per + MSM_POINTS_PER_CHUNK - 1) / MSM_POINTS_PER_CHUNK * MSM_POINTS_PER_CHUNK;
+  return (per + chunk_points - 1) / chunk_points * chunk_points;
 }
+
+size_t msm_partition_smem(uint32_t n_bins, uint32_t stage_cap) { return (size_t)n_bins * 4 + (size_t)stage_cap * 6; }
 
 size_t msm_scan_tmp_words(uint32_t n_buckets) {
   return 2ull * ((n_buckets + kScanBlock - 1) / kScanBlock) + 2;
@@ -1528,10 +1826,26 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   run(k_clear, std::min<uint32_t>(num_sms * 8, pb.n_buckets / 1024 + 1), 256, 0, pb);
   mark(0);
   const uint32_t pts_blocks = (uint32_t)((pb.n_points + 255) / 256);
-  if (pb.n_points > 0) {
+  const size_t part_smem = msm_partition_smem(pb.n_bins, pb.stage_cap);
+  const size_t place_smem = ((1u << pb.bin_shift) + 2 * kPlaceChunks + 1) * 4;
+  if (pb.n_points > 0 && pb.bin_total) {
+    if ((e = cudaFuncSetAttribute(k_partition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem)) ||
+        (e = cudaFuncSetAttribute(k_place_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place_smem)) ||
+        (e = cudaFuncSetAttribute(k_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place_smem)))
+      return e;
+    const uint64_t per = chunk_ready && nchunks > 0
+                             ? msm_upload_chunk_points(pb.n_points, nchunks, pb.chunk_points) : pb.n_points;
+    for (uint64_t g0 = 0, c = 0; g0 < pb.n_points; g0 += per, c++) {
+      const uint64_t g1 = std::min(g0 + per, pb.n_points);
+      if (chunk_ready && (e = cudaStreamWaitEvent(st, chunk_ready[c], 0))) return e;
+      run(k_partition, (uint32_t)((g1 - g0 + pb.chunk_points - 1) / pb.chunk_points), kPartThreads, part_smem, pb,
+          g0, g1);
+    }
+    run(k_place_count, pb.place_blocks, kPlaceThreads, place_smem, pb);
+  } else if (pb.n_points > 0) {
     if (chunk_ready && nchunks > 0) {
       // the scalars arrive in chunks on another stream: count each chunk as soon as it lands
-      const uint64_t per = msm_upload_chunk_points(pb.n_points, nchunks);
+      const uint64_t per = msm_upload_chunk_points(pb.n_points, nchunks, MSM_POINTS_PER_CHUNK);
       for (int c = 0; c < nchunks; c++) {
         const uint64_t g0 = (uint64_t)c * per, g1 = g0 + per < pb.n_points ? g0 + per : pb.n_points;
         if ((e = cudaStreamWaitEvent(st, chunk_ready[c], 0))) return e;
@@ -1552,7 +1866,9 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
     run(k_scan_apply, nblk, kScanThreads, 0, pb);
   }
   mark(2);
-  if (pb.n_points > 0 && pb.stage) {
+  if (pb.n_points > 0 && pb.bin_total) {
+    run(k_place, pb.place_blocks, kPlaceThreads, place_smem, pb);
+  } else if (pb.n_points > 0 && pb.stage) {
     // few chunks: several blocks each (a block walks a chunk of 256 points in ~17 dependent steps; 4096
     // points, 16 chunks: 12.8 us with a block each, 4.6 with eight)
     const uint32_t parts = std::max(1u, std::min(8u, (uint32_t)num_sms * 16u / pts_blocks));
