@@ -103,6 +103,7 @@ struct PassBuffers {
   uint32_t red_len_log2;        // level-1 reduction segment length = 1 << red_len_log2
   uint32_t grp_len_log2;        // level-2 group = 1 << grp_len_log2 level-1 segments
   uint32_t n_grps;              // level-2 groups
+  uint32_t min_grps, max_grps;  // least and most groups of a window
   uint64_t max_entries;         // capacity of vals
   uint32_t max_tasks;           // capacity of tasks / partials
 

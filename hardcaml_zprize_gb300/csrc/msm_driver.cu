@@ -636,6 +636,11 @@ PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void
   pb.n_buckets = pl.n_buckets;
   pb.n_segs = pl.n_segs;
   pb.n_grps = pl.n_grps;
+  pb.min_grps = ~0u;
+  for (const WinDesc &wd : pl.wins) {
+    pb.min_grps = std::min(pb.min_grps, wd.ngrp);
+    pb.max_grps = std::max(pb.max_grps, wd.ngrp);
+  }
   pb.seg_len = pl.seg_len;
   pb.seg_shift = seg_shift_of(pl.seg_len);
   pb.red_len_log2 = pl.red_log2;
@@ -2311,6 +2316,8 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.n_buckets = nbk;
   pb.n_segs = nsegs;
   pb.n_grps = ngrps;
+  pb.min_grps = jd.fixed ? ngrps : 0u;  // windows: both level-3 kernels run
+  pb.max_grps = ngrps;
   pb.seg_len = seg_len;
   pb.seg_shift = seg_shift_of(seg_len);
   pb.red_len_log2 = red_log2;

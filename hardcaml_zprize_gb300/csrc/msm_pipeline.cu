@@ -1529,7 +1529,7 @@ __device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log
 #pragma unroll 1
   for (uint32_t k = per - 1; k-- > 0;) {
     const uint32_t i = i0 + k;
-    T = dq_add(T, RR, kAllLanes);
+    T = k + 2 == per ? RR : dq_add(T, RR, kAllLanes);
     fq_t R = dq_identity(), A = dq_identity();
     if (i < cnt) {
       R = dq_load(items + (size_t)i * 24);
@@ -1652,9 +1652,9 @@ __global__ void __launch_bounds__(kRedThreads) k_merge(PassBuffers pb) {
     const uint32_t b = pb.heavy[pb.n_buckets - 1 - h];
     const uint32_t nt = ntask_of(pb.count[b], pb);
     const uint32_t t0 = pb.taskoff[b];
-    fq_t acc = dq_identity();
+    fq_t acc = q < nt ? dq_load(pb.partials + (size_t)(t0 + q) * 12) : dq_identity();
 #pragma unroll 1
-    for (uint32_t k0 = 0; k0 < nt; k0 += kRedQuads) {  // the same trip count for every quad
+    for (uint32_t k0 = kRedQuads; k0 < nt; k0 += kRedQuads) {  // the same trip count for every quad
       const fq_t p = k0 + q < nt ? dq_load(pb.partials + (size_t)(t0 + k0 + q) * 12) : dq_identity();
       acc = dq_add(acc, p, kAllLanes);
     }
@@ -1912,8 +1912,10 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   }
   mark(8);
   if (pb.n_wins > 0) {
-    run(k_reduce3_small, (pb.n_wins + 31) / 32, 128, 0, pb);
-    if (pb.n_wins <= (uint32_t)num_sms)
+    if (pb.min_grps <= kRed3SmallMax) run(k_reduce3_small, (pb.n_wins + 31) / 32, 128, 0, pb);
+    if (pb.max_grps <= kRed3SmallMax) {
+      // no window for k_reduce3
+    } else if (pb.n_wins <= (uint32_t)num_sms)
       run(k_reduce3<128>, pb.n_wins, 128, 0, pb);
     else
       run(k_reduce3<256>, pb.n_wins, 256, 0, pb);
