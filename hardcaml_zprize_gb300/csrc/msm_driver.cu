@@ -246,11 +246,11 @@ uint32_t quad_run(double mean) {
 // balance the two.  Measured on GB300 (one MSM on width-16 tables, mean bucket load 8: 2^14
 // points): runs of 8 0.72 ms, 4 0.71 ms, 16 0.82 ms; at load 2 (2^12 points) runs of 2 to 32
 // are within 4% of each other, and at load 32 (2^16 points) 16 is best (1.06 ms, 8: 1.08 ms).
-uint32_t seg_len_for(uint64_t n, uint32_t nb, uint32_t nwin_sharing, uint32_t epp) {
+uint32_t seg_len_for(uint64_t n, uint32_t nb, uint32_t nwin_sharing, uint32_t nwin, uint32_t epp) {
   const double mean = (double)n * nwin_sharing / std::max<uint32_t>(nb, 1);
   const uint32_t s = whole_bucket_run(mean);
-  const uint64_t entries = n * (uint64_t)epp;  // as the plan counts them
-  if (entries <= kQuadEntries) return quad_run(mean);
+  if (n * (uint64_t)epp <= kQuadEntries) return quad_run(mean);  // as the plan counts entries
+  const uint64_t entries = n * (uint64_t)nwin;
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 18) <= entries) cap <<= 1;  // entries / cap >= 2^17
   uint32_t r = std::min(s, cap);
@@ -274,7 +274,7 @@ Cfg heuristic_cfg(uint64_t n) {
   }
   uint32_t nwin, nb, nbt;
   layout(cfg.c, 1, nwin, nb, nbt);
-  cfg.seg_len = seg_len_for(n, nb, 1, entries_per_point(cfg.c, 1));
+  cfg.seg_len = seg_len_for(n, nb, 1, nwin, entries_per_point(cfg.c, 1));
   cfg.red_log2 = 0;
   return cfg;
 }
@@ -771,7 +771,7 @@ Cfg resolve_cfg(Ctx *cx, uint64_t n, const msm_options_t *opt, bool shared_pass 
       cfg.c = (uint32_t)std::min(std::max(opt->window_bits, 4), 22);
       uint32_t nwin, nb, nbt;
       layout(cfg.c, 1, nwin, nb, nbt);
-      cfg.seg_len = seg_len_for(n, nb, 1, entries_per_point(cfg.c, 1));
+      cfg.seg_len = seg_len_for(n, nb, 1, nwin, entries_per_point(cfg.c, 1));
     }
     if (opt->signed_digits == 1) cfg.signed_digits = 1;
     if (opt->signed_digits == 2) cfg.signed_digits = 0;
@@ -810,7 +810,7 @@ Cfg resolve_cfg(Ctx *cx, uint64_t n, const msm_options_t *opt, bool shared_pass 
     cfg.c = table_c(use);
     cfg.signed_digits = 1;
     if (tuned_fixed != use) {
-      cfg.seg_len = seg_len_for(n, std::max(nb, nbt), nwin, entries_per_point(cfg.c, 1));
+      cfg.seg_len = seg_len_for(n, std::max(nb, nbt), nwin, nwin, entries_per_point(cfg.c, 1));
       cfg.red_log2 = 0;
     }
   }
@@ -1639,7 +1639,7 @@ int msm_tune(void *context, uint64_t npoints, int32_t budget_ms, msm_options_t *
     cf.fixed = which;
     cf.c = tc;
     cf.signed_digits = 1;
-    cf.seg_len = seg_len_for(npoints, std::max(nb, nbt), nwin, entries_per_point(tc, 1));
+    cf.seg_len = seg_len_for(npoints, std::max(nb, nbt), nwin, nwin, entries_per_point(tc, 1));
     cf.red_log2 = 0;
     cands.push_back(cf);
     Cfg cf2 = cf;
