@@ -1808,6 +1808,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   };
   // one launch: kernel k on `grid` blocks, dependent on the one before it (see pdl_wait)
   cudaError_t bad = cudaSuccess;
+  bool dependent = true;
   auto run = [&](auto k, uint32_t grid, uint32_t block, size_t smem, auto... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1818,7 +1819,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     const cudaError_t r = cudaLaunchKernelEx(&cfg, k, args...);
     if (r != cudaSuccess && bad == cudaSuccess) bad = r;
     launched++;
@@ -1887,11 +1888,16 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
     run(k_tasks, (pb.n_buckets + 255) / 256, 256, 2 * (pb.seg_len + 1) * 4, pb);
   }
   mark(4);
+  // Fewer blocks than an SM holds (a server's passes) start when k_tasks has left: set up beside its
+  // blocks they would share some SMs four by four and leave others with two.  Measured on GB300, three
+  // per SM: 2^20 points 4.50 ms set up early, 3.72 ms so.
+  dependent = !pb.acc_blocks_per_sm;
   const uint32_t acc_blocks = num_sms * (pb.acc_blocks_per_sm ? pb.acc_blocks_per_sm : 4);
   if (pb.quads)
     run(k_accumulate_quad, acc_blocks, 128, 0, pb);
   else
     run(k_accumulate, acc_blocks, 128, 0, pb);
+  dependent = true;
   mark(5);
   run(k_merge, num_sms * 2, kRedThreads, 0, pb);
   mark(6);
