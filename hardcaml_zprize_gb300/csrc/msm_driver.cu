@@ -136,21 +136,18 @@ struct Cfg {
                        // then the tables' width); 0: windowed over the plain bases
 };
 
-// Level-1 reduction runs of 2^red buckets, 4 to 64.  Small passes are latency-bound: each thread
-// adds 2 x 2^red points in sequence.  Passes of 2^22 buckets or more take runs of 64 (about 2^16
+// Level-1 reduction runs of 2^red buckets, 4 to 64.  Small passes are latency-bound: each quad or
+// thread adds 2 x 2^red points in sequence.  Passes of 2^22 buckets or more take runs of 64 (about 2^16
 // of them still keep k_reduce1 near the product throughput), which leaves fewer groups for the
-// latency-bound levels 2 and 3.  Measured on GB300:
-//   2^15 buckets (one MSM on tables of width 16): 4 beats 8 by 0.1 ms (2^12 points: 0.76 against
-//   0.87 ms per MSM), and 16 is 0.33 ms worse;
-//   2^21 buckets: 16 is best (8 and 16 tie at 2^19);
-//   4.9 M shared buckets (tables of width 23): 64 beats 32 by 0.3 ms (level 1 +0.08 ms, levels 2
-//   and 3 -0.37 ms), and 64 is best at 2^23.
+// latency-bound levels 2 and 3.  Measured on GB300, whole MSMs, runs of 4 / 8 / 16 (us): 2^15 buckets
+// (4096 points on tables of width 16) 240 / 249 / 276, 50000 points 518 / 543 / 610; 2^19 buckets (2^20
+// points) runs of 8 / 16 / 32: 3738 / 3626 / 3688; 4.9 M (2^24 points) 32 / 64 / 128: 44.14 / 44.01 /
+// 44.00 ms.
 uint32_t red_log2_for(uint64_t buckets) {
   int lg = 0;
   while (lg < 63 && (2ull << lg) <= buckets) lg++;  // floor(log2(buckets))
   return lg <= 15 ? 2u : lg <= 18 ? 3u : lg <= 21 ? 4u : 6u;
 }
-
 
 // the scalar field's modulus r, little-endian 64-bit words
 const uint64_t R_WORDS[4] = {0x0a11800000000001ull, 0x59aa76fed0000001ull, 0x60b44d1e5c37b001ull,
@@ -211,9 +208,9 @@ double model_cost_fixed(uint64_t n, uint32_t c, uint32_t sgn) {
 
 // Run length that keeps buckets of mean load `mean` whole but for their Poisson tail: the
 // smallest power of two (32 to 4096) at or above mean + 2 sqrt(mean).  Measured on GB300 with
-// fixed-base tables: mean 26 (2^20 points, c = 20) 64 beats 32 and 128; mean 104 (2^22) 128
-// beats 64 (merges) and 256 (longer runs unbalance the warps) by 1%; means 38 and 151 (2^24,
-// 2^26 at c = 23) tie from 64 and 256 up.
+// fixed-base tables (ms, runs of 32 / 64 / 128 / 256): mean 26 (2^20 points, c = 20) 3.63 / 3.65 / 3.66 / -,
+// mean 52 (2^21) 6.89 / 6.67 / 6.74 / 6.74, mean 104 (2^22) - / 12.89 / 12.79 / 12.81, mean 38 (2^24,
+// c = 23) 45.33 / 44.01 / 44.00 / 44.01.
 uint32_t whole_bucket_run(double mean) {
   uint32_t s = 32;
   while (s < mean + 2.0 * std::sqrt(mean) && s < 4096) s <<= 1;
@@ -243,9 +240,9 @@ uint32_t quad_run(double mean) {
 // few, heavily loaded buckets (a fixed-base table of small width) whole-bucket runs would leave
 // most of the GPU idle.  A pass of at most 2^21 entries does not fill the GPU, and its time is
 // the longest run plus the merge of its split buckets: runs of about 2 sqrt(mean), at least 8,
-// balance the two.  Measured on GB300 (one MSM on width-16 tables, mean bucket load 8: 2^14
-// points): runs of 8 0.72 ms, 4 0.71 ms, 16 0.82 ms; at load 2 (2^12 points) runs of 2 to 32
-// are within 4% of each other, and at load 32 (2^16 points) 16 is best (1.06 ms, 8: 1.08 ms).
+// balance the two.  Measured on GB300 (us, one MSM on width-16 tables, runs of 8 / 16 / 32 / 64 / 128):
+// 66000 points (mean 32) 573 / 571 / 799 / 997 / 998, 131072 838 / 841 / 859 / 1357 / 1766, 262144
+// 1977 / 1362 / 1399 / 1458 / 2482, 10^6 5904 / 5764 / 4420 / 3993 / 4324.
 uint32_t seg_len_for(uint64_t n, uint32_t nb, uint32_t nwin_sharing, uint32_t nwin, uint32_t epp) {
   const double mean = (double)n * nwin_sharing / std::max<uint32_t>(nb, 1);
   const uint32_t s = whole_bucket_run(mean);
@@ -309,11 +306,13 @@ struct Plan {
 };
 
 // Run length of a pass of several MSMs: whole buckets at the largest mean bucket load among them
-// (as seg_len_for does for one MSM), capped so the whole pass makes at least 2^19 runs.  Each MSM's
-// own choice is capped by its own entries and is too short in a shared pass.  Measured on GB300,
-// the uneven 64-MSM mix (1.1e8 entries, 10% of each MSM's scalars one repeated value) over a
-// 2^24-base context: runs of 64 (the largest MSM's own choice) 35.8 ms, 256 34.4 ms, 512 36.0 ms,
-// 1024 42.2 ms; over a 2^20-base context 34.8, 33.8, 36.2 and 41.9 ms.
+// (as seg_len_for does for one MSM), capped so the whole pass makes at least 2^19 runs, and at 256
+// while that leaves no more than 16 runs a bucket: longer runs unbalance the warps of an uneven
+// pass, more are merged a block per bucket.  Each MSM's own choice is capped by its own entries and is
+// too short in a shared pass.  Measured on GB300, the uneven 64-MSM mix (1.1e8 entries, 10% of each
+// MSM's scalars one repeated value) over a 2^20-base context, runs of 64 / 128 / 256 / 512 / 1024:
+// 28.46 / 28.19 / 28.05 / 28.83 / 32.51 ms; 4 x 50000 points, 8 / 16 / 24 / 32 / 64: 1.21 / 1.12 / 1.14 /
+// 1.18 / 1.17; 4 x 200000, 16 / 24 / 32 / 48 / 64: 3.46 / 3.40 / 3.38 / 3.42 / 3.35.
 uint32_t pass_seg_len(const std::vector<JobSpec> &specs) {
   double mean = 0;
   uint64_t entries = 0;
@@ -330,7 +329,9 @@ uint32_t pass_seg_len(const std::vector<JobSpec> &specs) {
   const uint32_t seg = whole_bucket_run(mean);
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 19) <= entries) cap <<= 1;
-  return std::min(seg, cap);
+  uint32_t most = 256;
+  while (most < 4096 && 16.0 * most < mean) most <<= 1;
+  return std::min({seg, cap, most});
 }
 
 // Entries from which a key range is split over several blocks: short parts keep the slices that are

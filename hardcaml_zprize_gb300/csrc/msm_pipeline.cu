@@ -1909,10 +1909,9 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   }
   mark(7);
   // Level 2 in blocks of 256 threads; level 3 (one block per window) in blocks of 128 while
-  // they fit on the SMs in one wave.  Measured on GB300 (ms, 256 against 128 threads): level 3
-  // of one fixed-base MSM of 2^12 / 2^16 / 2^20 / 2^24 points 0.130 / 0.145 / 0.171 / 0.215
-  // against 0.107 / 0.123 / 0.154 / 0.206; level 2, groups of 512 runs at 2^20 / 2^24,
-  // 0.188 / 0.268 against 0.214 / 0.348 (each quad then sums twice as many runs in sequence).
+  // they fit on the SMs in one wave: with one warp per SMSP a quad addition takes 1.9 us, with two 2.8,
+  // but a quad of the smaller block sums twice as many runs in sequence.  Measured on GB300 (us, level 2
+  // with 256 / 128 threads): 2^12 points 63 / 66, 4 x 50000 72 / 74; level 3 with 128 threads 45 and 39.
   if (pb.n_grps > 0) {
     run(k_reduce2<256>, pb.n_grps, 256, 0, pb);
   }
