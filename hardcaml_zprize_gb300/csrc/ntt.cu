@@ -690,6 +690,30 @@ int ntt_evaluate_device(void *context, uint64_t *d_out, const uint64_t *d_in, vo
   return enqueue_ntt(cx, d_out, d_in, stream ? (cudaStream_t)stream : cx->st, false);
 }
 
+// One transform host to host on the context's stream, with its stages timed or not.
+static int evaluate_host(NttCtx *cx, uint64_t *out, const uint64_t *in, bool marks) {
+  // A copy kernel reads the input when the device reaches pageable memory and the buffer is
+  // 16-byte aligned (GB300 at 2^24: 0.67 ms against 0.77 ms for the driver's copy); otherwise the
+  // driver copies it.  The output always goes back through the driver: a kernel writing into
+  // pages the host has not touched yet takes a fault per page (29 ms at 2^24 against 4.9 ms).
+  const bool direct = cx->host_direct && cx->n >= 2 && ((uintptr_t)in & 15) == 0;
+  const uint32_t cblocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)cx->num_sms * 8, cx->n / 512));
+  if (marks) NCK(cudaEventRecord(cx->ev[0], cx->st));
+  if (direct) {
+    k_ntt_copy<<<cblocks, 256, 0, cx->st>>>((const uint4 *)in, (uint4 *)cx->d_in, cx->n / 2);
+    NCK(cudaGetLastError());
+  } else {
+    NCK(cudaMemcpyAsync(cx->d_in, in, cx->n * 8, cudaMemcpyHostToDevice, cx->st));
+  }
+  if (marks) NCK(cudaEventRecord(cx->ev[1], cx->st));
+  if (int rc = enqueue_ntt(cx, cx->d_out, cx->d_in, cx->st, marks)) return rc;
+  if (marks) NCK(cudaEventRecord(cx->ev[3], cx->st));
+  NCK(cudaMemcpyAsync(out, cx->d_out, cx->n * 8, cudaMemcpyDeviceToHost, cx->st));
+  if (marks) NCK(cudaEventRecord(cx->ev[4], cx->st));
+  NCK(cudaStreamSynchronize(cx->st));
+  return 0;
+}
+
 int ntt_evaluate(void *context, uint64_t *out, const uint64_t *in, uint64_t len) {
   g_err = 0;
   auto *cx = (NttCtx *)context;
@@ -698,25 +722,7 @@ int ntt_evaluate(void *context, uint64_t *out, const uint64_t *in, uint64_t len)
     return fail(NTT_ERR_ARG, "ntt_evaluate: %llu values for a transform of %llu points",
                 (unsigned long long)len, (unsigned long long)cx->n);
   NCK(cudaSetDevice(cx->device));
-  // A copy kernel reads the input when the device reaches pageable memory and the buffer is
-  // 16-byte aligned (GB300 at 2^24: 0.67 ms against 0.77 ms for the driver's copy); otherwise the
-  // driver copies it.  The output always goes back through the driver: a kernel writing into
-  // pages the host has not touched yet takes a fault per page (29 ms at 2^24 against 4.9 ms).
-  const bool direct = cx->host_direct && cx->n >= 2 && ((uintptr_t)in & 15) == 0;
-  const uint32_t cblocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)cx->num_sms * 8, cx->n / 512));
-  NCK(cudaEventRecord(cx->ev[0], cx->st));
-  if (direct) {
-    k_ntt_copy<<<cblocks, 256, 0, cx->st>>>((const uint4 *)in, (uint4 *)cx->d_in, cx->n / 2);
-    NCK(cudaGetLastError());
-  } else {
-    NCK(cudaMemcpyAsync(cx->d_in, in, cx->n * 8, cudaMemcpyHostToDevice, cx->st));
-  }
-  NCK(cudaEventRecord(cx->ev[1], cx->st));
-  if (int rc = enqueue_ntt(cx, cx->d_out, cx->d_in, cx->st, true)) return rc;
-  NCK(cudaEventRecord(cx->ev[3], cx->st));
-  NCK(cudaMemcpyAsync(out, cx->d_out, cx->n * 8, cudaMemcpyDeviceToHost, cx->st));
-  NCK(cudaEventRecord(cx->ev[4], cx->st));
-  NCK(cudaStreamSynchronize(cx->st));
+  if (int rc = evaluate_host(cx, out, in, true)) return rc;
   float ms[4] = {0, 0, 0, 0};
   for (int k = 0; k < 4; k++) cudaEventElapsedTime(&ms[k], cx->ev[k], cx->ev[k + 1]);
   for (int k = 0; k < 4; k++) cx->last_ms[k] = ms[k];
@@ -752,6 +758,16 @@ int ntt_evaluate_batch(void *context, uint64_t *out, const uint64_t *in, uint64_
   if (!cx || (count && (!out || !in))) return fail(NTT_ERR_ARG, "ntt_evaluate_batch: null argument");
   if (count == 0) return 0;
   NCK(cudaSetDevice(cx->device));
+  // A few vectors one after another on one stream: the worker thread below and the hand-over between
+  // three streams cost more than the overlap of few or small copies gains.  Measured on GB300 (us per
+  // call, with the worker / so): one vector of 2^12 / 2^16 / 2^20 / 2^22 points 85 / 104 / 193 / 513 and 29 /
+  // 36 / 126 / 426; four of 2^16 168 / 144, of 2^18 232 / 203, of 2^19 299 / 316; three of 2^20 382 / 379, of
+  // 2^21 637 / 681; eight of 2^16 268 / 288.
+  if (count <= (cx->log_n <= 18 ? 4u : cx->log_n <= 20 ? 3u : 1u)) {
+    for (uint64_t i = 0; i < count; i++)
+      if (int rc = evaluate_host(cx, out + i * cx->n, in + i * cx->n, false)) return rc;
+    return 0;
+  }
   if (!cx->d_in2) {  // the second buffer pair and the copy streams, on first use
     NCK(cudaMalloc(&cx->d_in2, cx->n * 8));
     NCK(cudaMalloc(&cx->d_out2, cx->n * 8));

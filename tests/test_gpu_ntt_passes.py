@@ -39,3 +39,22 @@ def test_every_size(engine, ocpu, log_n, inverse):
             assert np.array_equal(src.cpu().numpy().view(np.uint64), want)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("log_n,count", [(0, 1), (1, 4), (12, 1), (12, 4), (12, 5), (18, 4), (19, 3), (19, 4), (21, 1), (21, 2)])
+def test_batch_sizes(engine, ocpu, log_n, count):
+    """Host batches on both sides of the rule that runs a few vectors on one stream, from a buffer on a
+    16-byte boundary (read by the copy kernel) and one 8 bytes off it (copied by the driver)."""
+    from hardcaml_zprize_gb300.ntt import NttContext
+    n = 1 << log_n
+    buf = np.random.default_rng(5 * log_n + count).integers(0, 2**64, count * n + 3, dtype=np.uint64)
+    off = (buf.ctypes.data >> 3) & 1
+    ctx = NttContext(log_n)
+    try:
+        for start in (off, 1 + off):
+            xs = buf[start:start + count * n].reshape(count, n)
+            got = ctx.evaluate_batch(xs)
+            for i in range(count):
+                assert np.array_equal(got[i], ocpu.ntt(xs[i] % np.uint64(P))), (start, i)
+    finally:
+        ctx.close()
