@@ -55,7 +55,8 @@ int ntt_evaluate_batch(void *context, uint64_t *out, const uint64_t *in, uint64_
  * reference (its buffers are the driver's). */
 int ntt_evaluate_device(void *context, uint64_t *d_out, const uint64_t *d_in, void *stream);
 
-/* Device times (ms, CUDA events) of the last ntt_evaluate: host-to-device copy, pass A, pass B,
+/* Device times (ms, CUDA events) of the last ntt_evaluate: host-to-device copy, first pass, the
+ * passes after it (transforms of at most 2^12 points are one launch, timed as the first),
  * device-to-host copy.  Returns the number of values written. */
 int ntt_last_timings(void *context, double *ms, int32_t max_stages);
 
