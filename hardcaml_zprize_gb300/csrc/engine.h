@@ -74,6 +74,7 @@ enum : int {
 #define MSM_MAX_PART_BINS 4096    // key ranges of the partitioned sort
 #define MSM_MAX_PART_SHIFT 14     // log2 of a key range's buckets there, at most
 #define MSM_PLACE_CHUNKS 2048     // chunks of a part of a key range, at most
+#define MSM_PARTITION_SMEM (224 << 10)  // dynamic shared memory of k_partition, at most
 
 // Everything a pass needs on the device; sized by the host (msm_plan_pass).
 struct PassBuffers {

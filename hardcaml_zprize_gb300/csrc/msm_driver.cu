@@ -364,7 +364,7 @@ bool partitioned(const Plan &pl, uint32_t max_epp, bool host_read) {
 uint32_t chunk_points_for(const Plan &pl, uint32_t max_epp) {
   const uint32_t bins = ((pl.n_buckets - 1) >> pl.bin_shift) + 1;
   uint32_t k = pl.n_points >= (1u << 21) ? 2048 : 1024;
-  while (k > 256 && msm_partition_smem(bins, k * max_epp) > (224u << 10)) k -= 256;
+  while (k > 256 && msm_partition_smem(bins, k * max_epp) > MSM_PARTITION_SMEM) k -= 256;
   return k;
 }
 

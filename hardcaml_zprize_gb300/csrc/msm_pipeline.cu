@@ -585,6 +585,8 @@ __global__ void __launch_bounds__(256) k_scatter_staged(PassBuffers pb, uint32_t
 constexpr int kPartThreads = 1024;
 
 constexpr uint32_t kPlaceChunks = MSM_PLACE_CHUNKS;
+constexpr uint32_t kPlaceParts = 128;  // most parts of a key range by its entries: each reads the counts of those before it
+constexpr size_t kPlaceSmemMax = ((1u << MSM_MAX_PART_SHIFT) + 2 * kPlaceChunks + 1) * 4;
 constexpr int kPlaceThreads = 1024;
 constexpr int kPlaceUnroll = 4;
 
@@ -739,7 +741,8 @@ struct PlacePart {
 };
 
 __device__ __forceinline__ uint32_t parts_of(const PassBuffers &pb, uint32_t total) {
-  const uint32_t a = (total + pb.place_part - 1) / pb.place_part, b = (pb.n_chunks + kPlaceChunks - 1) / kPlaceChunks;
+  const uint32_t a = min((total + pb.place_part - 1) / pb.place_part, kPlaceParts);
+  const uint32_t b = (pb.n_chunks + kPlaceChunks - 1) / kPlaceChunks;
   return min(max(max(a, b), 1u), pb.n_chunks);
 }
 
@@ -1830,9 +1833,11 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   const size_t part_smem = msm_partition_smem(pb.n_bins, pb.stage_cap);
   const size_t place_smem = ((1u << pb.bin_shift) + 2 * kPlaceChunks + 1) * 4;
   if (pb.n_points > 0 && pb.bin_total) {
-    if ((e = cudaFuncSetAttribute(k_partition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem)) ||
-        (e = cudaFuncSetAttribute(k_place_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place_smem)) ||
-        (e = cudaFuncSetAttribute(k_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place_smem)))
+    // the limits are the kernels', not the pass's: another thread may be launching them too
+    const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if ((e = cudaFuncSetAttribute(k_partition, limit, MSM_PARTITION_SMEM)) ||
+        (e = cudaFuncSetAttribute(k_place_count, limit, (int)kPlaceSmemMax)) ||
+        (e = cudaFuncSetAttribute(k_place, limit, (int)kPlaceSmemMax)))
       return e;
     const uint64_t per = chunk_ready && nchunks > 0
                              ? msm_upload_chunk_points(pb.n_points, nchunks, pb.chunk_points) : pb.n_points;

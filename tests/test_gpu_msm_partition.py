@@ -82,3 +82,28 @@ def test_partition_by_size(engine, ocpu):
         check(ctx, ocpu, pts, [n, n], [0, 0], engine.generate_scalars(96, 2 * n), mode=1)
     finally:
         ctx.close()
+
+
+def test_partition_two_threads(engine, ocpu, monkeypatch):
+    """Two contexts whose partitions need different amounts of shared memory, from two threads at once."""
+    import threading
+    monkeypatch.setenv("MSM_SORT_PARTITION", "1")
+    n, res = 4000, {}
+    pts, sc = ocpu.gen_bases(97, n), engine.generate_scalars(98, n)
+    want = ocpu.msm(pts, sc)
+    ctxs = [engine.multi_scalar_mult_init(pts) for _ in range(2)]
+
+    def work(j):
+        opts = dict(window_bits=4, fixed_base=2) if j else dict(fixed_base=1)
+        res[j] = all(np.array_equal(ctxs[j].mult(sc, **opts)[0], want) for _ in range(200 if j == 0 else 40))
+
+    try:
+        threads = [threading.Thread(target=work, args=(j,)) for j in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert res == {0: True, 1: True}
+    finally:
+        for c in ctxs:
+            c.close()
