@@ -788,12 +788,19 @@ Cfg resolve_cfg(Ctx *cx, uint64_t n, const msm_options_t *opt, bool shared_pass 
   const int fb = opt ? opt->fixed_base : 0;
   uint32_t use = 0;
   if ((cx->fb_c || cx->fb2_c) && fb != 2) {
-    double best = 1e300;
+    double best = 1e300, best_between = 1e300;
     uint32_t cheapest = 0;
     for (uint32_t which = 1; which <= 2; which++) {
       if (!table_c(which)) continue;
       const double v = model_cost_fixed(n, table_c(which), 1);
-      if (v < best) {
+      // between two sets: alone on few buckets the runs are parts of buckets, too few to fill the GPU
+      // evenly, and are merged (ms on a context of 2^20 bases, width 16 / 20: 262144 points 1.39 / 1.30,
+      // 349525 1.66 / 1.58, 524288 2.45 / 2.08)
+      uint32_t nwin, nb, nbt;
+      layout(table_c(which), 1, nwin, nb, nbt);
+      const double between = !shared_pass && nb < (1u << 17) && n * nwin > 64ull * nb ? 1.2 * v : v;
+      if (between < best_between) {
+        best_between = between;
         best = v;
         cheapest = which;
       }
