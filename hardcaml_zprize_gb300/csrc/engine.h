@@ -45,11 +45,39 @@ struct WinDesc {
   uint32_t w;
   uint32_t bucket_begin;  // global id of this window's bucket index 0 (digit magnitude 1)
   uint32_t nb;            // buckets in this window
-  uint32_t seg_begin;     // first level-1 reduction segment
-  uint32_t nseg;          // level-1 segments in this window
-  uint32_t grp_begin;     // first level-2 group (2^grp_len_log2 segments each)
-  uint32_t ngrp;          // level-2 groups in this window
+  uint32_t seg_begin;     // first level-1 reduction segment (or piece of a line)
+  uint32_t nseg;          // level-1 segments (pieces) in this window
+  uint32_t grp_begin;     // first level-2 group (2^grp_len_log2 segments each; or sum by bit)
+  uint32_t ngrp;          // level-2 groups (sums) in this window
 };
+
+// The reduction of a window by lines and bits (k_lines): its buckets as a matrix of h rows and 2^wl
+// columns, rows and columns summed in pieces of at most 2^line_log2 buckets.
+struct Lines {
+  uint32_t wl, hl, w, h;  // columns w = 2^wl, rows h, hl bits of a row's number (at least 1)
+  uint32_t pr, pc;        // pieces of a row and of a column
+  uint32_t pieces, sums;  // pieces in all, sums by bit
+};
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline Lines lines_of(uint32_t nb, uint32_t line_log2) {
+  auto bits = [](uint32_t x) {
+    uint32_t k = 0;
+    while (x >> k) k++;
+    return k;
+  };
+  Lines l;
+  l.wl = nb > 1 ? (bits(nb - 1) + 1) / 2 : 0;
+  l.w = 1u << l.wl;
+  l.h = (nb + l.w - 1) >> l.wl;
+  l.hl = l.h > 2 ? bits(l.h - 1) : 1;
+  l.pr = (l.w + (1u << line_log2) - 1) >> line_log2;
+  l.pc = (l.h + (1u << line_log2) - 1) >> line_log2;
+  l.pieces = l.h * l.pr + l.w * l.pc;
+  l.sums = l.wl + l.hl;
+  return l;
+}
 
 struct Task {             // a run of sorted entries that one thread accumulates
   uint32_t start;         // first entry in the sorted value array
@@ -104,6 +132,8 @@ struct PassBuffers {
   uint32_t red_len_log2;        // level-1 reduction segment length = 1 << red_len_log2
   uint32_t grp_len_log2;        // level-2 group = 1 << grp_len_log2 level-1 segments
   uint32_t n_grps;              // level-2 groups
+  uint32_t lines;               // 1: reduction by lines and bits (n_segs pieces of lines, n_grps sums)
+  uint32_t line_log2;           // a piece has 2^line_log2 buckets at most
   uint32_t min_grps, max_grps;  // least and most groups of a window
   uint64_t max_entries;         // capacity of vals
   uint32_t max_tasks;           // capacity of tasks / partials

@@ -279,6 +279,16 @@ Cfg heuristic_cfg(uint64_t n) {
 // ---------------------------------------------------------------------------------------------
 // pass plan
 // ---------------------------------------------------------------------------------------------
+// Where the reduction goes by lines and bits (k_lines): up to 2^19 buckets, in windows that are large or few.
+// Beyond, one thread per run is as fast and needs no more additions than products (k_reduce1); many small
+// windows have short lines (four MSMs of 4096 points on plain records, 88 windows of 4096 buckets: 76 + 66 + 10
+// us by runs, 154 + 31 + 35 by lines; one: 31 + 63 + 18 / 51 + 18 + 35).
+bool use_lines(uint64_t buckets, uint64_t windows) {
+  return buckets <= (1u << 16) || (buckets <= (1u << 19) && buckets >= windows << 13);
+}
+// pieces of 128 buckets while whole lines would be too few and long to fill the GPU
+uint32_t line_log2_for(uint64_t buckets) { return buckets <= (1u << 16) ? 7u : 10u; }
+
 struct JobSpec {
   uint64_t n, base_off, scalar_off;
   Cfg cfg;
@@ -295,6 +305,8 @@ struct Plan {
   uint64_t n_points = 0, max_entries = 0;
   uint32_t n_buckets = 0, n_segs = 0, n_grps = 0, max_tasks = 0;
   uint32_t seg_len = 1024, red_log2 = 5, grp_log2 = 9;
+  bool lines = false;  // reduction by lines and bits, in pieces of 2^line_log2 buckets
+  uint32_t line_log2 = 0;
   // sort: chunks of chunk_points points, each with room for the largest window count of the pass, and
   // the key ranges
   uint64_t n_chunks = 0;
@@ -383,6 +395,11 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = fal
       total += s.cfg.fixed ? std::max(nb, nbt) : (uint64_t)(nwin - 1) * nb + nbt;
     }
     pl.red_log2 = red_log2_for(total);
+    uint64_t windows = 0;
+    for (const JobSpec &s : specs)
+      if (s.n) windows += s.cfg.fixed ? 1 : windows_of(s.cfg.c);
+    pl.lines = use_lines(total, windows);
+    pl.line_log2 = line_log2_for(total);
   }
   // Level-2 groups of 128 to 512 level-1 runs, at most about 128 groups while that allows: more blocks
   // than SMs run in several waves, fewer and longer ones leave SMs idle behind longer serial sums.  A
@@ -436,6 +453,11 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = fal
         wd.nseg = (wd.nb + L - 1) / L;
         wd.grp_begin = (uint32_t)grps;
         wd.ngrp = (wd.nseg + (1u << pl.grp_log2) - 1) >> pl.grp_log2;
+        if (pl.lines) {
+          const Lines l = lines_of(wd.nb, pl.line_log2);
+          wd.nseg = l.pieces;
+          wd.ngrp = l.sums;
+        }
         segs += wd.nseg;
         grps += wd.ngrp;
         pl.wins.push_back(wd);
@@ -487,7 +509,7 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = fal
   const uint64_t mt = buckets + pl.max_entries / pl.seg_len + 1;
   if (mt >= (1ull << 31)) return fail(ERR_BUDGET, "too many tasks");
   pl.max_tasks = (uint32_t)mt;
-  snprintf(tmp, sizeof(tmp), "|%u|%u|g%u", pl.seg_len, pl.red_log2, pl.grp_log2);
+  snprintf(tmp, sizeof(tmp), "|%u|%u|g%u", pl.seg_len, pl.lines ? 100u + pl.line_log2 : pl.red_log2, pl.grp_log2);
   pl.key += tmp;
   return 0;
 }
@@ -646,6 +668,8 @@ PassBuffers make_pass_buffers(Ctx *cx, Workspace &ws, const Plan &pl, const void
   pb.seg_len = pl.seg_len;
   pb.seg_shift = seg_shift_of(pl.seg_len);
   pb.red_len_log2 = pl.red_log2;
+  pb.lines = pl.lines;
+  pb.line_log2 = pl.line_log2;
   pb.grp_len_log2 = pl.grp_log2;
   pb.max_entries = pl.max_entries;
   pb.max_tasks = pl.max_tasks;
@@ -2182,7 +2206,6 @@ int msm_field_selftest(int32_t op, const uint32_t *a, const uint32_t *b, uint32_
 #define MSM_NOALLOC_SCRATCH_BYTES (24u << 20)
 #define MSM_NOALLOC_WINDOW_BITS 12u
 #define MSM_NOALLOC_SEG_LEN 256u
-#define MSM_NOALLOC_RED_LOG2 3u
 
 static __device__ __align__(256) uint8_t g_noalloc_scratch[MSM_NOALLOC_SCRATCH_BYTES];
 
@@ -2192,22 +2215,20 @@ std::mutex g_noalloc_mu;
 void *g_noalloc_ptr[256] = {};  // device address of g_noalloc_scratch, per device ordinal
 
 // the descriptors of the single MSM, written on the device so no host staging is needed
-__global__ void k_noalloc_plan(JobDesc jd, uint32_t red_log2, uint32_t grp_log2, JobDesc *jobs, WinDesc *wins) {
+__global__ void k_noalloc_plan(JobDesc jd, uint32_t line_log2, JobDesc *jobs, WinDesc *wins) {
   const uint32_t w = threadIdx.x;
   if (w == 0) jobs[0] = jd;
   if (w >= jd.nred) return;
-  const uint32_t L = 1u << red_log2, G = 1u << grp_log2;
-  const uint32_t nseg_low = (jd.nb + L - 1) / L;
-  const uint32_t ngrp_low = (nseg_low + G - 1) / G;
   WinDesc wd;
   wd.job = 0;
   wd.w = w;
   wd.bucket_begin = jd.bucket_begin + w * jd.nb;
   wd.nb = jd.fixed ? max(jd.nb, jd.nb_top) : (w + 1 == jd.nwin) ? jd.nb_top : jd.nb;
-  wd.seg_begin = w * nseg_low;
-  wd.nseg = (wd.nb + L - 1) / L;
-  wd.grp_begin = w * ngrp_low;
-  wd.ngrp = (wd.nseg + G - 1) / G;
+  const Lines low = lines_of(jd.nb, line_log2), l = lines_of(wd.nb, line_log2);
+  wd.seg_begin = w * low.pieces;
+  wd.nseg = l.pieces;
+  wd.grp_begin = w * low.sums;
+  wd.ngrp = l.sums;
   wins[w] = wd;
 }
 
@@ -2255,7 +2276,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   jd.base_off = base_offset;
   jd.c = MSM_NOALLOC_WINDOW_BITS;
   jd.signed_digits = 1;
-  uint32_t seg_len = MSM_NOALLOC_SEG_LEN, red_log2 = MSM_NOALLOC_RED_LOG2, grp_log2 = 9;
+  uint32_t seg_len = MSM_NOALLOC_SEG_LEN;
   if (cx->fb2_c && cx->fb2_c <= 16) {
     jd.c = cx->fb2_c;
     jd.fixed = 1;
@@ -2272,18 +2293,17 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
       jd.fb_stride = cx->npoints;
       nbk = std::max(jd.nb, jd.nb_top);
       seg_len = quad_run((double)n * jd.nwin / nbk);
-      red_log2 = red_log2_for(nbk);
-      grp_log2 = 7;
-      nsegs = (nbk + (1u << red_log2) - 1) >> red_log2;
-      ngrps = (nsegs + (1u << grp_log2) - 1) >> grp_log2;
     } else {
-      const uint32_t L = 1u << red_log2;
       jd.nred = jd.nwin;
       nbk = (jd.nwin - 1) * jd.nb + jd.nb_top;
-      const uint32_t nseg_low = (jd.nb + L - 1) / L, nseg_top = (jd.nb_top + L - 1) / L;
-      nsegs = (jd.nwin - 1) * nseg_low + nseg_top;
-      ngrps = (jd.nwin - 1) * ((nseg_low + 511) / 512) + (nseg_top + 511) / 512;
     }
+  }
+  // at most 2^16 buckets in either layout: the reduction goes by lines and bits
+  const uint32_t line_log2 = line_log2_for(nbk);
+  if (n) {
+    const Lines low = lines_of(jd.nb, line_log2), top = lines_of(jd.fixed ? nbk : jd.nb_top, line_log2);
+    nsegs = (jd.nred - 1) * low.pieces + top.pieces;
+    ngrps = (jd.nred - 1) * low.sums + top.sums;
   }
   const uint64_t entries = n * entries_per_point(jd.c, 1);
   const uint32_t tasks = (uint32_t)(nbk + entries / seg_len + 1);
@@ -2325,12 +2345,10 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.n_buckets = nbk;
   pb.n_segs = nsegs;
   pb.n_grps = ngrps;
-  pb.min_grps = jd.fixed ? ngrps : 0u;  // windows: both level-3 kernels run
-  pb.max_grps = ngrps;
   pb.seg_len = seg_len;
   pb.seg_shift = seg_shift_of(seg_len);
-  pb.red_len_log2 = red_log2;
-  pb.grp_len_log2 = grp_log2;
+  pb.lines = 1;
+  pb.line_log2 = line_log2;
   pb.max_entries = entries;
   pb.max_tasks = tasks;
   pb.count = (uint32_t *)(s + o_count);
@@ -2350,7 +2368,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.win_sum = (uint4 *)(s + o_win);
   pb.results = (uint64_t *)d_out;
   cudaStream_t st = (cudaStream_t)stream;
-  k_noalloc_plan<<<1, 64, 0, st>>>(jd, red_log2, grp_log2, (JobDesc *)(s + o_jobs), (WinDesc *)(s + o_wins));
+  k_noalloc_plan<<<1, 64, 0, st>>>(jd, line_log2, (JobDesc *)(s + o_jobs), (WinDesc *)(s + o_wins));
   CK(cudaGetLastError());
   CK(msm_launch_pass(pb, cx->num_sms, st, nullptr));
   return 0;

@@ -1625,6 +1625,142 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// 7-8 for few buckets, by lines and bits: bucket b = hi W + lo of a window is in row hi and column lo of a
+// matrix, W = 2^wl, and its weight b + 1 is W hi + (lo + 1), so with R_hi, C_lo the sums of the rows and columns
+//   window sum = W sum_hi hi R_hi + sum_lo (lo + 1) C_lo,
+// where a sum of i X_i is sum_k 2^k (sum of the X_i with bit k of i).  All those are plain sums, a
+// block of 32 quads each (a warp per SMSP, the fastest a quad adds): k_lines the rows and columns, in
+// pieces of 2^line_log2 buckets, k_bits the sums by bit; k_weigh then has one chain of doublings per window.
+// Two additions a bucket, as by runs, in fewer dependent ones.  Measured on GB300 (us, levels 1 + 2 + 3 by
+// runs / so): tables of width 16, 4096 points 33 + 63 + 45 / 43 + 27 + 45, 4 x 50000 99 + 72 + 39 / 116 + 25 + 45;
+// width 20 332 + 92 + 68 / 357 + 53 + 55; pieces of 64 / 128 / 256 / 1024 buckets at 4096 points 45 + 37 / 43 + 27 /
+// 45 + 25 / 45 + 25, at width 20 547 + 338 / 434 + 176 / 375 + 96 / 357 + 53.
+// In this form a window's seg_begin and nseg count its pieces of lines, grp_begin and ngrp its sums.
+// ---------------------------------------------------------------------------------------------
+constexpr uint32_t kLineQuads = 32;
+
+// The sum of n points over the block's quads (valid in quad 0); point(i, live) sets live where there is
+// one, else it returns the identity.  A warp with nothing to add skips the addition.
+template <class F>
+__device__ __forceinline__ fq_t block_line_sum(uint32_t n, uint4 *sh, F point) {
+  __shared__ bool sh_live[kLineQuads];
+  const uint32_t q = threadIdx.x >> 2;
+  const uint32_t warp_q0 = (threadIdx.x >> 5) * 8;
+  bool live = false, next_live = false;
+  fq_t acc = point(q, live), next = point(q + kLineQuads, next_live);
+#pragma unroll 1
+  for (uint32_t i0 = kLineQuads; i0 < n; i0 += kLineQuads) {
+    const fq_t b = next;
+    const bool add = next_live;
+    next_live = false;
+    next = point(i0 + kLineQuads + q, next_live);
+    if (__any_sync(kAllLanes, add)) acc = dq_add(acc, b, kAllLanes);
+    live = live || add;
+  }
+  if (n <= 1) return acc;
+  dq_store(sh + q * 12, acc);
+  if ((threadIdx.x & 3) == 0) sh_live[q] = live;
+  __syncthreads();
+  uint32_t stride = kLineQuads / 2;
+  while (stride >= n) stride >>= 1;  // quads from n on hold the identity
+#pragma unroll 1
+  for (; stride > 0; stride >>= 1) {
+    fq_t o = dq_identity();
+    bool add = false;
+    if (q < stride) {
+      o = dq_load(sh + (q + stride) * 12);
+      add = sh_live[q + stride];
+    }
+    if (warp_q0 < stride && __any_sync(kAllLanes, add)) acc = dq_add(acc, o, kAllLanes);
+    live = live || add;
+    __syncthreads();
+    if (q < stride) {
+      dq_store(sh + q * 12, acc);
+      if ((threadIdx.x & 3) == 0) sh_live[q] = live;
+    }
+    __syncthreads();
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(4 * kLineQuads) k_lines(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  __shared__ uint4 sh[kLineQuads * 12];
+  const WinDesc wd = pb.wins[find_win(pb.wins, pb.n_wins, blockIdx.x)];
+  const Lines l = lines_of(wd.nb, pb.line_log2);
+  uint32_t li = blockIdx.x - wd.seg_begin, b0, step, n;
+  if (li < l.h * l.pr) {
+    const uint32_t i0 = (li % l.pr) << pb.line_log2;
+    b0 = ((li / l.pr) << l.wl) + i0;
+    step = 1;
+    n = min(l.w - i0, 1u << pb.line_log2);
+  } else {
+    li -= l.h * l.pr;
+    const uint32_t i0 = (li % l.pc) << pb.line_log2;
+    b0 = li / l.pc + (i0 << l.wl);
+    step = l.w;
+    n = min(l.h - i0, 1u << pb.line_log2);
+  }
+  const fq_t sum = block_line_sum(n, sh, [&](uint32_t i, bool &live) {
+    const uint32_t b = b0 + i * step, gb = wd.bucket_begin + b;
+    live = i < n && b < wd.nb && pb.count[gb] != 0;
+    return live ? dq_load(pb.partials + (size_t)pb.taskoff[gb] * 12) : dq_identity();
+  });
+  if (threadIdx.x < 4) dq_store(pb.seg_out + (size_t)blockIdx.x * 12, sum);
+}
+
+__global__ void __launch_bounds__(4 * kLineQuads) k_bits(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  __shared__ uint4 sh[kLineQuads * 12];
+  const WinDesc wd = pb.wins[find_win_grp(pb.wins, pb.n_wins, blockIdx.x)];
+  const Lines l = lines_of(wd.nb, pb.line_log2);
+  const uint32_t s = blockIdx.x - wd.grp_begin;
+  const uint4 *rows = pb.seg_out + (size_t)wd.seg_begin * 12, *cols = rows + (size_t)l.h * l.pr * 12;
+  const bool col = s < l.wl;
+  const uint32_t bit = col ? s : s - l.wl, p = col ? l.pc : l.pr;
+  const uint32_t n = (col ? l.w >> 1 : 1u << (l.hl - 1)) * p;
+  const uint32_t more = s == l.wl ? l.pc : 0u;  // lo + 1 = W, the last column, counts as a row of bit 0
+  const fq_t sum = block_line_sum(n + more, sh, [&](uint32_t i, bool &live) {
+    if (i >= n + more) return dq_identity();
+    live = true;
+    if (i >= n) return dq_load(cols + ((size_t)(l.w - 1) * l.pc + (i - n)) * 12);
+    const uint32_t e = i / p, j = ((e >> bit) << (bit + 1)) | (1u << bit) | (e & ((1u << bit) - 1u));
+    if (col) return dq_load(cols + ((size_t)(j - 1) * p + i % p) * 12);
+    return j < l.h ? dq_load(rows + ((size_t)j * p + i % p) * 12) : dq_identity();
+  });
+  if (threadIdx.x < 4) dq_store(pb.grp_out + (size_t)blockIdx.x * 12, sum);
+}
+
+// One warp per window: four quads weigh a quarter of the bits each, then theirs are weighed together.
+__global__ void __launch_bounds__(32) k_weigh(PassBuffers pb) {
+  pdl_begin();
+  if (pb.counters[CNT_ERROR]) return;
+  const WinDesc wd = pb.wins[blockIdx.x];
+  const Lines l = lines_of(wd.nb, pb.line_log2);
+  const uint32_t n = l.wl + l.hl, per = (n + 3) / 4, q = threadIdx.x >> 2;
+  const uint4 *sums = pb.grp_out + (size_t)wd.grp_begin * 12;
+  auto bit_sum = [&](uint32_t k) { return k < per && q * per + k < n ? dq_load(sums + (size_t)(q * per + k) * 12) : dq_identity(); };
+  fq_t v = bit_sum(per - 1);
+#pragma unroll 1
+  for (uint32_t k = per - 1; k-- > 0;) {
+    v = dq_dbl(v, kAllLanes);
+    v = dq_add(v, bit_sum(k), kAllLanes);
+  }
+#pragma unroll 1
+  for (uint32_t d = 1; d <= 2; d++) {  // quad q + d's, 2^(d per) times, to quad q's
+    fq_t o = v;
+#pragma unroll 1
+    for (uint32_t k = 0; k < d * per; k++) o = dq_dbl(o, kAllLanes);
+#pragma unroll
+    for (int j = 0; j < FQ_LIMBS; j++) o.v[j] = __shfl_down_sync(kAllLanes, o.v[j], 4 * d);
+    v = dq_add(v, o, kAllLanes);
+  }
+  if (threadIdx.x < 4) dq_store(pb.win_sum + (size_t)blockIdx.x * 12, v);
+}
+
+// ---------------------------------------------------------------------------------------------
 // 6. buckets spread over several tasks: a quad per bucket of at most kMergeQuadMax runs (the common
 //    case: a few more entries than seg_len), then a block of 64 quads per larger one (a value repeated
 //    across many scalars): each quad sums a strided share of the partials, a tree over the quads in
@@ -1906,7 +2042,9 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   mark(5);
   run(k_merge, num_sms * 2, kRedThreads, 0, pb);
   mark(6);
-  if (pb.n_segs > 0) {
+  if (pb.lines && pb.n_segs > 0) {
+    run(k_lines, pb.n_segs, 4 * kLineQuads, 0, pb);
+  } else if (pb.n_segs > 0) {
     if (pb.n_segs <= kReduceQuadSegs)
       run(k_reduce1_quad, (pb.n_segs + 31) / 32, 128, 0, pb);
     else
@@ -1917,11 +2055,15 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   // they fit on the SMs in one wave: with one warp per SMSP a quad addition takes 1.9 us, with two 2.8,
   // but a quad of the smaller block sums twice as many runs in sequence.  Measured on GB300 (us, level 2
   // with 256 / 128 threads): 2^12 points 63 / 66, 4 x 50000 72 / 74; level 3 with 128 threads 45 and 39.
-  if (pb.n_grps > 0) {
+  if (pb.lines && pb.n_grps > 0) {
+    run(k_bits, pb.n_grps, 4 * kLineQuads, 0, pb);
+  } else if (pb.n_grps > 0) {
     run(k_reduce2<256>, pb.n_grps, 256, 0, pb);
   }
   mark(8);
-  if (pb.n_wins > 0) {
+  if (pb.lines && pb.n_wins > 0) {
+    run(k_weigh, pb.n_wins, 32, 0, pb);
+  } else if (pb.n_wins > 0) {
     if (pb.min_grps <= kRed3SmallMax) run(k_reduce3_small, (pb.n_wins + 31) / 32, 128, 0, pb);
     if (pb.max_grps <= kRed3SmallMax) {
       // no window for k_reduce3
