@@ -13,9 +13,10 @@
 //                  k_accumulate_quad, k_reduce1_quad: four lanes a run, small passes
 //   6. k_merge     buckets split over several runs: sum of their partials (a quad or a block per
 //                  bucket, by the number of runs)
-//   7. k_reduce1   per run of buckets: running sum R and triangle sum A (pippenger.h:25-33),
+//   7-8. few buckets: k_lines, k_bits, k_weigh, by rows, columns and bits of the buckets' numbers; else
+//      k_reduce1   per run of buckets: running sum R and triangle sum A (pippenger.h:25-33),
 //                  by the dedicated addition (8 products; the unified one where it fails)
-//   8. k_reduce2/3 combine runs into groups, groups into window sums (k_reduce3_small: one
+//      k_reduce2/3 combine runs into groups, groups into window sums (k_reduce3_small: one
 //                  quad per window of few groups), by quad additions of two product latencies
 //   9. k_final     per MSM: Horner window combine (pippenger.h:36-45), map back to affine
 //                  Weierstrass, add the bases without a twisted-Edwards image
@@ -1630,30 +1631,31 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
 //   window sum = W sum_hi hi R_hi + sum_lo (lo + 1) C_lo,
 // where a sum of i X_i is sum_k 2^k (sum of the X_i with bit k of i).  All those are plain sums, a
 // block of 32 quads each (a warp per SMSP, the fastest a quad adds): k_lines the rows and columns, in
-// pieces of 2^line_log2 buckets, k_bits the sums by bit; k_weigh then has one chain of doublings per window.
+// pieces of 2^line_log2 buckets, k_bits the sums by bit (64 quads); k_weigh then has one chain of doublings per window.
 // Two additions a bucket, as by runs, in fewer dependent ones.  Measured on GB300 (us, levels 1 + 2 + 3 by
-// runs / so): tables of width 16, 4096 points 33 + 63 + 45 / 43 + 27 + 45, 4 x 50000 99 + 72 + 39 / 116 + 25 + 45;
-// width 20 332 + 92 + 68 / 357 + 53 + 55; pieces of 64 / 128 / 256 / 1024 buckets at 4096 points 45 + 37 / 43 + 27 /
-// 45 + 25 / 45 + 25, at width 20 547 + 338 / 434 + 176 / 375 + 96 / 357 + 53.
+// runs / so): tables of width 16, 4096 points 33 + 63 + 45 / 43 + 25 + 45, 4 x 50000 99 + 72 + 39 / 119 + 23 + 45;
+// width 20 332 + 92 + 68 / 365 + 43 + 55.  Pieces of 64 / 128 / 256 / 1024 buckets, lines + bits: at 4096 points 45 +
+// 37 / 43 + 27 / 45 + 25 / 45 + 25, at width 20 547 + 338 / 434 + 176 / 375 + 96 / 357 + 53.  k_bits with 32 / 64
+// quads at width 20: 53 / 43.
 // In this form a window's seg_begin and nseg count its pieces of lines, grp_begin and ngrp its sums.
 // ---------------------------------------------------------------------------------------------
-constexpr uint32_t kLineQuads = 32;
+constexpr uint32_t kLineQuads = 32, kBitQuads = 64;
 
-// The sum of n points over the block's quads (valid in quad 0); point(i, live) sets live where there is
+// The sum of n points over the block's Q quads (valid in quad 0); point(i, live) sets live where there is
 // one, else it returns the identity.  A warp with nothing to add skips the addition.
-template <class F>
+template <uint32_t Q, class F>
 __device__ __forceinline__ fq_t block_line_sum(uint32_t n, uint4 *sh, F point) {
-  __shared__ bool sh_live[kLineQuads];
+  __shared__ bool sh_live[Q];
   const uint32_t q = threadIdx.x >> 2;
   const uint32_t warp_q0 = (threadIdx.x >> 5) * 8;
   bool live = false, next_live = false;
-  fq_t acc = point(q, live), next = point(q + kLineQuads, next_live);
+  fq_t acc = point(q, live), next = point(q + Q, next_live);
 #pragma unroll 1
-  for (uint32_t i0 = kLineQuads; i0 < n; i0 += kLineQuads) {
+  for (uint32_t i0 = Q; i0 < n; i0 += Q) {
     const fq_t b = next;
     const bool add = next_live;
     next_live = false;
-    next = point(i0 + kLineQuads + q, next_live);
+    next = point(i0 + Q + q, next_live);
     if (__any_sync(kAllLanes, add)) acc = dq_add(acc, b, kAllLanes);
     live = live || add;
   }
@@ -1661,7 +1663,7 @@ __device__ __forceinline__ fq_t block_line_sum(uint32_t n, uint4 *sh, F point) {
   dq_store(sh + q * 12, acc);
   if ((threadIdx.x & 3) == 0) sh_live[q] = live;
   __syncthreads();
-  uint32_t stride = kLineQuads / 2;
+  uint32_t stride = Q / 2;
   while (stride >= n) stride >>= 1;  // quads from n on hold the identity
 #pragma unroll 1
   for (; stride > 0; stride >>= 1) {
@@ -1702,7 +1704,7 @@ __global__ void __launch_bounds__(4 * kLineQuads) k_lines(PassBuffers pb) {
     step = l.w;
     n = min(l.h - i0, 1u << pb.line_log2);
   }
-  const fq_t sum = block_line_sum(n, sh, [&](uint32_t i, bool &live) {
+  const fq_t sum = block_line_sum<kLineQuads>(n, sh, [&](uint32_t i, bool &live) {
     const uint32_t b = b0 + i * step, gb = wd.bucket_begin + b;
     live = i < n && b < wd.nb && pb.count[gb] != 0;
     return live ? dq_load(pb.partials + (size_t)pb.taskoff[gb] * 12) : dq_identity();
@@ -1710,10 +1712,10 @@ __global__ void __launch_bounds__(4 * kLineQuads) k_lines(PassBuffers pb) {
   if (threadIdx.x < 4) dq_store(pb.seg_out + (size_t)blockIdx.x * 12, sum);
 }
 
-__global__ void __launch_bounds__(4 * kLineQuads) k_bits(PassBuffers pb) {
+__global__ void __launch_bounds__(4 * kBitQuads) k_bits(PassBuffers pb) {
   pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
-  __shared__ uint4 sh[kLineQuads * 12];
+  __shared__ uint4 sh[kBitQuads * 12];
   const WinDesc wd = pb.wins[find_win_grp(pb.wins, pb.n_wins, blockIdx.x)];
   const Lines l = lines_of(wd.nb, pb.line_log2);
   const uint32_t s = blockIdx.x - wd.grp_begin;
@@ -1722,7 +1724,7 @@ __global__ void __launch_bounds__(4 * kLineQuads) k_bits(PassBuffers pb) {
   const uint32_t bit = col ? s : s - l.wl, p = col ? l.pc : l.pr;
   const uint32_t n = (col ? l.w >> 1 : 1u << (l.hl - 1)) * p;
   const uint32_t more = s == l.wl ? l.pc : 0u;  // lo + 1 = W, the last column, counts as a row of bit 0
-  const fq_t sum = block_line_sum(n + more, sh, [&](uint32_t i, bool &live) {
+  const fq_t sum = block_line_sum<kBitQuads>(n + more, sh, [&](uint32_t i, bool &live) {
     if (i >= n + more) return dq_identity();
     live = true;
     if (i >= n) return dq_load(cols + ((size_t)(l.w - 1) * l.pc + (i - n)) * 12);
@@ -2056,7 +2058,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   // but a quad of the smaller block sums twice as many runs in sequence.  Measured on GB300 (us, level 2
   // with 256 / 128 threads): 2^12 points 63 / 66, 4 x 50000 72 / 74; level 3 with 128 threads 45 and 39.
   if (pb.lines && pb.n_grps > 0) {
-    run(k_bits, pb.n_grps, 4 * kLineQuads, 0, pb);
+    run(k_bits, pb.n_grps, 4 * kBitQuads, 0, pb);
   } else if (pb.n_grps > 0) {
     run(k_reduce2<256>, pb.n_grps, 256, 0, pb);
   }
