@@ -1631,12 +1631,13 @@ __global__ void __launch_bounds__(NT) k_reduce3(PassBuffers pb) {
 //   window sum = W sum_hi hi R_hi + sum_lo (lo + 1) C_lo,
 // where a sum of i X_i is sum_k 2^k (sum of the X_i with bit k of i).  All those are plain sums, a
 // block of 32 quads each (a warp per SMSP, the fastest a quad adds): k_lines the rows and columns, in
-// pieces of 2^line_log2 buckets, k_bits the sums by bit (64 quads); k_weigh then has one chain of doublings per window.
-// Two additions a bucket, as by runs, in fewer dependent ones.  Measured on GB300 (us, levels 1 + 2 + 3 by
-// runs / so): tables of width 16, 4096 points 33 + 63 + 45 / 43 + 25 + 45, 4 x 50000 99 + 72 + 39 / 119 + 23 + 45;
-// width 20 332 + 92 + 68 / 365 + 43 + 55.  Pieces of 64 / 128 / 256 / 1024 buckets, lines + bits: at 4096 points 45 +
-// 37 / 43 + 27 / 45 + 25 / 45 + 25, at width 20 547 + 338 / 434 + 176 / 375 + 96 / 357 + 53.  k_bits with 32 / 64
-// quads at width 20: 53 / 43.
+// pieces of 2^line_log2 buckets, k_bits the sums by bit (64 quads), each doubled to its weight there, side by
+// side; k_weigh adds a window's up.  Two additions a bucket, as by runs, in fewer dependent ones.  Measured
+// on GB300 (us, levels 1 + 2 + 3 by runs / so): tables of width 16, 4096 points 33 + 63 + 45 / 43 + 49 + 14, 4 x
+// 50000 99 + 72 + 39 / 118 + 51 + 14; width 20 332 + 92 + 68 / 365 + 68 + 16.  With the doublings in one chain in
+// k_weigh 43 + 25 + 45.  Pieces of 64 / 128 / 256 / 1024 buckets, lines + bits without doublings: at 4096 points 45 +
+// 37 / 43 + 27 / 45 + 25 / 45 + 25, at width 20 547 + 338 / 434 + 176 / 375 + 96 / 357 + 53; k_bits with 32 / 64 quads
+// there 53 / 43.
 // In this form a window's seg_begin and nseg count its pieces of lines, grp_begin and ngrp its sums.
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kLineQuads = 32, kBitQuads = 64;
@@ -1732,32 +1733,32 @@ __global__ void __launch_bounds__(4 * kBitQuads) k_bits(PassBuffers pb) {
     if (col) return dq_load(cols + ((size_t)(j - 1) * p + i % p) * 12);
     return j < l.h ? dq_load(rows + ((size_t)j * p + i % p) * 12) : dq_identity();
   });
-  if (threadIdx.x < 4) dq_store(pb.grp_out + (size_t)blockIdx.x * 12, sum);
+  if (threadIdx.x < 4) {  // 2^s times the sum: the blocks' doublings run side by side
+    fq_t v = sum;
+#pragma unroll 1
+    for (uint32_t k = 0; k < s; k++) v = dq_dbl(v, 0xfu);
+    dq_store(pb.grp_out + (size_t)blockIdx.x * 12, v);
+  }
 }
 
-// One warp per window: four quads weigh a quarter of the bits each, then theirs are weighed together.
+// One warp per window: the sum of its weighed sums.
 __global__ void __launch_bounds__(32) k_weigh(PassBuffers pb) {
   pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const WinDesc wd = pb.wins[blockIdx.x];
-  const Lines l = lines_of(wd.nb, pb.line_log2);
-  const uint32_t n = l.wl + l.hl, per = (n + 3) / 4, q = threadIdx.x >> 2;
+  const uint32_t n = wd.ngrp, q = threadIdx.x >> 2;
   const uint4 *sums = pb.grp_out + (size_t)wd.grp_begin * 12;
-  auto bit_sum = [&](uint32_t k) { return k < per && q * per + k < n ? dq_load(sums + (size_t)(q * per + k) * 12) : dq_identity(); };
-  fq_t v = bit_sum(per - 1);
+  fq_t v = q < n ? dq_load(sums + (size_t)q * 12) : dq_identity();
 #pragma unroll 1
-  for (uint32_t k = per - 1; k-- > 0;) {
-    v = dq_dbl(v, kAllLanes);
-    v = dq_add(v, bit_sum(k), kAllLanes);
-  }
+  for (uint32_t k0 = 8; k0 < n; k0 += 8)
+    v = dq_add(v, k0 + q < n ? dq_load(sums + (size_t)(k0 + q) * 12) : dq_identity(), kAllLanes);
 #pragma unroll 1
-  for (uint32_t d = 1; d <= 2; d++) {  // quad q + d's, 2^(d per) times, to quad q's
-    fq_t o = v;
-#pragma unroll 1
-    for (uint32_t k = 0; k < d * per; k++) o = dq_dbl(o, kAllLanes);
+  for (int d = 16; d >= 4; d >>= 1) {
+    fq_t o;
 #pragma unroll
-    for (int j = 0; j < FQ_LIMBS; j++) o.v[j] = __shfl_down_sync(kAllLanes, o.v[j], 4 * d);
-    v = dq_add(v, o, kAllLanes);
+    for (int j = 0; j < FQ_LIMBS; j++) o.v[j] = __shfl_down_sync(kAllLanes, v.v[j], d);
+    // the quads past the end got their own point back: adding it would be a doubling
+    v = dq_add(v, fq_select((int)threadIdx.x + d < 32, o, dq_identity()), kAllLanes);
   }
   if (threadIdx.x < 4) dq_store(pb.win_sum + (size_t)blockIdx.x * 12, v);
 }
