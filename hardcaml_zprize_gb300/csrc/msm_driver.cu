@@ -90,18 +90,21 @@ struct DevBuf {
     p = nullptr;
     bytes = 0;
   }
-  // grow-only; returns true if the address changed
+  // grow-only; moved: set when the old address is no longer valid (also where the new size is refused)
   cudaError_t ensure(size_t want, bool *moved = nullptr) {
     if (want <= bytes && p) return cudaSuccess;
     release();
+    if (moved) *moved = true;
     size_t sz = std::max<size_t>(want, 256);
-    cudaError_t e = cudaMalloc(&p, sz);
+    // MSM_ALLOC_FAIL_MB=<n>: buffers of more than n MB are refused (tests of what follows)
+    const char *most = getenv("MSM_ALLOC_FAIL_MB");
+    cudaError_t e = most && sz > (size_t)atoll(most) << 20 ? cudaErrorMemoryAllocation : cudaMalloc(&p, sz);
     if (e != cudaSuccess) {
       p = nullptr;
+      if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by a later call
       return e;
     }
     bytes = sz;
-    if (moved) *moved = true;
     return cudaSuccess;
   }
   template <class T> T *as() const { return (T *)p; }
@@ -551,39 +554,60 @@ struct Workspace {
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
   }
-  int ensure(const Plan &pl) {
+  // room for a pass of plan `pl`; graphs of buffers that moved go, also when a later buffer does not fit
+  cudaError_t reserve(const Plan &pl) {
     bool moved = false;
-    CK(count.ensure((size_t)pl.n_buckets * 4, &moved));
-    CK(offset.ensure((size_t)pl.n_buckets * 4, &moved));
-    CK(taskoff.ensure((size_t)pl.n_buckets * 4, &moved));
-    CK(heavy.ensure((size_t)pl.n_buckets * 4, &moved));
-    CK(scan_tmp.ensure(msm_scan_tmp_words(pl.n_buckets) * 4, &moved));
-    CK(vals.ensure((size_t)pl.max_entries * 4, &moved));
-    CK(stage.ensure((size_t)pl.n_chunks * pl.stage_cap * (pl.place ? 6 : 8), &moved));
-    if (!pl.place) CK(stage_rank.ensure((size_t)pl.n_chunks * pl.stage_cap * 4, &moved));
-    CK(blk_off.ensure((size_t)pl.n_chunks * (pl.n_bins + 1) * 4, &moved));
-    if (pl.place) CK(part_first.ensure((size_t)pl.place_blocks << (2 + pl.bin_shift), &moved));
-    if (pl.place) CK(bin_total.ensure((size_t)pl.n_bins * 4, &moved));
-    CK(tasks.ensure((size_t)pl.max_tasks * sizeof(Task), &moved));
-    CK(partials.ensure((size_t)pl.max_tasks * MSM_BUCKET_BYTES, &moved));
-    CK(order.ensure((size_t)pl.max_tasks * 4, &moved));
-    CK(len_hist.ensure((size_t)(pl.seg_len + 1) * 8, &moved));
-    CK(counters.ensure(CNT_WORDS * 4, &moved));
-    CK(seg_out.ensure((size_t)pl.n_segs * 2 * MSM_BUCKET_BYTES, &moved));
-    CK(grp_out.ensure((size_t)pl.n_grps * 2 * MSM_BUCKET_BYTES, &moved));
-    CK(win_sum.ensure(pl.wins.size() * MSM_BUCKET_BYTES, &moved));
-    CK(results.ensure(pl.jobs.size() * MSM_PROJ_BYTES, &moved));
-    CK(jobs.ensure(pl.jobs.size() * sizeof(JobDesc), &moved));
-    CK(wins.ensure(pl.wins.size() * sizeof(WinDesc), &moved));
-    CK(res_host.ensure(pl.jobs.size() * MSM_PROJ_BYTES));
+    const cudaError_t e = grow(pl, moved);
+    if (moved) drop_graphs();
+    return e;
+  }
+  int ensure(const Plan &pl) {
+    CK(reserve(pl));
     if (!ev[0])
       for (auto &e : ev) CK(cudaEventCreate(&e));
-    if (moved) {
-      generation++;
-      for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.exec);
-      graphs.clear();
-    }
     return 0;
+  }
+  // gives the pass buffers back (nothing may be in flight on them)
+  void release() {
+    for (DevBuf *b : {&count, &offset, &taskoff, &heavy, &scan_tmp, &vals, &stage, &stage_rank, &blk_off,
+                      &part_first, &bin_total, &tasks, &partials, &order, &len_hist, &counters, &seg_out,
+                      &grp_out, &win_sum, &results, &jobs, &wins, &scalars[0], &scalars[1]})
+      b->release();
+    drop_graphs();
+  }
+
+ private:
+  void drop_graphs() {
+    generation++;
+    for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.exec);
+    graphs.clear();
+  }
+  cudaError_t grow(const Plan &pl, bool &moved) {
+    cudaError_t e;
+    if ((e = count.ensure((size_t)pl.n_buckets * 4, &moved))) return e;
+    if ((e = offset.ensure((size_t)pl.n_buckets * 4, &moved))) return e;
+    if ((e = taskoff.ensure((size_t)pl.n_buckets * 4, &moved))) return e;
+    if ((e = heavy.ensure((size_t)pl.n_buckets * 4, &moved))) return e;
+    if ((e = scan_tmp.ensure(msm_scan_tmp_words(pl.n_buckets) * 4, &moved))) return e;
+    if ((e = vals.ensure((size_t)pl.max_entries * 4, &moved))) return e;
+    if ((e = stage.ensure((size_t)pl.n_chunks * pl.stage_cap * (pl.place ? 6 : 8), &moved))) return e;
+    if (!pl.place && (e = stage_rank.ensure((size_t)pl.n_chunks * pl.stage_cap * 4, &moved))) return e;
+    if ((e = blk_off.ensure((size_t)pl.n_chunks * (pl.n_bins + 1) * 4, &moved))) return e;
+    if (pl.place && (e = part_first.ensure((size_t)pl.place_blocks << (2 + pl.bin_shift), &moved))) return e;
+    if (pl.place && (e = bin_total.ensure((size_t)pl.n_bins * 4, &moved))) return e;
+    if ((e = tasks.ensure((size_t)pl.max_tasks * sizeof(Task), &moved))) return e;
+    if ((e = partials.ensure((size_t)pl.max_tasks * MSM_BUCKET_BYTES, &moved))) return e;
+    if ((e = order.ensure((size_t)pl.max_tasks * 4, &moved))) return e;
+    if ((e = len_hist.ensure((size_t)(pl.seg_len + 1) * 8, &moved))) return e;
+    if ((e = counters.ensure(CNT_WORDS * 4, &moved))) return e;
+    if ((e = seg_out.ensure((size_t)pl.n_segs * 2 * MSM_BUCKET_BYTES, &moved))) return e;
+    if ((e = grp_out.ensure((size_t)pl.n_grps * 2 * MSM_BUCKET_BYTES, &moved))) return e;
+    if ((e = win_sum.ensure(pl.wins.size() * MSM_BUCKET_BYTES, &moved))) return e;
+    if ((e = results.ensure(pl.jobs.size() * MSM_PROJ_BYTES, &moved))) return e;
+    if ((e = jobs.ensure(pl.jobs.size() * sizeof(JobDesc), &moved))) return e;
+    if ((e = wins.ensure(pl.wins.size() * sizeof(WinDesc), &moved))) return e;
+    if ((e = res_host.ensure(pl.jobs.size() * MSM_PROJ_BYTES))) return e;
+    return cudaSuccess;
   }
 };
 
@@ -868,10 +892,11 @@ bool host_pullable(const Ctx *cx, const void *h) {
 }
 
 // Run MSMs whose bases are known to be resident.  mode 1: one pass per MSM with the next MSM's scalars
-// copied during the current pass; mode 2: all MSMs in one pass with one shared sort.
+// copied during the current pass; mode 2: all MSMs in one pass with one shared sort.  no_room (mode 2): set
+// when the pass does not fit the limits of a pass or the free device memory; nothing has been launched then.
 int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
                 const std::vector<uint64_t> &offs, const biginteger256_t *h_scalars,
-                const void *d_scalars, const msm_options_t *opt, int mode) {
+                const void *d_scalars, const msm_options_t *opt, int mode, bool *no_room = nullptr) {
   const size_t m = sizes.size();
   if (m == 0) return 0;
   const bool use_graph = !(opt && opt->use_graph == 2) && !cx->timing;
@@ -883,10 +908,11 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
     std::vector<JobSpec> specs(m);
     uint64_t maxn = 0;
     for (size_t j = 0; j < m; j++) maxn = std::max(maxn, sizes[j]);
+    const Cfg largest = resolve_cfg(cx, maxn, opt, m > 1);
     for (size_t j = 0; j < m; j++) {
       specs[j] = {sizes[j], offs[j], first[j], resolve_cfg(cx, sizes[j], opt, m > 1)};
-      specs[j].cfg.seg_len = resolve_cfg(cx, maxn, opt, m > 1).seg_len;
-      specs[j].cfg.red_log2 = resolve_cfg(cx, maxn, opt, m > 1).red_log2;
+      specs[j].cfg.seg_len = largest.seg_len;
+      specs[j].cfg.red_log2 = largest.red_log2;
       set_tables(cx, specs[j]);
     }
     if (m > 1 && !(opt && opt->seg_len > 0)) {
@@ -895,10 +921,16 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
     }
     Plan pl;
     const bool pulls = !d_scalars && host_pullable(cx, h_scalars);
-    if (build_plan(specs, pl, pulls)) return g_err;
+    if (build_plan(specs, pl, pulls)) {
+      if (no_room) *no_room = g_err == ERR_BUDGET;
+      return g_err;
+    }
+    cudaError_t room = ws.reserve(pl);
+    if (!room && !d_scalars) room = ws.scalars[0].ensure(first[m] * 32);
+    if (no_room) *no_room = room == cudaErrorMemoryAllocation;
+    CK(room);
     const void *src = d_scalars, *pull = nullptr;
     if (!src) {
-      CK(ws.scalars[0].ensure(first[m] * 32));
       if (pulls) {
         pull = h_scalars;
       } else if (first[m]) {
@@ -979,16 +1011,32 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
   return 0;
 }
 
-// Points of one shared pass when the caller leaves the mode open.  A pass ends in serial reductions
-// and a final map (0.2 ms) and a small one leaves the GPU idle; together the MSMs share both.  Measured
-// on GB300 (host scalars, one pass per MSM / shared, ms): 4 x 4096 1.19 / 0.49, 4 x 50000 2.37 / 1.53,
-// 4 x 2^18 6.33 / 4.87, 4 x 2^20 15.75 / 14.46, 2 x 2^21 14.72 / 14.08.  Larger groups gain less and
-// their sort and partial sums take more memory (about 1.5 GB at this limit).
+// Points and workspace of one shared pass when the caller leaves the mode open.  A pass ends in serial
+// reductions and a final map (0.1 to 0.2 ms) and a small one leaves the GPU idle; together the MSMs share
+// both.  Measured on GB300 (host scalars, one pass per MSM / shared, ms): 4 x 4096 0.95 / 0.36, 4 x 50000
+// 2.00 / 1.09, 4 x 2^18 5.49 / 4.33, 4 x 2^20 14.71 / 14.22, 2 x 2^21 14.02 / 13.79.  Larger groups gain less.
+// The points bound a pass's sort; every MSM also brings its buckets, 2^15 however few its points on tables
+// of width 16, and those are bounded by the bytes (2 GB hold 250 such MSMs; us per MSM of 1000 points
+// alone / 64 / 256 / 1024 / 4096 in a pass: 170 / 31 / 26 / 23 / 22, the last with 32 GB).
 constexpr uint64_t kSharePoints = 1ull << 22;
+constexpr uint64_t kShareBytes = 2ull << 30;
+
+// About what an MSM adds to a shared pass's workspace (see plan_bytes).
+uint64_t share_bytes(const Cfg &cfg, uint64_t n, const msm_options_t *opt) {
+  constexpr uint64_t task = sizeof(Task) + 4 + MSM_BUCKET_BYTES;
+  uint64_t bytes = 1024;
+  if (n == 0) return bytes;
+  uint32_t nwin, nb, nbt;
+  layout(cfg.c, cfg.signed_digits, nwin, nb, nbt);
+  const uint64_t buckets = cfg.fixed ? std::max(nb, nbt) : (uint64_t)(nwin - 1) * nb + nbt;
+  const uint64_t run = opt && opt->seg_len > 0 ? opt->seg_len : 32;
+  bytes += buckets * (16 + task) + (cfg.fixed ? 1 : nwin) * 8192ull;
+  return bytes + n * (32 + entries_per_point(cfg.c, cfg.signed_digits) * (16 + task / run));
+}
 
 // Run a list of MSMs whose scalars are in host memory (d_scalars == nullptr) or already on the
 // device, in the mode the options ask for, or else with consecutive MSMs of at most kSharePoints
-// points together in one pass.
+// points and kShareBytes of workspace together in one pass (less where that much memory is not free).
 int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
              const std::vector<uint64_t> &offs, const biginteger256_t *h_scalars,
              const void *d_scalars, const msm_options_t *opt) {
@@ -1000,20 +1048,42 @@ int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
                   (unsigned long long)cx->npoints);
   if (m <= 1 || (opt && opt->mode > 0))
     return run_msms_as(cx, out, sizes, offs, h_scalars, d_scalars, opt, opt && opt->mode == 2 ? 2 : 1);
-  // the next group: MSMs that share a pass, or a run of MSMs that each need one of their own
-  uint64_t first = 0;
-  for (size_t a = 0; a < m;) {
-    uint64_t points = sizes[a];
+  std::vector<uint64_t> bytes(m);
+  for (size_t j = 0; j < m; j++)
+    bytes[j] = j && sizes[j] == sizes[j - 1] ? bytes[j - 1]
+                                             : share_bytes(resolve_cfg(cx, sizes[j], opt, true), sizes[j], opt);
+  uint64_t first = 0, room = kShareBytes;
+  // the end of the group that starts with MSM a
+  auto group_end = [&](size_t a) {
+    uint64_t points = sizes[a], need = bytes[a];
     size_t b = a + 1;
-    while (b < m && points + sizes[b] <= kSharePoints) points += sizes[b++];
+    while (b < m && points + sizes[b] <= kSharePoints && need + bytes[b] <= room) {
+      points += sizes[b];
+      need += bytes[b++];
+    }
+    return b;
+  };
+  // the next group: MSMs that share a pass, or a run of MSMs that each need one of their own
+  for (size_t a = 0; a < m;) {
+    size_t b = group_end(a);
     const int mode = b > a + 1 ? 2 : 1;
     if (mode == 1)
-      while (b < m && (b + 1 == m || sizes[b] + sizes[b + 1] > kSharePoints)) points += sizes[b++];
+      while (b < m && group_end(b) == b + 1) b++;
     const std::vector<uint64_t> sz(sizes.begin() + a, sizes.begin() + b), of(offs.begin() + a, offs.begin() + b);
+    bool no_room = false;
     if (int rc = run_msms_as(cx, out + a, sz, of, h_scalars ? h_scalars + first : nullptr,
-                             d_scalars ? (const char *)d_scalars + first * 32 : nullptr, opt, mode))
-      return rc;
-    first += points;
+                             d_scalars ? (const char *)d_scalars + first * 32 : nullptr, opt, mode,
+                             mode == 2 ? &no_room : nullptr)) {
+      if (!no_room) return rc;
+      // smaller groups, down to single MSMs; what this one took of the memory first goes back
+      CK(cudaStreamSynchronize(cx->stream));
+      cx->ws.release();
+      cudaGetLastError();
+      g_err = 0;
+      room /= 2;
+      continue;
+    }
+    for (size_t j = a; j < b; j++) first += sizes[j];
     a = b;
   }
   return 0;
