@@ -1020,6 +1020,12 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
 // alone / 64 / 256 / 1024 / 4096 in a pass: 170 / 31 / 26 / 23 / 22, the last with 32 GB).
 constexpr uint64_t kSharePoints = 1ull << 22;
 constexpr uint64_t kShareBytes = 2ull << 30;
+// Scalars that the histogram kernel cannot read from host memory are copied whole before a shared pass
+// starts, while passes of their own hide all but the first MSM's copy: MSMs of more points than this keep
+// to themselves then (ms, one pass each / shared: 4 x 2^18 5.52 / 4.42, 4 x 2^20 14.70 / 14.53, 16 x 2^20
+// 58.0 / 58.1, 2 x 2^21 13.79 / 13.91, 3 x 2^21 20.50 / 21.02; the shared copy in four pieces beside their
+// histograms costs 0.07 to 0.1 ms more at each of these).
+constexpr uint64_t kShareCopiedPoints = 1ull << 20;
 
 // About what an MSM adds to a shared pass's workspace (see plan_bytes).
 uint64_t share_bytes(const Cfg &cfg, uint64_t n, const msm_options_t *opt) {
@@ -1052,12 +1058,13 @@ int run_msms(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &sizes,
   for (size_t j = 0; j < m; j++)
     bytes[j] = j && sizes[j] == sizes[j - 1] ? bytes[j - 1]
                                              : share_bytes(resolve_cfg(cx, sizes[j], opt, true), sizes[j], opt);
+  const uint64_t most = d_scalars || host_pullable(cx, h_scalars) ? kSharePoints : kShareCopiedPoints;
   uint64_t first = 0, room = kShareBytes;
   // the end of the group that starts with MSM a
   auto group_end = [&](size_t a) {
     uint64_t points = sizes[a], need = bytes[a];
     size_t b = a + 1;
-    while (b < m && points + sizes[b] <= kSharePoints && need + bytes[b] <= room) {
+    while (b < m && std::max(sizes[a], sizes[b]) <= most && points + sizes[b] <= kSharePoints && need + bytes[b] <= room) {
       points += sizes[b];
       need += bytes[b++];
     }

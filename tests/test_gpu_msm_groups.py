@@ -83,3 +83,23 @@ def test_no_room(engine, ocpu, monkeypatch, mb):
         assert np.array_equal(ctx.mult_device(sizes, offs, d_sc.data_ptr(), mode=2), out)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("pull", ["0", "1"])
+def test_large_and_small_msms_from_host(engine, ocpu, monkeypatch, pull):
+    """Around the size up to which scalars that are copied first share a pass, both ways of uploading."""
+    big = (1 << 20) + 1
+    pts = np.concatenate([engine.generate_bases(408, 1 << 12)] * 257)[:big]
+    sizes = [7, big, 1 << 20, 5, 0, big, big, 100]
+    offs = [3, 0, 1, 0, 0, 0, 0, 50]
+    sc = np.concatenate([engine.generate_scalars(409, 1 << 16)] * 65)[:sum(sizes)]
+    monkeypatch.setenv("MSM_HOST_PULL", pull)
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        out = ctx.mult_uneven(sizes, offs, sc)
+        assert np.array_equal(ctx.mult_uneven(sizes, offs, sc, mode=1), out)
+    finally:
+        ctx.close()
+    first = np.concatenate([[0], np.cumsum(sizes)])
+    for j in (0, 3, 4, 7):
+        assert np.array_equal(out[j], ocpu.msm(pts[offs[j]:offs[j] + sizes[j]], sc[first[j]:first[j + 1]])), j
