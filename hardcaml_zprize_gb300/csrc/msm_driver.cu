@@ -227,14 +227,17 @@ constexpr uint64_t kQuadEntries = 7ull << 17;
 
 // Run length of such a pass: a run costs a quad two product latencies per entry, a split bucket a
 // merge kernel's passes over its parts, so buckets stay whole but for the upper tail: the smallest
-// power of two (at least 8) at or above 1.3 mean loads.  Measured on GB300 (ms per MSM on width-16
-// tables, runs of 8 / 16 / 32 / 64): 10000 points (mean 4.9) 0.407 / 0.416 / 0.421 / 0.422; 16384 (8)
-// 0.470 / 0.443 / 0.458 / 0.457; 25000 (12.2) 0.566 / 0.506 / 0.522 / 0.543; 50000 (24.4) 0.731 /
-// 0.704 / 0.665 / 0.681.  One thread per run at its best run length: 0.474, 0.524, 0.602, 0.738; at
-// 75000 points (1.2e6 entries) 0.838 against 0.816, at 2^17 1.113 against 1.154.
-uint32_t quad_run(double mean) {
+// power of two (at least 8) at or above 1.3 mean loads.  Measured on GB300 (us per MSM on width-16 tables,
+// runs of 4 / 8 / 16 / 32 / 64): 8000 points (mean 3.9) 225 / 222 / 236 / 234 / 234; 20011 (9.8) 321 / 298 /
+// 298 / 310 / 309; 39000 (19) 459 / 420 / 409 / 423 / 444; 53000 (26) 557 / 509 / 486 / 497 / 519.
+// The GPU holds 19456 quads: runs are shorter where there would be fewer than about 14000 of them, and 64 at
+// most (few, heavily loaded buckets, of narrow tables or windows).  us, runs of 16 / 32 / 64 / 128 / 256 /
+// whole buckets: 20011 points on tables of width 11 449 / 462 / 423 / 560 / 856 / 1497, on width 12 422 / 411 /
+// 408 / 544 / 828 / 1462, 39000 on width 12 717 / 573 / 625 / 676 / 1015 / 2951; 8192 in windows of 4 bits 1084 /
+// 1107 / 1091 / 1227 / 1450 / 5510, of 6 959 / 935 / 968 / 1068 / 1368 / 1939.
+uint32_t quad_run(double mean, uint64_t entries) {
   uint32_t s = 8;
-  while (s < 1.3 * mean && s < 4096) s <<= 1;
+  while (s < 64 && s < 1.3 * mean && entries > 14000ull * s) s <<= 1;
   return s;
 }
 
@@ -249,7 +252,8 @@ uint32_t quad_run(double mean) {
 uint32_t seg_len_for(uint64_t n, uint32_t nb, uint32_t nwin_sharing, uint32_t nwin, uint32_t epp) {
   const double mean = (double)n * nwin_sharing / std::max<uint32_t>(nb, 1);
   const uint32_t s = whole_bucket_run(mean);
-  if (n * (uint64_t)epp <= kQuadEntries) return quad_run(mean);  // as the plan counts entries
+  const uint64_t most = n * (uint64_t)epp;  // as the plan counts entries
+  if (most <= kQuadEntries) return quad_run(mean, most);
   const uint64_t entries = n * (uint64_t)nwin;
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 18) <= entries) cap <<= 1;  // entries / cap >= 2^17
@@ -340,7 +344,7 @@ uint32_t pass_seg_len(const std::vector<JobSpec> &specs) {
     mean = std::max(mean, load);
     entries += sp.n * entries_per_point(sp.cfg.c, sp.cfg.signed_digits);
   }
-  if (entries <= kQuadEntries) return quad_run(mean);
+  if (entries <= kQuadEntries) return quad_run(mean, entries);
   const uint32_t seg = whole_bucket_run(mean);
   uint32_t cap = 16;
   while (cap < 4096 && ((uint64_t)cap << 19) <= entries) cap <<= 1;
@@ -2347,7 +2351,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   // most 2^15 buckets, no serial window combine) where it has such a set, or else signed windows of
   // 12 bits over the plain records (22 windows of 2048 buckets, 2 in the top one).  Both fit the
   // scratch array for any n up to the limit.  Measured on GB300, 20011 points: tables of width 16
-  // 421 us, windows 1684 us (of which 650 the window combine).
+  // 277 us, windows 1409 us (of which 500 the window combine).
   JobDesc jd{};
   jd.n = n;
   jd.base_off = base_offset;
@@ -2369,7 +2373,7 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
       jd.nred = 1;
       jd.fb_stride = cx->npoints;
       nbk = std::max(jd.nb, jd.nb_top);
-      seg_len = quad_run((double)n * jd.nwin / nbk);
+      seg_len = quad_run((double)n * jd.nwin / nbk, n * entries_per_point(jd.c, 1));
     } else {
       jd.nred = jd.nwin;
       nbk = (jd.nwin - 1) * jd.nb + jd.nb_top;
@@ -2412,7 +2416,10 @@ extern "C" int msm_mult_noalloc(void *context, g1_projective_t *d_out, uint64_t 
   pb.n_special = cx->n_special;
   pb.n_classes = cx->n_classes;
   pb.n_bases = cx->npoints * (cx->fb_w + cx->fb2_w);
-  pb.quads = jd.fixed || entries <= kQuadEntries;  // fixed: at most 1.1e6, with quad_run's run length
+  // On tables quads throughout, up to 1.6e6 entries (65536 points on width 11): the runs of 16 that threads
+  // want there don't fit the scratch array.  us, quads at runs of 64 / threads at 32 (the shortest that fit),
+  // 65536 points: width 11 982 / 1060, 13 683 / 859, 16 559 / 742.
+  pb.quads = jd.fixed || entries <= kQuadEntries;
   pb.scalars = (const uint4 *)d_scalars;
   pb.jobs = (const JobDesc *)(s + o_jobs);
   pb.wins = (const WinDesc *)(s + o_wins);

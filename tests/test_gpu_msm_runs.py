@@ -1,0 +1,23 @@
+"""The runs that a pass of few entries is split into: enough of them where a few buckets hold most of the
+entries (narrow tables, narrow windows), against the CPU oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("table,bits,n", [(11, 0, 20011), (12, 0, 39000), (13, 0, 9001), (0, 4, 8192), (0, 6, 13001)])
+def test_runs_of_few_buckets(engine, ocpu, monkeypatch, table, bits, n, kind):
+    pts = ocpu.gen_bases(500 + table + bits, n)
+    sc = engine.generate_scalars(501, n, kind=kind, msm_index=2)
+    monkeypatch.setenv("MSM_FIXED_BASE", str(table))
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        opts = dict(fixed_base=1) if table else dict(fixed_base=2, window_bits=bits)
+        assert np.array_equal(ctx.mult(sc, **opts)[0], ocpu.msm(pts, sc))
+        st = ctx.last_pass_stats()
+    finally:
+        ctx.close()
+    assert st["entries"] <= 7 << 17  # four lanes a run
+    assert st["tasks"] >= min(st["entries"] // 64, 7000)
