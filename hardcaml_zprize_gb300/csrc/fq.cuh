@@ -122,7 +122,8 @@ struct fq_lanes {  // six 64-bit lanes
   uint32_t w[FQ_LIMBS];
 };
 
-// x += sum over k of a[k] b at lane k, carry out added to top
+// x += sum over k of a[k] b at lane k, carry out added to top.  In these four every output is written before
+// the last input is read: all are early clobbers.
 __device__ __forceinline__ void fq_chain(fq_lanes &x, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t a4, uint32_t a5, uint32_t b, uint32_t &top) {
   asm("mad.lo.cc.u32 %0, %13, %19, %0;\n\tmadc.hi.cc.u32 %1, %13, %19, %1;\n\t"
@@ -132,8 +133,8 @@ __device__ __forceinline__ void fq_chain(fq_lanes &x, uint32_t a0, uint32_t a1, 
       "madc.lo.cc.u32 %8, %17, %19, %8;\n\tmadc.hi.cc.u32 %9, %17, %19, %9;\n\t"
       "madc.lo.cc.u32 %10, %18, %19, %10;\n\tmadc.hi.cc.u32 %11, %18, %19, %11;\n\t"
       "addc.u32 %12, %12, 0;"
-      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
-        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11]), "+r"(top)
+      : "+&r"(x.w[0]), "+&r"(x.w[1]), "+&r"(x.w[2]), "+&r"(x.w[3]), "+&r"(x.w[4]), "+&r"(x.w[5]), "+&r"(x.w[6]),
+        "+&r"(x.w[7]), "+&r"(x.w[8]), "+&r"(x.w[9]), "+&r"(x.w[10]), "+&r"(x.w[11]), "+&r"(top)
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b));
 }
 // the same without a carry out
@@ -145,8 +146,8 @@ __device__ __forceinline__ void fq_chain_end(fq_lanes &x, uint32_t a0, uint32_t 
       "madc.lo.cc.u32 %6, %15, %18, %6;\n\tmadc.hi.cc.u32 %7, %15, %18, %7;\n\t"
       "madc.lo.cc.u32 %8, %16, %18, %8;\n\tmadc.hi.cc.u32 %9, %16, %18, %9;\n\t"
       "madc.lo.cc.u32 %10, %17, %18, %10;\n\tmadc.hi.u32 %11, %17, %18, %11;"
-      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
-        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11])
+      : "+&r"(x.w[0]), "+&r"(x.w[1]), "+&r"(x.w[2]), "+&r"(x.w[3]), "+&r"(x.w[4]), "+&r"(x.w[5]), "+&r"(x.w[6]),
+        "+&r"(x.w[7]), "+&r"(x.w[8]), "+&r"(x.w[9]), "+&r"(x.w[10]), "+&r"(x.w[11])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b));
 }
 // e0 += s, then lanes 0 to 4 of x and a new lane 5 (from zero) take the products, the sum's carry first
@@ -159,8 +160,8 @@ __device__ __forceinline__ void fq_chain_shifted(fq_lanes &x, uint32_t &e0, uint
       "madc.lo.cc.u32 %6, %16, %19, %6;\n\tmadc.hi.cc.u32 %7, %16, %19, %7;\n\t"
       "madc.lo.cc.u32 %8, %17, %19, %8;\n\tmadc.hi.cc.u32 %9, %17, %19, %9;\n\t"
       "madc.lo.cc.u32 %10, %18, %19, 0;\n\tmadc.hi.u32 %11, %18, %19, 0;"
-      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
-        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "=r"(x.w[10]), "=r"(x.w[11]), "+r"(e0)
+      : "+&r"(x.w[0]), "+&r"(x.w[1]), "+&r"(x.w[2]), "+&r"(x.w[3]), "+&r"(x.w[4]), "+&r"(x.w[5]), "+&r"(x.w[6]),
+        "+&r"(x.w[7]), "+&r"(x.w[8]), "+&r"(x.w[9]), "=&r"(x.w[10]), "=&r"(x.w[11]), "+&r"(e0)
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(b), "r"(s));
 }
 // x += m (1 + sum over k >= 1 of a[k] 2^64k), word 0 becomes zero (m = -x.w[0]), carry out added to top
@@ -173,8 +174,8 @@ __device__ __forceinline__ void fq_chain_reduce(fq_lanes &x, uint32_t a1, uint32
       "madc.lo.cc.u32 %8, %16, %18, %8;\n\tmadc.hi.cc.u32 %9, %16, %18, %9;\n\t"
       "madc.lo.cc.u32 %10, %17, %18, %10;\n\tmadc.hi.cc.u32 %11, %17, %18, %11;\n\t"
       "addc.u32 %12, %12, 0;\n\t}"
-      : "+r"(x.w[0]), "+r"(x.w[1]), "+r"(x.w[2]), "+r"(x.w[3]), "+r"(x.w[4]), "+r"(x.w[5]), "+r"(x.w[6]),
-        "+r"(x.w[7]), "+r"(x.w[8]), "+r"(x.w[9]), "+r"(x.w[10]), "+r"(x.w[11]), "+r"(top)
+      : "+&r"(x.w[0]), "+&r"(x.w[1]), "+&r"(x.w[2]), "+&r"(x.w[3]), "+&r"(x.w[4]), "+&r"(x.w[5]), "+&r"(x.w[6]),
+        "+&r"(x.w[7]), "+&r"(x.w[8]), "+&r"(x.w[9]), "+&r"(x.w[10]), "+&r"(x.w[11]), "+&r"(top)
       : "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5), "r"(m));
 }
 // -x, kept apart from the products that use it (see above)
