@@ -257,6 +257,19 @@ __global__ void k_field_test(int op, const uint32_t *a, const uint32_t *b, uint3
   for (int k = 0; k < FQ_LIMBS; k++) out[i * FQ_LIMBS + k] = r.v[k];
 }
 
+// the inversion of a whole warp, element by element
+__global__ void __launch_bounds__(128) k_field_test_warp(const uint32_t *a, uint32_t *out, size_t n) {
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
+  fq_t x;
+#pragma unroll
+  for (int k = 0; k < FQ_LIMBS; k++) x.v[k] = a[i * FQ_LIMBS + k];
+  const fq_t r = fq_inv_warp(x);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < FQ_LIMBS; k++) out[i * FQ_LIMBS + k] = r.v[k];
+}
+
 // Peak IMAD rates: 8 independent chains per thread of mad.lo/mad.hi pairs (mode 0), mad.lo only
 // (mode 1) or mad.hi only (mode 2); 16 IMAD per chain step.
 template <int MODE>
@@ -344,7 +357,8 @@ cudaError_t msm_launch_gen_bases(uint64_t seed, uint64_t first, size_t n, void *
 cudaError_t msm_launch_field_test(int op, const uint32_t *a, const uint32_t *b, uint32_t *out,
                                   size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_field_test<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(op, a, b, out, n);
+  if (op == 7) k_field_test_warp<<<(unsigned)((n + 3) / 4), 128, 0, st>>>(a, out, n);
+  else k_field_test<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(op, a, b, out, n);
   return cudaGetLastError();
 }
 

@@ -231,7 +231,8 @@ int msm_measure_int_peaks(double *rates, int32_t n);
 /* Device name, SM count and clock as text. */
 int msm_device_info(char *buf, size_t len);
 /* Field self-test: op 0 mul (Montgomery), 1 add, 2 sub, 3 inverse (Fermat), 4 canonicalise,
- * 5 negate, 6 inverse (binary extended Euclid);
+ * 5 negate, 6 inverse (divsteps, one thread), 7 inverse by a warp, not times a power of R and not
+ * reduced (below 2^383; a != 0 modulo q);
  * operands are 12 little-endian u32 limbs each. */
 int msm_field_selftest(int32_t op, const uint32_t *a, const uint32_t *b, uint32_t *out, uint64_t n);
 /* Throughput of the mixed twisted-Edwards addition on cached bases (adds per second). */
