@@ -21,3 +21,21 @@ def test_runs_of_few_buckets(engine, ocpu, monkeypatch, table, bits, n, kind):
         ctx.close()
     assert st["entries"] <= 7 << 17  # four lanes a run
     assert st["tasks"] >= min(st["entries"] // 64, 7000)
+
+
+@pytest.mark.parametrize("bits", [6, 13])
+def test_windowed_against_the_oracle(engine, ocpu, bits):
+    """A windowed pass on quads, with scalars of zero and at or above r, of which 253 bits are used."""
+    n = 4099
+    pts = ocpu.gen_bases(511, n)
+    sc = engine.generate_scalars(512, n, kind=1, msm_index=1)
+    sc[5] = 0
+    sc[7] = np.uint64(2**64 - 1)
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        out = ctx.mult(sc, window_bits=bits, fixed_base=2)
+    finally:
+        ctx.close()
+    masked = sc.copy()
+    masked[:, 3] &= np.uint64(2**61 - 1)
+    assert np.array_equal(out[0], ocpu.msm(pts, masked))
