@@ -289,9 +289,14 @@ Cfg heuristic_cfg(uint64_t n) {
 // Where the reduction goes by lines and bits (k_lines): up to 2^19 buckets, in windows that are large or few.
 // Beyond, one thread per run is as fast and needs no more additions than products (k_reduce1); many small
 // windows have short lines (four MSMs of 4096 points on plain records, 88 windows of 4096 buckets: 76 + 66 + 10
-// us by runs, 154 + 31 + 35 by lines; one: 31 + 63 + 18 / 51 + 18 + 35).
-bool use_lines(uint64_t buckets, uint64_t windows) {
-  return buckets <= (1u << 16) || (buckets <= (1u << 19) && buckets >= windows << 13);
+// us by runs, 154 + 31 + 35 by lines; one: 31 + 63 + 18 / 51 + 18 + 35).  Up to 2^16 buckets the lines cost a
+// block per piece, of 32 quads for lines of 4 to 16 buckets.  us per call, lines / runs of 4: one MSM in windows of
+// 4 bits (406 pieces) 1079 / 1107, 16 MSMs in windows of 4, 5, 6, 7 and 8 bits (6096, 6496, 8112, 9264, 12080 pieces)
+// 1297 / 1518, 1148 / 1280, 1135 / 1155, 1133 / 1056, 1167 / 1021; 16 MSMs of 16 points on plain records (8112) 1034 /
+// 932, of 64 points (12080) 1107 / 967.
+bool use_lines(uint64_t buckets, uint64_t windows, uint64_t pieces) {
+  if (buckets <= (1u << 16)) return pieces <= 7000;
+  return buckets <= (1u << 19) && buckets >= windows << 13;
 }
 // pieces of 128 buckets while whole lines would be too few and long to fill the GPU
 uint32_t line_log2_for(uint64_t buckets) { return buckets <= (1u << 16) ? 7u : 10u; }
@@ -402,11 +407,17 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = fal
       total += s.cfg.fixed ? std::max(nb, nbt) : (uint64_t)(nwin - 1) * nb + nbt;
     }
     pl.red_log2 = red_log2_for(total);
-    uint64_t windows = 0;
-    for (const JobSpec &s : specs)
-      if (s.n) windows += s.cfg.fixed ? 1 : windows_of(s.cfg.c);
-    pl.lines = use_lines(total, windows);
     pl.line_log2 = line_log2_for(total);
+    uint64_t windows = 0, pieces = 0;
+    for (const JobSpec &s : specs) {
+      if (s.n == 0) continue;
+      uint32_t nwin, nb, nbt;
+      layout(s.cfg.c, s.cfg.signed_digits, nwin, nb, nbt);
+      windows += s.cfg.fixed ? 1 : nwin;
+      pieces += lines_of(s.cfg.fixed ? std::max(nb, nbt) : nbt, pl.line_log2).pieces;
+      if (!s.cfg.fixed) pieces += (uint64_t)(nwin - 1) * lines_of(nb, pl.line_log2).pieces;
+    }
+    pl.lines = use_lines(total, windows, pieces);
   }
   // Level-2 groups of 128 to 512 level-1 runs, at most about 128 groups while that allows: more blocks
   // than SMs run in several waves, fewer and longer ones leave SMs idle behind longer serial sums.  A

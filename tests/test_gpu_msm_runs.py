@@ -39,3 +39,18 @@ def test_windowed_against_the_oracle(engine, ocpu, bits):
     masked = sc.copy()
     masked[:, 3] &= np.uint64(2**61 - 1)
     assert np.array_equal(out[0], ocpu.msm(pts, masked))
+
+
+@pytest.mark.parametrize("bits,msms", [(4, 18), (5, 17), (6, 13), (6, 14), (7, 16), (8, 9), (8, 10)])
+def test_reduction_of_many_small_windows(engine, ocpu, bits, msms):
+    """Passes of up to 2^16 buckets on both sides of the limit on pieces of lines."""
+    n = 60
+    pts = ocpu.gen_bases(521, n)
+    sc = engine.generate_scalars(522, n * msms, kind=1)
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        out = ctx.mult(sc, window_bits=bits, fixed_base=2, mode=2)
+    finally:
+        ctx.close()
+    for j in range(0, msms, 4):
+        assert np.array_equal(out[j], ocpu.msm(pts, sc[j * n:(j + 1) * n])), j
