@@ -116,8 +116,10 @@ struct HostPinned {
   ~HostPinned() {
     if (p) cudaFreeHost(p);
   }
-  cudaError_t ensure(size_t want) {
+  // grow-only, as DevBuf::ensure
+  cudaError_t ensure(size_t want, bool *moved) {
     if (want <= bytes && p) return cudaSuccess;
+    *moved = true;
     if (p) cudaFreeHost(p);
     p = nullptr;
     bytes = 0;
@@ -569,10 +571,12 @@ struct Workspace {
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
   }
-  // room for a pass of plan `pl`; graphs of buffers that moved go, also when a later buffer does not fit
-  cudaError_t reserve(const Plan &pl) {
+  // Room for a pass of plan `pl`, and for the results of `n_results` MSMs on the host.  Graphs of buffers
+  // that moved go, also when a later buffer does not fit.
+  cudaError_t reserve(const Plan &pl, size_t n_results = 0) {
     bool moved = false;
-    const cudaError_t e = grow(pl, moved);
+    cudaError_t e = grow(pl, moved);
+    if (!e) e = res_host.ensure(std::max(n_results, pl.jobs.size()) * MSM_PROJ_BYTES, &moved);
     if (moved) drop_graphs();
     return e;
   }
@@ -621,7 +625,6 @@ struct Workspace {
     if ((e = results.ensure(pl.jobs.size() * MSM_PROJ_BYTES, &moved))) return e;
     if ((e = jobs.ensure(pl.jobs.size() * sizeof(JobDesc), &moved))) return e;
     if ((e = wins.ensure(pl.wins.size() * sizeof(WinDesc), &moved))) return e;
-    if ((e = res_host.ensure(pl.jobs.size() * MSM_PROJ_BYTES))) return e;
     return cudaSuccess;
   }
 };
@@ -972,9 +975,8 @@ int run_msms_as(Ctx *cx, g1_projective_t *out, const std::vector<uint64_t> &size
     one[0] = {maxn, 0, 0, resolve_cfg(cx, maxn, opt)};
     set_tables(cx, one[0]);
     if (build_plan(one, probe)) return g_err;
-    if (ws.ensure(probe)) return g_err;
+    CK(ws.reserve(probe, m));
   }
-  CK(ws.res_host.ensure(m * MSM_PROJ_BYTES));
   uint64_t maxn = 0;
   for (size_t j = 0; j < m; j++) maxn = std::max(maxn, sizes[j]);
   if (!d_scalars)

@@ -103,3 +103,23 @@ def test_large_and_small_msms_from_host(engine, ocpu, monkeypatch, pull):
     first = np.concatenate([[0], np.cumsum(sizes)])
     for j in (0, 3, 4, 7):
         assert np.array_equal(out[j], ocpu.msm(pts[offs[j]:offs[j] + sizes[j]], sc[first[j]:first[j + 1]])), j
+
+
+def test_graphs_when_the_results_move(engine, ocpu):
+    """One pass per MSM from device scalars, in calls of more and more MSMs: each replays graphs of the calls
+    before it, unless the pinned results that those write to have moved."""
+    import torch
+
+    n, sizes = 200, [1, 16, 256, 512, 700, 256]
+    pts = engine.generate_bases(411, n)
+    sc = engine.generate_scalars(412, 4 * n)
+    want = [ocpu.msm(pts, sc[k * n:(k + 1) * n]) for k in range(4)]
+    d_sc = torch.from_numpy(np.tile(sc.view(np.uint8).reshape(-1), max(sizes) // 4)).cuda()
+    torch.cuda.synchronize()
+    ctx = engine.multi_scalar_mult_init(pts)
+    try:
+        for m in sizes:
+            out = ctx.mult_device([n] * m, [0] * m, d_sc.data_ptr(), mode=1)
+            assert all(np.array_equal(out[j], want[j % 4]) for j in range(m)), m
+    finally:
+        ctx.close()
