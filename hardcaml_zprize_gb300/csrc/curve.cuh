@@ -25,10 +25,9 @@ struct wpt_t {  // Weierstrass point, Jacobian (X/Z^2, Y/Z^3); z = 0 is infinity
   fq_t x, y, z;
 };
 
-// Out-of-line Montgomery product with operands by value.  The point formulas call it instead of
-// inlining seven or nine copies of the fully unrolled product: the hot loop then fits the
-// instruction cache (inlined, instruction-fetch stalls dominated k_accumulate) and runs ~20%
-// faster on GB300.
+// Out-of-line Montgomery product with operands by value.  The point formulas here call it instead of
+// inlining up to sixteen copies of the fully unrolled product, which would not fit the instruction
+// cache (k_reduce1 of 2^24 points: 2.80 ms so, 3.02 inlined).  k_accumulate's loop inlines its seven.
 static __device__ __noinline__ fq_t fq_mul_nv(fq_t a, fq_t b) { return fq_mul(a, b); }
 
 __device__ __forceinline__ xyzt_t xyzt_identity() {
@@ -98,7 +97,7 @@ __device__ __forceinline__ xyzt_t te_dbl(const xyzt_t &p) {
 }
 
 // Out-of-line copies for the cold kernels (reductions, combine, generators): one body each
-// keeps compile time and code size down; the hot accumulate loop inlines te_madd instead.
+// keeps compile time and code size down.
 static __device__ __noinline__ xyzt_t te_add_ool(const xyzt_t &p, const xyzt_t &q) { return te_add(p, q); }
 static __device__ __noinline__ xyzt_t te_dbl_ool(const xyzt_t &p) { return te_dbl(p); }
 static __device__ __noinline__ fq_t fq_mul_ool(const fq_t &a, const fq_t &b) { return fq_mul(a, b); }
@@ -129,21 +128,6 @@ __device__ __forceinline__ xyzt_t te_add_fast(const xyzt_t &p, const xyzt_t &q) 
   r.x = fq_mul_nv(E, F);
   r.y = fq_mul_nv(G, H);
   r.t = fq_mul_nv(E, H);
-  return r;
-}
-
-// small scalar multiple k*p (k >= 0) by double-and-add from the top bit
-static __device__ __noinline__ xyzt_t te_mul_small(const xyzt_t &p, uint32_t k) {
-  xyzt_t r = xyzt_identity();
-  bool started = false;
-#pragma unroll 1
-  for (int i = 31; i >= 0; i--) {
-    if (started) r = te_dbl_ool(r);
-    if ((k >> i) & 1u) {
-      r = started ? te_add_ool(r, p) : p;
-      started = true;
-    }
-  }
   return r;
 }
 

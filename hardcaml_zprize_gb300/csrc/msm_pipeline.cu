@@ -400,7 +400,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(PassBuffers pb) {
   for (int k = 0; k < kScanItems; k++) {
     if (base + k < pb.n_buckets) {
       pb.offset[base + k] = ex.x;
-      if (pb.fill) pb.fill[base + k] = ex.x;  // the scatter's slot cursor starts at the bucket's offset
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
@@ -445,7 +444,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(PassBuffers pb) {
   for (int k = 0; k < kScanItems; k++) {
     if (base + k < pb.n_buckets) {
       pb.offset[base + k] = ex.x;
-      if (pb.fill) pb.fill[base + k] = ex.x;
+      if (pb.fill) pb.fill[base + k] = ex.x;  // k_scatter's slot cursor starts at the bucket's offset
       pb.taskoff[base + k] = ex.y;
     }
     ex.x += c[k];
@@ -849,7 +848,7 @@ __global__ void __launch_bounds__(kPlaceThreads, 2) k_place_count(PassBuffers pb
   pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   extern __shared__ uint32_t sh[];
-  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < (1u << pb.bin_shift); i += kPlaceThreads) sh[i] = 0;
   PlacePart p;
   if (!place_part(pb, sh, p)) return;
@@ -1558,13 +1557,12 @@ __device__ void block_combine(const uint4 *items, uint32_t cnt, uint32_t lin_log
   }
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT) k_reduce2(PassBuffers pb) {
+__global__ void __launch_bounds__(kRedThreads) k_reduce2(PassBuffers pb) {
   pdl_begin();
   if (pb.counters[CNT_ERROR]) return;
   const uint32_t g = blockIdx.x;
   if (g >= pb.n_grps) return;
-  __shared__ uint4 sh[3 * (NT / 4) * 12];
+  __shared__ uint4 sh[3 * kRedQuads * 12];
   const WinDesc wd = pb.wins[find_win_grp(pb.wins, pb.n_wins, g)];
   const uint32_t G = 1u << pb.grp_len_log2;
   const uint32_t first = (g - wd.grp_begin) * G;
@@ -1572,10 +1570,10 @@ __global__ void __launch_bounds__(NT) k_reduce2(PassBuffers pb) {
   fq_t A, R;
   // level 3 weighs the group's R by the buckets of a group, a power of two: the doublings are done
   // here, beside the sums, instead of one after another at the end of level 3
-  block_combine<NT>(pb.seg_out + (size_t)(wd.seg_begin + first) * 24, cnt, pb.red_len_log2,
+  block_combine<kRedThreads>(pb.seg_out + (size_t)(wd.seg_begin + first) * 24, cnt, pb.red_len_log2,
                     pb.red_len_log2 + pb.grp_len_log2, sh, A, R);
   if (threadIdx.x < 4) dq_store(pb.grp_out + (size_t)g * 24 + 12, A);  // one coordinate per lane
-  if (threadIdx.x >= NT - 32 && threadIdx.x < NT - 28) dq_store(pb.grp_out + (size_t)g * 24, R);
+  if (threadIdx.x >= kRedThreads - 32 && threadIdx.x < kRedThreads - 28) dq_store(pb.grp_out + (size_t)g * 24, R);
 }
 
 // Windows of at most kRed3SmallMax groups (windowed MSMs: 2^(c-1) buckets make a few groups)
@@ -2061,7 +2059,7 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
   if (pb.lines && pb.n_grps > 0) {
     run(k_bits, pb.n_grps, 4 * kBitQuads, 0, pb);
   } else if (pb.n_grps > 0) {
-    run(k_reduce2<256>, pb.n_grps, 256, 0, pb);
+    run(k_reduce2, pb.n_grps, kRedThreads, 0, pb);
   }
   mark(8);
   if (pb.lines && pb.n_wins > 0) {
