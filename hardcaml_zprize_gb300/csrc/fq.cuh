@@ -99,6 +99,10 @@ __device__ __forceinline__ fq_t fq_one() {
 }
 
 // ---- a * b * 2^-384 mod q (CIOS; inputs and output in [0, 2q)) ----
+// The steps are CIOS (Koc, Acar, Kaliski, "Analyzing and Comparing Montgomery Multiplication Algorithms", IEEE
+// Micro 1996) with the even and the odd columns kept as two carry chains, the published arrangement for 32-bit
+// GPU multipliers (Emmart, Luitjens, Weems, Woolley, "Optimizing Modular Multiplication for NVIDIA's Maxwell
+// GPUs", ARITH 2016).
 // Row i adds b_i a and then m q to the running value and drops its lowest word, m = -t0 (q = 1 mod
 // 2^32 and -q^-1 = -1 mod 2^32, so the row factor needs no product and m q0 + t0 = 0 with a carry of
 // (t0 != 0)).  The running value is the sum of two word vectors on 64-bit lanes: E, words 0 to 11,

@@ -144,10 +144,13 @@ struct Cfg {
 // Level-1 reduction runs of 2^red buckets, 4 to 64.  Small passes are latency-bound: each quad or
 // thread adds 2 x 2^red points in sequence.  Passes of 2^22 buckets or more take runs of 64 (about 2^16
 // of them still keep k_reduce1 near the product throughput), which leaves fewer groups for the
-// latency-bound levels 2 and 3.  Measured on GB300, whole MSMs, runs of 4 / 8 / 16 (us): 2^15 buckets
-// (4096 points on tables of width 16) 240 / 249 / 276, 50000 points 518 / 543 / 610; 2^19 buckets (2^20
-// points) runs of 8 / 16 / 32: 3738 / 3626 / 3688; 4.9 M (2^24 points) 32 / 64 / 128: 44.14 / 44.01 /
-// 44.00 ms.
+// latency-bound levels 2 and 3.  Measured on GB300, us per call of passes that are reduced by runs (see
+// use_lines), runs of 4 / 8 / 16 / 32 / 64 buckets: 0.95e5 buckets (4 MSMs of 4096 points on plain records) 872 /
+// 870 / 899 / 957 / 1120, 2.6e5 (64 of 64 points) 1675 / 1713 / 1762 / 1795 / 1938, 5.6e5 (17 of 50000 on width 16)
+// 3824 / 3671 / 3659 / 3709 / 3866, 2^20 (32 of 1000) 1399 / 1206 / 1067 / 1030 / 1162, 2^21 (64 of 1000) 2418 / 2052 /
+// 1952 / 1817 / 1779 and (4 of 2^20) 14328 / 14007 / 13934 / 13831 / 13824, 4.9e6 (2^24 points, the
+// same 2^16 scalars over and over) 48392 / 47095 / 46499 / 46287 / 46080 (128: 46077), 8.2e6 (250 of 1000) 8609 / 7191 /
+// 6431 / 6146 / 6253.
 uint32_t red_log2_for(uint64_t buckets) {
   int lg = 0;
   while (lg < 63 && (2ull << lg) <= buckets) lg++;  // floor(log2(buckets))
@@ -224,7 +227,7 @@ uint32_t whole_bucket_run(double mean) {
 
 // A pass of at most this many entries sums each run with four lanes (k_accumulate_quad): it has too
 // few runs to fill the GPU with one thread each.  Measured on GB300 (us per MSM on width-16 tables, quads /
-// threads): 50000 points (0.85e6 entries) 526 / 545, 55000 572 / 557, 61000 609 / 558.
+// threads, each at its own run length): 40000 points (0.68e6 entries) 379 / 465, 52000 473 / 484, 55000 491 / 487.
 constexpr uint64_t kQuadEntries = 7ull << 17;
 
 // Run length of such a pass: a run costs a quad two product latencies per entry, a split bucket a
@@ -370,9 +373,11 @@ constexpr uint32_t kPlacePart = 16384;
 // 66000 points (1.06e6 entries) 588 / 589, 100000 738 / 732, 140000 904 / 890, 350000 1748 / 1692,
 // 800000 3494 / 3403; without tables 80000 (1.6e6) 1243 / 1217, 350000 2390 / 2345.
 // A pass that reads its scalars from host memory while it counts hides the ranked sort's atomics behind
-// the C2C link, and k_place_count comes on top: for those the line lies higher (ms per call, ranked /
-// partitioned: 4 x 100000 1.96 / 1.99, 4 x 200000 3.44 / 3.48, 4 x 2^20 in one pass 14.22 / 14.26, one
-// MSM of 3e6 9.80 / 9.77).
+// the C2C link, and k_place_count comes on top: for those the line lies higher (us per call, two runs of 11
+// calls each, ranked / partitioned: 4 x 50000 1066, 1066 / 1118, 1118; 4 x 100000 1904, 1904 / 1929, 1927; 4 x
+// 200000 3401, 3398 / 3450, 3447; 16 x 2^18 16302, 16316 / 16469, 16489; 4 x 2^20 14270, 14274 / 14368, 14362; one MSM
+// of 2^20 3790, 3774 / 3787, 3775; 2^21 7028, 7030 / 6993, 6997; 3e6 9744, 9747 / 9714, 9721; 2^22 13266, 13253 /
+// 13267, 13268).
 constexpr uint64_t kPartitionEntries = 1ull << 20;
 constexpr uint64_t kPartitionEntriesHost = 1ull << 25, kPartitionEntriesHostMany = 1ull << 27;
 
@@ -424,9 +429,9 @@ int build_plan(const std::vector<JobSpec> &specs, Plan &pl, bool host_read = fal
   // Level-2 groups of 128 to 512 level-1 runs, at most about 128 groups while that allows: more blocks
   // than SMs run in several waves, fewer and longer ones leave SMs idle behind longer serial sums.  A
   // window of more than 16 groups is then combined by a block, one of fewer serially by one quad.
-  // Measured on GB300 (levels 2 + 3, us, groups of 128 / 256 / 512 runs): 2^12 points (8192 runs) 129 /
-  // 158 / -, 2^20 (32 K runs) 215 / 200 / 219; a shared pass of 4 x 50000 (16 K runs) 103 / - / 187;
-  // the uneven mix of 64 (131 K runs) keeps 512.
+  // Measured on GB300 (us per call, groups of 128 / 256 / 512 runs): 4 MSMs of 4096 points on plain records (12 K
+  // runs) 879 / 892 / 894, 17 of 50000 on width 16 (35 K) 3757 / 3664 / 3670, 32 of 1000 (65 K) 1292 / 1152 / 1081,
+  // 64 of 1000 (131 K) 2237 / 2072 / 1956, 2^24 points (76 K) 46438 / 46217 / 46099.
   {
     uint64_t runs = 0;
     for (const JobSpec &s : specs) {
@@ -860,8 +865,8 @@ Cfg resolve_cfg(Ctx *cx, uint64_t n, const msm_options_t *opt, bool shared_pass 
       if (!table_c(which)) continue;
       const double v = model_cost_fixed(n, table_c(which), 1);
       // between two sets: alone on few buckets the runs are parts of buckets, too few to fill the GPU
-      // evenly, and are merged (ms on a context of 2^20 bases, width 16 / 20: 262144 points 1.39 / 1.30,
-      // 349525 1.66 / 1.58, 524288 2.45 / 2.08)
+      // evenly, and are merged (ms, width 16 / 20: 131072 points 0.79 / 0.88, 262144 1.35 / 1.26, 524288 2.42 /
+      // 2.04)
       uint32_t nwin, nb, nbt;
       layout(table_c(which), 1, nwin, nb, nbt);
       const double between = !shared_pass && nb < (1u << 17) && n * nwin > 64ull * nb ? 1.2 * v : v;
@@ -1194,9 +1199,12 @@ uint32_t choose_fixed_base(uint64_t n) {
       return (uint32_t)c;
     if (strcmp(e, "auto")) return 0;
   }
-  // below 2^20 bases MSMs are latency-bound: the windowed form's serial combine (c (W - 1)
-  // dependent doublings, ~1.2 ms) dominates, and tables of width 16 (16 windows, 2^15 shared
-  // buckets, at most 2.4 GB) measured fastest or within 5% at 2^12..2^18 bases
+  // below 2^20 bases MSMs are latency-bound: the windowed form's serial combine (c (W - 1) dependent
+  // doublings, ~0.5 ms) dominates.  Tables of width 16 (16 windows, 2^15 shared buckets, at most 2.4 GB) are the
+  // fastest of 11 to 20 or within 11% of it up to 2^18 bases (us per MSM over as many bases, width 13 / 15 / 16 /
+  // 17 / 20): 2^10 173 / 173 / 185 / 222 / 743, 2^12 219 / 185 / 202 / 236 / 732, 2^14 341 / 272 / 271 / 284 / 844, 2^16
+  // 845 / 519 / 518 / 507 / 1162, 2^17 1198 / 828 / 791 / 743 / 877, 2^18 1755 / 1419 / 1347 / 1212 / 1257; at 2^19
+  // 3009 / 2526 / 2416 / 2097 / 2035
   if (n < (1ull << 20)) return fits(16) ? 16u : 0u;
   uint32_t best = 0;
   double best_cost = 1e300;

@@ -1933,10 +1933,10 @@ size_t msm_scan_tmp_words(uint32_t n_buckets) {
 }
 
 // Level-1 reductions of at most this many runs take a quad each (k_reduce1_quad): one thread each
-// would leave the GPU idle behind a chain of 8 products per addition.  Measured on GB300 (us, threads /
-// quads): 8192 runs of 4 buckets (tables of width 16) 61 / 33, 32768 runs of 16 (2^20 points) 346 / 332;
-// 65536 runs of 8 there 327 / 301, but with 35 more in level 2.  Larger reductions are bound by product
-// throughput in either form.
+// would leave the GPU idle behind a chain of 8 products per addition.  Measured on GB300 (us per call, threads /
+// quads): 4 MSMs of 4096 points on plain records (12 K runs) 929 / 879, 65536 points there (10 K) 1238 / 1176, 17 MSMs of
+// 50000 points on width 16 (35 K) 3670 / 3692.  Far above the line the two are within a few percent: 2^24 points (76 K
+// runs of 64 buckets) 46.11 / 45.80 ms, 64 MSMs of 1000 points (131 K of 16) 1954 / 1863.
 constexpr uint32_t kReduceQuadSegs = 32768;
 
 cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st, cudaEvent_t *ev,
@@ -2052,10 +2052,11 @@ cudaError_t msm_launch_pass(const PassBuffers &pb, int num_sms, cudaStream_t st,
       run(k_reduce1, (pb.n_segs + 127) / 128, 128, 0, pb);
   }
   mark(7);
-  // Level 2 in blocks of 256 threads; level 3 (one block per window) in blocks of 128 while
-  // they fit on the SMs in one wave: with one warp per SMSP a quad addition takes 1.9 us, with two 2.8,
-  // but a quad of the smaller block sums twice as many runs in sequence.  Measured on GB300 (us, level 2
-  // with 256 / 128 threads): 2^12 points 63 / 66, 4 x 50000 72 / 74; level 3 with 128 threads 45 and 39.
+  // Level 2 in blocks of 256 threads; level 3 (one block per window of more than 16 groups) in blocks of 128
+  // while they fit on the SMs in one wave: with one warp per SMSP a quad addition takes 1.9 us, with two 2.8,
+  // but a quad of the smaller block sums twice as many runs in sequence.  Measured on GB300 (us, 256 / 128
+  // threads): level 2 of 4 MSMs of 4096 points on plain records 66 / 68, of 32 of 1000 on width 16 133 / 158, of
+  // 64 of those 256 / 201, of 2^24 points 135 / 160; level 3 of 2^24 points (150 groups) 88 / 100.
   if (pb.lines && pb.n_grps > 0) {
     run(k_bits, pb.n_grps, 4 * kBitQuads, 0, pb);
   } else if (pb.n_grps > 0) {
