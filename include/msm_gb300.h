@@ -110,7 +110,7 @@ int msm_mult_ex(void *context, g1_projective_t *out, uint64_t batch_size,
 /* Many MSMs of uneven sizes in one pass with one shared sort. MSM j uses sizes[j] bases starting
  * at base_offsets[j] and the next sizes[j] scalars of the concatenated `scalars` array.
  * opt->mode == 1 runs them one pass per MSM instead (the plain form); 0 groups them into passes of
- * a few million points. */
+ * a few million points and about 2 GB of workspace, less where that much memory is not free. */
 int msm_mult_uneven(void *context, g1_projective_t *out, uint64_t num_msms, const uint64_t *sizes,
                     const uint64_t *base_offsets, const biginteger256_t *scalars,
                     const msm_options_t *opt);
